@@ -383,8 +383,8 @@ struct RabiReq {
 
 // The kinetic pass with the Rabi sums of the requested components folded in:
 // after FFT_x every axis is in k-space and |psi^|^2 does not see the kinetic
-// phase, so the sums of the state after the pass are taken there.  Unscaled
-// sums go to ctx->red_partial (one row per CTA), the totals to sums[c*n+m].
+// phase, so the sums of the state after the pass are taken there: unscaled, to
+// sums[c*n+m].
 // ATUS_E_UNSUPPORTED (fields untouched) where the register-staged x pass does
 // not apply.
 static int kinetic_pass_rabi(atus_ctx *ctx, int half, const RabiReq &rr, double *sums) {
@@ -411,15 +411,12 @@ static int kinetic_pass_rabi(atus_ctx *ctx, int half, const RabiReq &rr, double 
   }
   a.rabi_thr = rr.thr;
   a.rabi_partial = ctx->red_partial;
-  CK(cudaMemsetAsync(ctx->red_partial, 0, sizeof(double) * RED_BLOCKS * RED_MAXQ, ctx->stream));
+  a.rabi_count = ctx->red_count;
+  a.rabi_out = ctx->h_red;
   const int r = (ctx->prec == ATUS_PREC_FP64) ? launch_pass2_d_kr(ctx, a, 0) : launch_pass2_f_kr(ctx, a, 0);
   if (r != ATUS_OK) return r;
-  const int nq = rr.ncomp * rr.n;
-  reduce_final<<<1, 32, 0, ctx->stream>>>(ctx->red_partial, RED_BLOCKS, nq, ctx->red_out);
-  LAUNCHED(ctx);
-  CK(cudaMemcpyAsync(ctx->h_red, ctx->red_out, sizeof(double) * nq, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  for (int q = 0; q < nq; q++) sums[q] = ctx->h_red[q];
+  for (int q = 0; q < rr.ncomp * rr.n; q++) sums[q] = ctx->h_red[q];
   return ATUS_OK;
 }
 
@@ -433,42 +430,42 @@ static int potential_pass(atus_ctx *ctx, const NLArgs &nl) {
 }
 
 // ------------------------------------------------------------------ reductions
-static int reduce(atus_ctx *ctx, RedArgs &a, double *out) {
+// One launch: as many blocks as give each thread RED_AHEAD points, at most
+// four per SM; totals to dst (device memory, or host memory mapped into the
+// device, which saves the copy back).
+static int launch_reduce(atus_ctx *ctx, RedArgs &a, double *dst) {
   a.g = geo(ctx);
-  a.dim = ctx->dim;
   for (int ax = 0; ax < 3; ax++) {
     a.d[ax] = ctx->d[ax];
     a.dk[ax] = ctx->dk[ax];
     a.n[ax] = (int)ctx->n[ax];
     a.shift[ax] = (int)(ctx->n[ax] / 2);
   }
-  if (ctx->prec == ATUS_PREC_FP64 || a.mode == RED_MOM || a.mode == RED_RABI)
-    reduce_kernel<double><<<RED_BLOCKS, RED_THREADS, 0, ctx->stream>>>(a, ctx->red_partial);
-  else
-    reduce_kernel<float><<<RED_BLOCKS, RED_THREADS, 0, ctx->stream>>>(a, ctx->red_partial);
+  const int64_t per = (int64_t)RED_THREADS * RED_AHEAD;
+  const int64_t want = (ctx->npts + per - 1) / per;
+  const unsigned grid = (unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS);
+  const bool fp64 = ctx->prec == ATUS_PREC_FP64;
+#define ATUS_RED(R, M) reduce_kernel<R, M><<<grid, RED_THREADS, 0, ctx->stream>>>(a, ctx->red_partial, ctx->red_count, dst)
+  switch (a.mode) {
+    case RED_NORM: if (fp64) ATUS_RED(double, RED_NORM); else ATUS_RED(float, RED_NORM); break;
+    case RED_POS: if (fp64) ATUS_RED(double, RED_POS); else ATUS_RED(float, RED_POS); break;
+    case RED_MOM: ATUS_RED(double, RED_MOM); break;    // spectra are FP64
+    case RED_RABI: ATUS_RED(double, RED_RABI); break;
+    case RED_DOT2: ATUS_RED(double, RED_DOT2); break;  // the Sobolev descent runs in FP64
+    case RED_MU: ATUS_RED(double, RED_MU); break;
+    case RED_PROJ: ATUS_RED(double, RED_PROJ); break;
+    case RED_SOBG: ATUS_RED(double, RED_SOBG); break;
+    default: return fail(ctx, ATUS_E_ARG, "unknown reduction");
+  }
+#undef ATUS_RED
   LAUNCHED(ctx);
-  reduce_final<<<1, 32, 0, ctx->stream>>>(ctx->red_partial, RED_BLOCKS, a.nq, ctx->red_out);
-  LAUNCHED(ctx);
-  CK(cudaMemcpyAsync(ctx->h_red, ctx->red_out, sizeof(double) * a.nq, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  for (int i = 0; i < a.nq; i++) out[i] = ctx->h_red[i];
   return ATUS_OK;
 }
 
-// The same reduction, result left in device memory (no host round trip).
-static int reduce_dev(atus_ctx *ctx, RedArgs &a, double *dst) {
-  a.g = geo(ctx);
-  a.dim = ctx->dim;
-  for (int ax = 0; ax < 3; ax++) {
-    a.d[ax] = ctx->d[ax];
-    a.dk[ax] = ctx->dk[ax];
-    a.n[ax] = (int)ctx->n[ax];
-    a.shift[ax] = (int)(ctx->n[ax] / 2);
-  }
-  reduce_kernel<double><<<RED_BLOCKS, RED_THREADS, 0, ctx->stream>>>(a, ctx->red_partial);
-  LAUNCHED(ctx);
-  reduce_final<<<1, 32, 0, ctx->stream>>>(ctx->red_partial, RED_BLOCKS, a.nq, dst);
-  LAUNCHED(ctx);
+static int reduce(atus_ctx *ctx, RedArgs &a, double *out) {
+  RUN(launch_reduce(ctx, a, ctx->h_red));
+  CK(cudaStreamSynchronize(ctx->stream));
+  for (int i = 0; i < a.nq; i++) out[i] = ctx->h_red[i];
   return ATUS_OK;
 }
 
@@ -586,9 +583,12 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
     if (ok) ok = cudaMemset(ctx->psi[c], 0, ctx->csize * ctx->npts) == cudaSuccess;
   }
   if (ok) ok = cudaMalloc(&ctx->scratch, 16 * ctx->npts) == cudaSuccess;
-  if (ok) ok = cudaMalloc(&ctx->err_dev, sizeof(int)) == cudaSuccess && cudaMemset(ctx->err_dev, 0, sizeof(int)) == cudaSuccess;
+  if (ok) ok = cudaMallocHost(&ctx->err_word, sizeof(int)) == cudaSuccess;
+  if (ok) *ctx->err_word = 0;
   if (ok) ok = cudaMalloc(&ctx->red_partial, sizeof(double) * RED_BLOCKS * RED_MAXQ) == cudaSuccess;
-  if (ok) ok = cudaMalloc(&ctx->red_out, sizeof(double) * RED_MAXQ) == cudaSuccess;
+  if (ok)
+    ok = cudaMalloc(&ctx->red_count, sizeof(unsigned)) == cudaSuccess &&
+         cudaMemset(ctx->red_count, 0, sizeof(unsigned)) == cudaSuccess;
   if (ok) ok = cudaMallocHost(&ctx->h_red, sizeof(double) * RED_MAXQ) == cudaSuccess;
   if (ok) ok = cudaMallocHost(&ctx->h_sob, sizeof(SobDev)) == cudaSuccess;
   if (ok) {
@@ -667,7 +667,7 @@ void atus_destroy(atus_ctx *ctx) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   cudaFree(ctx->fs_tw);
   cudaFree(ctx->fs_tmp);
-  cudaFree(ctx->err_dev);
+  if (ctx->err_word) cudaFreeHost(ctx->err_word);
   cudaFree(ctx->scratch);
   cudaFree(ctx->sob_dev);
   if (ctx->sob_graph) cudaGraphExecDestroy(ctx->sob_graph);
@@ -675,7 +675,7 @@ void atus_destroy(atus_ctx *ctx) {
   if (ctx->tw != ctx->tw64) cudaFree(ctx->tw);
   cudaFree(ctx->tw64);
   cudaFree(ctx->red_partial);
-  cudaFree(ctx->red_out);
+  cudaFree(ctx->red_count);
   if (ctx->h_red) cudaFreeHost(ctx->h_red);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
@@ -683,16 +683,16 @@ void atus_destroy(atus_ctx *ctx) {
 
 const char *atus_last_error(const atus_ctx *ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
-// The device error word after kernels with bounded waits (the TMA-fed
-// passes): read once they are done, reset, and reported as ATUS_E_CUDA.
+// The error word after kernels with bounded waits (the TMA-fed passes): host
+// memory that the kernels write to, read once they are done, reset, and
+// reported as ATUS_E_CUDA.
 static int wait_check(atus_ctx *ctx) {
   if (!ctx->err_armed) return ATUS_OK;
   ctx->err_armed = false;
-  int e = 0;
-  CK(cudaMemcpyAsync(&e, ctx->err_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (e == 0) return ATUS_OK;
-  CK(cudaMemsetAsync(ctx->err_dev, 0, sizeof(int), ctx->stream));
+  volatile int *word = ctx->err_word;
+  if (*word == 0) return ATUS_OK;
+  *word = 0;
   return fail(ctx, ATUS_E_CUDA, "a TMA tile copy did not complete within the wait limit");
 }
 
@@ -1492,7 +1492,7 @@ static int sob_iterate_dev(atus_ctx *ctx) {
     r.a = ctx->psi[i];
     r.c = ctx->sob_psi[i];
     r.w = (double2 *)ctx->sob_grad[i];
-    RUN(reduce_dev(ctx, r, d->q[i]));
+    RUN(launch_reduce(ctx, r, d->q[i]));
     RedArgs p;  // Project_Sobolev_Gradient fused with the norm of the projected gradient
     memset(&p, 0, sizeof(p));
     p.mode = RED_PROJ;
@@ -1500,7 +1500,7 @@ static int sob_iterate_dev(atus_ctx *ctx) {
     p.w = (double2 *)ctx->sob_grad[i];
     p.c = ctx->sob_psi[i];
     p.fq = d->q[i];
-    RUN(reduce_dev(ctx, p, &d->g2[i]));
+    RUN(launch_reduce(ctx, p, &d->g2[i]));
   }
   sob_scalars_kernel<<<1, 1, 0, ctx->stream>>>(d, ctx->ar, n);
   LAUNCHED(ctx);

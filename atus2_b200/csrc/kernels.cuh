@@ -106,14 +106,15 @@ struct PassArgs {
   double dk[3];
   int n[3];
   // M2_KIN_RABI: balls k0[c * rabi_n + m] (m < rabi_n) of component
-  // rabi_comp[c] (c < rabi_ncomp), radius rabi_thr; per-CTA sums of the
-  // unscaled |psi^|^2 to rabi_partial[blockIdx.x * 8 + q]
+  // rabi_comp[c] (c < rabi_ncomp), radius rabi_thr; sums of the unscaled
+  // |psi^|^2 to rabi_out (red_finish with rabi_partial and rabi_count)
   int rabi_ncomp, rabi_n;
   int rabi_comp[2];
   double rabi_thr;
   double rabi_k0[8][3];
-  double *rabi_partial;
-  int *err;  // device error word (bounded waits that ran out set bits)
+  double *rabi_partial, *rabi_out;
+  unsigned *rabi_count;
+  int *err;  // error word, mapped host memory (a bounded wait that ran out sets it)
   long wait_limit;       // try_wait rounds before a TMA tile counts as lost
   int drop_copies;       // issue no tile copies, so every wait runs out (error-path tests; 0)
 };
@@ -1034,7 +1035,7 @@ struct SobArgs {
 
 // ------------------------------------------------------------ reductions
 // Quantities per mode (all FP64 accumulations, fixed order per thread, fixed
-// tree per block, partials summed in block order by reduce_final).
+// tree per block, block sums in a fixed order).
 enum { RED_NORM = 0, RED_POS = 1, RED_MOM = 2, RED_RABI = 3, RED_DOT2 = 4, RED_MU = 5, RED_PROJ = 6, RED_SOBG = 7 };
 constexpr int RED_MAXQ = 8;
 constexpr int RED_BLOCKS = 592;  // 4 x 148 SMs
@@ -1046,7 +1047,6 @@ struct RedArgs {
   const void *a, *b, *c;   // field operands
   const double *V;
   Geo g;
-  int dim;
   double d[3], dk[3];
   int n[3], shift[3];
   double k0[8][3];         // Rabi centres
@@ -1060,107 +1060,188 @@ struct RedArgs {
   const double *fq;
 };
 
-template <typename R>
-__device__ __forceinline__ void red_point(const RedArgs &a, int64_t l, double *q) {
+// |psi^|^2 = den at wavenumber k into the Rabi bins, with the bin rule of
+// compute_rabi_integrals (include/CRT_Base_IF.h:231-257): a point inside a
+// ball adds to the current bin and the bin index does not advance for it.
+// Inside is sqrt(|k0 - k|^2) < thr; the root is only taken within a few
+// roundings of the surface, elsewhere the squares decide.
+template <int ND>
+__device__ __forceinline__ void red_balls(const double (*k0)[3], int n, double thr, const double *k, double den,
+                                          double *q) {
+  const double t2 = thr * thr, lo = thr > 0 ? t2 * (1 - 1e-14) : -1.0, hi = thr > 0 ? t2 * (1 + 1e-14) : -1.0;
+  int j = 0;
+  #pragma unroll
+  for (int m = 0; m < RED_MAXQ; m++) {
+    if (m >= n) break;
+    double dd = 0;
+    #pragma unroll
+    for (int ax = 0; ax < ND; ax++) {
+      const double d = k0[m][ax] - k[ax];
+      dd += d * d;
+    }
+    if (dd < lo || (!(dd > hi) && sqrt(dd) < thr)) {
+      #pragma unroll
+      for (int i = 0; i <= m; i++) q[i] += (i == j) ? den : 0.0;
+      continue;
+    }
+    j++;
+  }
+}
+
+// The operands of one point, loaded before any is used, so that a thread's
+// loads of several points are in flight together.
+template <typename R, int MODE> struct RedIn {
+  cplx<R> v, b, c;
+  double pot;
+};
+
+template <typename R, int MODE>
+__device__ __forceinline__ void red_fetch(const RedArgs &a, int64_t l, RedIn<R, MODE> &in) {
   using C = cplx<R>;
-  if (a.mode == RED_SOBG) {
+  if constexpr (MODE == RED_SOBG || MODE == RED_PROJ) in.b = ((const C *)a.w)[l];
+  if constexpr (MODE == RED_DOT2 || MODE == RED_MU) in.b = ((const C *)a.b)[l];
+  if constexpr (MODE != RED_PROJ) in.v = ((const C *)a.a)[l];
+  if constexpr (MODE == RED_SOBG || MODE == RED_PROJ) in.c = ((const C *)a.c)[l];
+  if constexpr (MODE == RED_DOT2) in.c = a.c ? ((const C *)a.c)[l] : mk<R>(0, 0);
+  if constexpr (MODE == RED_MU) in.pot = a.V ? a.V[l] : 0.0;
+}
+
+template <typename R, int MODE>
+__device__ __forceinline__ void red_point(const RedArgs &a, int64_t l, const RedIn<R, MODE> &in, double *q) {
+  using C = cplx<R>;
+  if constexpr (MODE == RED_SOBG) {
     // w = S(W psi) becomes the Sobolev gradient S(-Lap psi + W psi) =
     // S(W psi) + psi - S psi (S = 1/(1 + alpha k^2), so S alpha k^2 = 1 - S),
     // then Re<psi, G>, Re<psi, S psi>, <psi, psi>
-    const double2 p = ((const double2 *)a.a)[l], ps = ((const double2 *)a.c)[l];
-    double2 g = a.w[l];
+    const double2 p = to_d<R>(in.v), ps = to_d<R>(in.c);
+    double2 g = to_d<R>(in.b);
     g.x += p.x - ps.x;
     g.y += p.y - ps.y;
     a.w[l] = g;
     q[0] += p.x * g.x + p.y * g.y;
     q[1] += p.x * ps.x + p.y * ps.y;
     q[2] += p.x * p.x + p.y * p.y;
-    return;
-  }
-  if (a.mode == RED_PROJ) {  // Project_Sobolev_Gradient and the norm of the result in one pass
+  } else if constexpr (MODE == RED_PROJ) {  // Project_Sobolev_Gradient and the norm of the result in one pass
     const double fak = a.fq[0] / a.fq[1];
-    double2 v = a.w[l];
-    const double2 u = ((const double2 *)a.c)[l];
+    double2 v = to_d<R>(in.b);
+    const double2 u = to_d<R>(in.c);
     v.x -= fak * u.x;
     v.y -= fak * u.y;
     a.w[l] = v;
     q[0] += v.x * v.x + v.y * v.y;
-    return;
-  }
-  const C v = ((const C *)a.a)[l];
-  const double den = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
-  if (a.mode == RED_NORM) { q[0] += den; return; }
-  int ijk[3];
-  idx3(a.g, l, ijk[0], ijk[1], ijk[2]);
-  if (a.mode == RED_POS) {
-    for (int ax = 0; ax < a.dim; ax++) q[ax] += ((double)(ijk[ax] - a.shift[ax]) * a.d[ax]) * den;
-    return;
-  }
-  double k[3];
-  for (int ax = 0; ax < a.dim; ax++) {
-    const int t = (ijk[ax] + a.shift[ax]) % a.n[ax];
-    k[ax] = a.dk[ax] * (double)(t - a.shift[ax]);
-  }
-  if (a.mode == RED_MOM) {
-    for (int ax = 0; ax < a.dim; ax++) q[ax] += k[ax] * den;
-    return;
-  }
-  if (a.mode == RED_RABI) {
-    int j = 0;
-    for (int m = 0; m < a.nq; m++) {
-      double dd = 0;
-      for (int ax = 0; ax < a.dim; ax++) {
-        const double d = a.k0[m][ax] - k[ax];
-        dd += d * d;
+  } else {
+    const C v = in.v;
+    const double den = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
+    if constexpr (MODE == RED_NORM) q[0] += den;
+    if constexpr (MODE == RED_POS || MODE == RED_MOM || MODE == RED_RABI) {
+      int ijk[3];
+      idx3(a.g, l, ijk[0], ijk[1], ijk[2]);
+      double x[3];
+      #pragma unroll
+      for (int ax = 0; ax < 3; ax++) {  // axis lengths are powers of two (unused axes: one point)
+        const int t = (MODE == RED_POS) ? ijk[ax] : ((ijk[ax] + a.shift[ax]) & (a.n[ax] - 1));
+        x[ax] = (double)(t - a.shift[ax]) * ((MODE == RED_POS) ? a.d[ax] : a.dk[ax]);
       }
-      if (sqrt(dd) < a.thr) { q[j] += den; continue; }
-      j++;
-    }
-    return;
-  }
-  if (a.mode == RED_DOT2) {  // Re<a,b>, Re<a,c> (and <a,a> when nq is 3)
-    const C b = ((const C *)a.b)[l];
-    q[0] += (double)v.x * (double)b.x + (double)v.y * (double)b.y;
-    if (a.c) {
-      const C c = ((const C *)a.c)[l];
-      q[1] += (double)v.x * (double)c.x + (double)v.y * (double)c.y;
-    }
-    if (a.nq > 2) q[2] += den;
-    return;
-  }
-  if (a.mode == RED_MU) {  // a = psi_i, b = Lap psi_i
-    const C lp = ((const C *)a.b)[l];
-    double nl = 0;
-    #pragma unroll
-    for (int j = 0; j < MAXC; j++) {
-      if (j < a.ncomp) {
-        const C pj = ((const C *)a.psi_all[j])[l];
-        nl += a.gs[a.comp * MAXC + j] * ((double)pj.x * (double)pj.x + (double)pj.y * (double)pj.y);
+      if constexpr (MODE != RED_RABI) {
+        #pragma unroll
+        for (int ax = 0; ax < 3; ax++) q[ax] += x[ax] * den;
+      } else {
+        red_balls<3>(a.k0, a.nq, a.thr, x, den, q);
       }
     }
-    const double pot = a.V ? a.V[l] : 0.0;
-    q[0] += -((double)v.x * (double)lp.x + (double)v.y * (double)lp.y) + (pot + nl) * den;
+    if constexpr (MODE == RED_DOT2) {  // Re<a,b>, Re<a,c> (and <a,a> when nq is 3)
+      q[0] += (double)v.x * (double)in.b.x + (double)v.y * (double)in.b.y;
+      q[1] += (double)v.x * (double)in.c.x + (double)v.y * (double)in.c.y;
+      q[2] += den;
+    }
+    if constexpr (MODE == RED_MU) {  // a = psi_i, b = Lap psi_i
+      double nl = 0;
+      #pragma unroll
+      for (int j = 0; j < MAXC; j++) {
+        if (j < a.ncomp) {
+          const C pj = ((const C *)a.psi_all[j])[l];
+          nl += a.gs[a.comp * MAXC + j] * ((double)pj.x * (double)pj.x + (double)pj.y * (double)pj.y);
+        }
+      }
+      q[0] += -((double)v.x * (double)in.b.x + (double)v.y * (double)in.b.y) + (in.pot + nl) * den;
+    }
   }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs a, double *partial) {
+// Block sums of q[0..nq) over NT threads, then -- in the block that finishes
+// last -- the sums over all blocks, in a fixed order whichever block that is.
+// partial: gridDim.x rows of RED_MAXQ; count: zero before the launch and left
+// at zero; out: nq totals (device memory or mapped host memory).
+// Measured against a second launch whose one thread per quantity added 592
+// rows: that launch took 25-29 us by itself, of 50 us for a reduction over
+// 2^21 points.
+template <int NT>
+__device__ __forceinline__ void red_finish(double *q, int nq, double *partial, unsigned *count, double *out) {
+  static_assert(NT % 32 == 0 && NT >= 4 * RED_MAXQ, "whole warps, several rows per quantity");
+  constexpr int NW = NT / 32, ROWS = NT / RED_MAXQ;
+  __shared__ double sh[NT];
+  __shared__ int last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __syncthreads();
+  #pragma unroll
+  for (int i = 0; i < RED_MAXQ; i++) {
+    if (i < nq) {
+      double v = q[i];
+      #pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) sh[warp * RED_MAXQ + i] = v;
+    }
+  }
+  __syncthreads();
+  if (tid < nq) {
+    double v = sh[tid];
+    #pragma unroll
+    for (int w = 1; w < NW; w++) v += sh[w * RED_MAXQ + tid];
+    partial[(int64_t)blockIdx.x * RED_MAXQ + tid] = v;
+    __threadfence();
+  }
+  __syncthreads();
+  if (tid == 0) last = (atomicAdd(count, 1u) == gridDim.x - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int i = tid % RED_MAXQ, r0 = tid / RED_MAXQ;
+  double v = 0;
+  if (i < nq) {
+    #pragma unroll 8
+    for (int r = r0; r < (int)gridDim.x; r += ROWS) v += __ldcg(&partial[(int64_t)r * RED_MAXQ + i]);
+  }
+  sh[tid] = v;
+  __syncthreads();
+  if (tid < nq) {
+    v = sh[tid];
+    for (int r = 1; r < ROWS; r++) v += sh[r * RED_MAXQ + tid];
+    out[tid] = v;
+  }
+  if (tid == 0) *count = 0;
+}
+
+// Points a thread loads before it uses the first: with 32 warps on an SM
+// four 16-byte loads each keep 64 KB in flight, more than the ~45 KB that
+// HBM's latency times its rate asks of an SM.
+constexpr int RED_AHEAD = 4;
+
+template <typename R, int MODE>
+__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs a, double *partial, unsigned *count, double *out) {
   double q[RED_MAXQ];
   #pragma unroll
   for (int i = 0; i < RED_MAXQ; i++) q[i] = 0;
-  for (int64_t l = blockIdx.x * (int64_t)RED_THREADS + threadIdx.x; l < a.g.npts; l += (int64_t)gridDim.x * RED_THREADS)
-    red_point<R>(a, l, q);
-  __shared__ double sh[RED_THREADS];
-  for (int i = 0; i < a.nq; i++) {
-    sh[threadIdx.x] = q[i];
-    __syncthreads();
-    for (int s = RED_THREADS / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[blockIdx.x * RED_MAXQ + i] = sh[0];
-    __syncthreads();
+  const int64_t stride = (int64_t)gridDim.x * RED_THREADS;
+  for (int64_t l0 = blockIdx.x * (int64_t)RED_THREADS + threadIdx.x; l0 < a.g.npts; l0 += RED_AHEAD * stride) {
+    RedIn<R, MODE> in[RED_AHEAD];
+    #pragma unroll
+    for (int u = 0; u < RED_AHEAD; u++)
+      if (l0 + u * stride < a.g.npts) red_fetch<R, MODE>(a, l0 + u * stride, in[u]);
+    #pragma unroll
+    for (int u = 0; u < RED_AHEAD; u++)
+      if (l0 + u * stride < a.g.npts) red_point<R, MODE>(a, l0 + u * stride, in[u], q);
   }
+  red_finish<RED_THREADS>(q, a.nq, partial, count, out);
 }
 
 

@@ -46,15 +46,6 @@ __global__ void scale_kernel(double2 *y, double f, int64_t n) {
   }
 }
 
-__global__ void reduce_final(const double *partial, int nblocks, int nq, double *out) {
-  const int i = threadIdx.x;
-  if (i < nq) {
-    double s = 0;
-    for (int b = 0; b < nblocks; b++) s += partial[b * RED_MAXQ + i];
-    out[i] = s;
-  }
-}
-
 // ------------------------------------------------------------ Sobolev run on the device
 // Scalars of the descent kept in device memory, so that a chunk of iterations
 // runs (as a CUDA graph) without host round trips.  Per component: q = the two
@@ -72,18 +63,6 @@ struct SobDev {
   int stop;             // its residual is <= eps
   int done;             // no further iteration updates psi
 };
-
-// G -= (Re<psi,G> / Re<psi,psi_sob>) psi_sob  (Project_Sobolev_Gradient)
-__global__ void sob_proj_kernel(double2 *g, const double2 *ps, const SobDev *d, int comp, int64_t n) {
-  const double fak = d->q[comp][0] / d->q[comp][1];
-  for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < n; l += (int64_t)gridDim.x * blockDim.x) {
-    double2 v = g[l];
-    const double2 u = ps[l];
-    v.x -= fak * u.x;
-    v.y -= fak * u.y;
-    g[l] = v;
-  }
-}
 
 // Residual, particle numbers and the renormalisation decision of one
 // iteration (Compute_res, Renormalize_All_Psi), and whether it updates psi.

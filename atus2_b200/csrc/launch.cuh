@@ -234,7 +234,7 @@ static inline int launch_pass2_tma_t(atus_ctx *ctx, PassArgs &a, int axis) {
   }
   a.ntiles = ntiles;
   a.ncomp_grid = ctx->ncomp;
-  a.err = ctx->err_dev;
+  a.err = ctx->err_word;
   a.wait_limit = ctx->wait_limit;
   a.drop_copies = ctx->drop_copies;
   const int64_t work = ntiles * ctx->ncomp;
@@ -252,7 +252,7 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   // iteration) the TMA-fed passes measured no faster (0.253 vs 0.252 ms per
   // iteration)
   if constexpr (STRIDED && N == 256 && TC == 1 && (MODE == M2_FWD || MODE == M2_INV || MODE == M2_KIN)) {
-    if (ctx->use_tma && a.per_comp && ctx->err_dev && ctx->npts / ctx->n[axis] >= 2) {
+    if (ctx->use_tma && a.per_comp && ctx->err_word && ctx->npts / ctx->n[axis] >= 2) {
       const int r = launch_pass2_tma_t<R, N, MODE>(ctx, a, axis);
       if (r != ATUS_E_UNSUPPORTED) return r;
     }

@@ -145,20 +145,7 @@ __device__ __forceinline__ void p2_rabi(const PassArgs &a, int ci, const int *p0
       const int t = (idx + sh) % a.n[ax];
       k[ax] = a.dk[ax] * (double)(t - sh);
     }
-    int jb = 0;
-    for (int q = 0; q < a.rabi_n; q++) {
-      double dd = 0;
-      #pragma unroll
-      for (int ax = 0; ax < 3; ax++) {
-        const double d = a.rabi_k0[ci * a.rabi_n + q][ax] - k[ax];
-        dd += d * d;
-      }
-      if (sqrt(dd) < a.rabi_thr) {
-        rq[ci * a.rabi_n + jb] += den;
-        continue;
-      }
-      jb++;
-    }
+    red_balls<3>(&a.rabi_k0[ci * a.rabi_n], a.rabi_n, a.rabi_thr, k, den, &rq[ci * a.rabi_n]);
   }
 }
 
@@ -417,20 +404,9 @@ __global__ void __launch_bounds__(Tile2<R>::NT, Tile2<R>::MINB) pass2_kernel(Pas
     p2_item<R, N, TC, MODE, STRIDED>(a, tile_geo<Cfg::B, N>(a, w), smem_raw, kt_shared, s_om, s_ec, s_es, rq);
   }
   if constexpr (MODE == M2_KIN_RABI) {
-    // per-CTA sums in a fixed tree (the tiles of a CTA are fixed by the grid
-    // size, so the result does not depend on scheduling)
-    __syncthreads();
-    double *sh = reinterpret_cast<double *>(smem_raw);
-    for (int q = 0; q < a.rabi_ncomp * a.rabi_n; q++) {
-      sh[threadIdx.x] = rq[q];
-      __syncthreads();
-      for (int s = Cfg::NT / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) a.rabi_partial[blockIdx.x * RED_MAXQ + q] = sh[0];
-      __syncthreads();
-    }
+    // the tiles of a CTA are fixed by the grid size, so the result does not
+    // depend on scheduling
+    red_finish<Cfg::NT>(rq, a.rabi_ncomp * a.rabi_n, a.rabi_partial, a.rabi_count, a.rabi_out);
   }
 }
 

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(Tile2<R>::NT, 3) pass2_tma_kernel(PassArgs a, 
     bool ok = false;
     for (long it = 0; it < a.wait_limit && !ok; it++) ok = mbar_try_wait(mb, parity);
     if (!__syncthreads_and(ok)) {
-      if (tid == 0 && a.err) atomicOr(a.err, 1);
+      if (tid == 0 && a.err) *(volatile int *)a.err = 1;
       break;
     }
     parity ^= 1;
