@@ -453,8 +453,6 @@ static int launch_reduce(atus_ctx *ctx, RedArgs &a, double *dst) {
     case RED_RABI: ATUS_RED(double, RED_RABI); break;
     case RED_DOT2: ATUS_RED(double, RED_DOT2); break;  // the Sobolev descent runs in FP64
     case RED_MU: ATUS_RED(double, RED_MU); break;
-    case RED_PROJ: ATUS_RED(double, RED_PROJ); break;
-    case RED_SOBG: ATUS_RED(double, RED_SOBG); break;
     default: return fail(ctx, ATUS_E_ARG, "unknown reduction");
   }
 #undef ATUS_RED
@@ -585,7 +583,7 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
   if (ok) ok = cudaMalloc(&ctx->scratch, 16 * ctx->npts) == cudaSuccess;
   if (ok) ok = cudaMallocHost(&ctx->err_word, sizeof(int)) == cudaSuccess;
   if (ok) *ctx->err_word = 0;
-  if (ok) ok = cudaMalloc(&ctx->red_partial, sizeof(double) * RED_BLOCKS * RED_MAXQ) == cudaSuccess;
+  if (ok) ok = cudaMalloc(&ctx->red_partial, sizeof(double) * RED_ROWS * RED_MAXQ) == cudaSuccess;
   if (ok)
     ok = cudaMalloc(&ctx->red_count, sizeof(unsigned)) == cudaSuccess &&
          cudaMemset(ctx->red_count, 0, sizeof(unsigned)) == cudaSuccess;
@@ -1331,13 +1329,15 @@ int atus_rabi_integrals_comp(atus_ctx *ctx, int comp, const double *k0, int n, d
 
 // ------------------------------------------------------------------ Sobolev gradient
 // Real k-space filter of an FP64 buffer over all axes: forward transforms,
-// filter inside the axis-0 pass, inverse transforms.
-static int sob_filter_n(atus_ctx *ctx, void *const *bufs, int nb, int mode, double alpha) {
+// filter inside the axis-0 pass, inverse transforms.  inner: without the
+// contiguous axis (2D and 3D), whose passes the caller runs.
+static int sob_filter_n(atus_ctx *ctx, void *const *bufs, int nb, int mode, double alpha, bool inner) {
   if (ctx->fs_tw) return fail(ctx, ATUS_E_UNSUPPORTED, "the Sobolev filter takes 1D grids of at most 8192 points");
   const int saved = ctx->prec;
   ctx->prec = ATUS_PREC_FP64;
   int r = ATUS_OK;
-  for (int ax = ctx->dim - 1; ax >= 1 && r == ATUS_OK; ax--) r = run_pass(ctx, ax, T_FWD, OP_NONE, T_NONE, nullptr, 0, bufs, nb);
+  const int top = ctx->dim - (inner ? 1 : 0);
+  for (int ax = top - 1; ax >= 1 && r == ATUS_OK; ax--) r = run_pass(ctx, ax, T_FWD, OP_NONE, T_NONE, nullptr, 0, bufs, nb);
   if (r == ATUS_OK) {
     PassArgs a;
     memset(&a, 0, sizeof(a));
@@ -1350,19 +1350,22 @@ static int sob_filter_n(atus_ctx *ctx, void *const *bufs, int nb, int mode, doub
     a.filt_mode = mode;
     a.filt_alpha = alpha;
     a.filt_scale = round_trip_scale(ctx);
+    double k2 = 0;
+    for (int ax = 0; ax < ctx->dim; ax++) k2 += pow(0.5 * ctx->dk[ax] * (double)ctx->n[ax], 2);
+    a.filt_batch = alpha >= 0 && alpha * k2 < 1e60;
     const int saved_nc = ctx->ncomp;
     ctx->ncomp = nb;
     r = dispatch_pass(ctx, a, 0, 1);
     ctx->ncomp = saved_nc;
   }
-  for (int ax = 1; ax < ctx->dim && r == ATUS_OK; ax++) r = run_pass(ctx, ax, T_INV, OP_NONE, T_NONE, nullptr, 0, bufs, nb);
+  for (int ax = 1; ax < top && r == ATUS_OK; ax++) r = run_pass(ctx, ax, T_INV, OP_NONE, T_NONE, nullptr, 0, bufs, nb);
   ctx->prec = saved;
   return r;
 }
 
 static int sob_filter(atus_ctx *ctx, void *buf, int mode, double alpha) {
   void *f[1] = {buf};
-  return sob_filter_n(ctx, f, 1, mode, alpha);
+  return sob_filter_n(ctx, f, 1, mode, alpha, false);
 }
 
 static int sob_norms(atus_ctx *ctx, double *N) {
@@ -1456,18 +1459,60 @@ static int sob_iterate_once(atus_ctx *ctx, double *res_out, double *N_out) {
   return ATUS_OK;
 }
 
-// One iteration of sob_iterate_once with every scalar in device memory:
-// the same kernels and reductions in the same order; psi changes only in an
+// First or last pass of a Sobolev iteration along the contiguous axis (modes
+// M2_FWD_SOB / M2_INV_SOB of component i) over bufs = {S psi, S(W psi)}.
+// ATUS_E_UNSUPPORTED, nothing launched, where the register-staged pass has no
+// instantiation (1D, contiguous axis outside 32..256 points).
+static int sob_end_pass(atus_ctx *ctx, void *const *bufs, int i, int mode) {
+  const int64_t nl = ctx->n[ctx->dim - 1];
+  if (!ctx->use_pass2 || ctx->dim < 2 || nl < 32 || nl > 256) return ATUS_E_UNSUPPORTED;
+  PassArgs a;
+  memset(&a, 0, sizeof(a));
+  a.psi[0] = bufs[0];
+  a.psi[1] = bufs[1];
+  a.per_comp = 1;
+  a.nc = 1;
+  for (int c = 0; c < ctx->ncomp; c++) {
+    a.sob_psi[c] = (const double2 *)ctx->psi[c];
+    a.sob_gs[c] = ctx->gs[i * MAXC + c];
+  }
+  a.sob_comp = i;
+  a.sob_ncomp = ctx->ncomp;
+  a.nl.V[0] = ctx->V[i];
+  a.rabi_partial = ctx->red_partial;
+  a.rabi_count = ctx->red_count;
+  a.rabi_out = ((SobDev *)ctx->sob_dev)->q[i];
+  const int saved = ctx->ncomp;
+  ctx->ncomp = 2;  // items: the two buffers
+  const int r = launch_pass2_d_sob(ctx, a, ctx->dim - 1, mode);
+  ctx->ncomp = saved;
+  return r;
+}
+
+// One iteration with every scalar in device memory; psi changes only in an
 // active iteration (not yet converged, below max_iter).
+//
+// The reference's gradient S(-Lap psi + W psi), W = V + sum_j g_ij |psi_j|^2,
+// S = 1/(1 + alpha k^2), is taken as S(W psi) + psi - S psi: S alpha k^2 = 1 - S,
+// so the Laplacian's transforms drop out (two filters per component instead of
+// three; the same quantities up to rounding).  S psi and S(W psi) go through
+// the same passes; the first reads psi and forms W psi on the way in, the last
+// sums their products with psi on the way out, and sob_step_kernel does the
+// rest, so an iteration in 3D is six launches and 24 field sweeps (128^3: 193
+// -> 167 us against separate assembly, projection, norm and update passes).
 static int sob_iterate_dev(atus_ctx *ctx) {
-  // The reference's gradient S(-Lap psi + W psi), W = V + sum_j g_ij |psi_j|^2,
-  // S = 1/(1 + alpha k^2), taken as S(W psi) + psi - S psi: S alpha k^2 = 1 - S,
-  // so the Laplacian's transforms drop out (two filters per component instead
-  // of three; the same quantities up to rounding).
   const int n = ctx->ncomp;
   const int blocks = grid_blocks(ctx->npts, 256);
   SobDev *d = (SobDev *)ctx->sob_dev;
-  for (int i = 0; i < n; i++) {  // S psi (Compute_Sobolev_Psi) and S(W psi), filtered together
+  for (int i = 0; i < n; i++) {
+    void *bufs[2] = {ctx->sob_psi[i], ctx->sob_grad[i]};
+    int r = sob_end_pass(ctx, bufs, i, M2_FWD_SOB);
+    if (r == ATUS_OK) {
+      RUN(sob_filter_n(ctx, bufs, 2, FILT_SOBOLEV, ctx->sob_alpha[i], true));
+      RUN(sob_end_pass(ctx, bufs, i, M2_INV_SOB));
+      continue;
+    }
+    if (r != ATUS_E_UNSUPPORTED) return r;
     SobArgs a;  // W psi into the gradient buffer, psi into the Sobolev buffer, one pass
     memset(&a, 0, sizeof(a));
     for (int j = 0; j < MAXC; j++) a.psi[j] = (const double2 *)ctx->psi[j];
@@ -1481,36 +1526,24 @@ static int sob_iterate_dev(atus_ctx *ctx) {
     a.npts = ctx->npts;
     sob_assemble_kernel<<<blocks, 256, 0, ctx->stream>>>(a);
     LAUNCHED(ctx);
-    void *bufs[2] = {ctx->sob_psi[i], ctx->sob_grad[i]};
-    RUN(sob_filter_n(ctx, bufs, 2, FILT_SOBOLEV, ctx->sob_alpha[i]));
+    RUN(sob_filter_n(ctx, bufs, 2, FILT_SOBOLEV, ctx->sob_alpha[i], false));
+    RedArgs q;
+    memset(&q, 0, sizeof(q));
+    q.mode = RED_DOT2;
+    q.nq = 3;
+    q.a = ctx->psi[i];
+    q.b = ctx->sob_grad[i];  // <psi, S(W psi)>
+    q.c = ctx->sob_psi[i];
+    RUN(launch_reduce(ctx, q, d->q[i]));
   }
   for (int i = 0; i < n; i++) {
-    RedArgs r;  // G = S(W psi) + psi - S psi, the projection's two products and <psi, psi> in one pass
-    memset(&r, 0, sizeof(r));
-    r.mode = RED_SOBG;
-    r.nq = 3;
-    r.a = ctx->psi[i];
-    r.c = ctx->sob_psi[i];
-    r.w = (double2 *)ctx->sob_grad[i];
-    RUN(launch_reduce(ctx, r, d->q[i]));
-    RedArgs p;  // Project_Sobolev_Gradient fused with the norm of the projected gradient
-    memset(&p, 0, sizeof(p));
-    p.mode = RED_PROJ;
-    p.nq = 1;
-    p.w = (double2 *)ctx->sob_grad[i];
-    p.c = ctx->sob_psi[i];
-    p.fq = d->q[i];
-    RUN(launch_reduce(ctx, p, &d->g2[i]));
-  }
-  sob_scalars_kernel<<<1, 1, 0, ctx->stream>>>(d, ctx->ar, n);
-  LAUNCHED(ctx);
-  for (int i = 0; i < n; i++) {
-    sob_update_kernel<<<blocks, 256, 0, ctx->stream>>>((double2 *)ctx->psi[i], (const double2 *)ctx->sob_grad[i],
-                                                      ctx->stepsize, d, i, ctx->npts);
+    const int64_t per = (int64_t)RED_THREADS * RED_AHEAD;
+    const int64_t want = (ctx->npts + per - 1) / per;
+    sob_step_kernel<<<(unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS), RED_THREADS, 0, ctx->stream>>>(
+        (double2 *)ctx->psi[i], (const double2 *)ctx->sob_grad[i], (const double2 *)ctx->sob_psi[i], ctx->stepsize, d,
+        i, n, i == n - 1, ctx->ar, ctx->npts, ctx->red_partial, ctx->red_count);
     LAUNCHED(ctx);
   }
-  sob_commit_kernel<<<1, 1, 0, ctx->stream>>>(d);
-  LAUNCHED(ctx);
   return ATUS_OK;
 }
 

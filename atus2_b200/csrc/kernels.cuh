@@ -45,7 +45,10 @@ enum { K_NL = 0, K_NL_IF = 1, K_BRAGG = 2, K_DBRAGG = 3, K_NL_IF2 = 4, K_BRAGG_D
 // M2_KIN_RABI: M2_KIN that also sums |psi^(k)|^2 over the Rabi balls of the
 // requested components while every axis is in k-space (the last kinetic pass
 // of a block); a separate instantiation, so M2_KIN keeps its registers.
-enum { M2_FWD = 0, M2_INV = 1, M2_KIN = 2, M2_NL = 3, M2_KIN_RABI = 4 };
+// M2_FWD_SOB, M2_INV_SOB: the first and the last pass of a Sobolev iteration
+// (the transform of psi and W psi straight from psi; the inverse transform of
+// S psi and S(W psi) with their products with psi).
+enum { M2_FWD = 0, M2_INV = 1, M2_KIN = 2, M2_NL = 3, M2_KIN_RABI = 4, M2_FWD_SOB = 5, M2_INV_SOB = 6 };
 
 struct LaserD {
   double beta0, DeltaL[MAXC], Amp0, laser_k0, laser_dk0, laser_domh0, phase0, chirp_rate0, chirp;
@@ -103,6 +106,7 @@ struct PassArgs {
   // 1/(1 + alpha k^2) or -alpha k^2, times the transform scale.
   int filt_mode;
   double filt_alpha, filt_scale;
+  int filt_batch;  // 1 + alpha k^2 of four points multiplies without overflow
   double dk[3];
   int n[3];
   // M2_KIN_RABI: balls k0[c * rabi_n + m] (m < rabi_n) of component
@@ -114,6 +118,11 @@ struct PassArgs {
   double rabi_k0[8][3];
   double *rabi_partial, *rabi_out;
   unsigned *rabi_count;
+  // M2_FWD_SOB / M2_INV_SOB: the components' fields, the one this pass works
+  // for and its interaction row (potential: nl.V[0]); sums to rabi_out
+  const double2 *sob_psi[MAXC];
+  int sob_comp, sob_ncomp;
+  double sob_gs[MAXC];
   int *err;  // error word, mapped host memory (a bounded wait that ran out sets it)
   long wait_limit;       // try_wait rounds before a TMA tile counts as lost
   int drop_copies;       // issue no tile copies, so every wait runs out (error-path tests; 0)
@@ -794,7 +803,7 @@ __global__ void __launch_bounds__(Tile<R>::NT, Tile<R>::MINB) pass_kernel(PassAr
           double phi = 0;
           #pragma unroll
           for (int ax = 0; ax < 3; ax++) {
-            const int t = (ijk[ax] + a.n[ax] / 2) % a.n[ax];
+            const int t = (ijk[ax] + a.n[ax] / 2) & (a.n[ax] - 1);
             const double k = a.dk[ax] * (double)(t - a.n[ax] / 2);
             phi += (k * a.filt_alpha) * k;
           }
@@ -1036,9 +1045,10 @@ struct SobArgs {
 // ------------------------------------------------------------ reductions
 // Quantities per mode (all FP64 accumulations, fixed order per thread, fixed
 // tree per block, block sums in a fixed order).
-enum { RED_NORM = 0, RED_POS = 1, RED_MOM = 2, RED_RABI = 3, RED_DOT2 = 4, RED_MU = 5, RED_PROJ = 6, RED_SOBG = 7 };
+enum { RED_NORM = 0, RED_POS = 1, RED_MOM = 2, RED_RABI = 3, RED_DOT2 = 4, RED_MU = 5 };
 constexpr int RED_MAXQ = 8;
 constexpr int RED_BLOCKS = 592;  // 4 x 148 SMs
+constexpr int RED_ROWS = 1184;   // rows of block sums (the passes that sum run up to 8 CTAs per SM)
 constexpr int RED_THREADS = 256;
 
 struct RedArgs {
@@ -1055,9 +1065,6 @@ struct RedArgs {
   const void *psi_all[MAXC];
   int ncomp, comp;
   double gs[MAXC * MAXC];
-  // projection: w <- w - (fq[0] / fq[1]) c, then |w|^2 (FP64 fields)
-  double2 *w;
-  const double *fq;
 };
 
 // |psi^|^2 = den at wavenumber k into the Rabi bins, with the bin rule of
@@ -1098,10 +1105,8 @@ template <typename R, int MODE> struct RedIn {
 template <typename R, int MODE>
 __device__ __forceinline__ void red_fetch(const RedArgs &a, int64_t l, RedIn<R, MODE> &in) {
   using C = cplx<R>;
-  if constexpr (MODE == RED_SOBG || MODE == RED_PROJ) in.b = ((const C *)a.w)[l];
+  in.v = ((const C *)a.a)[l];
   if constexpr (MODE == RED_DOT2 || MODE == RED_MU) in.b = ((const C *)a.b)[l];
-  if constexpr (MODE != RED_PROJ) in.v = ((const C *)a.a)[l];
-  if constexpr (MODE == RED_SOBG || MODE == RED_PROJ) in.c = ((const C *)a.c)[l];
   if constexpr (MODE == RED_DOT2) in.c = a.c ? ((const C *)a.c)[l] : mk<R>(0, 0);
   if constexpr (MODE == RED_MU) in.pot = a.V ? a.V[l] : 0.0;
 }
@@ -1109,62 +1114,40 @@ __device__ __forceinline__ void red_fetch(const RedArgs &a, int64_t l, RedIn<R, 
 template <typename R, int MODE>
 __device__ __forceinline__ void red_point(const RedArgs &a, int64_t l, const RedIn<R, MODE> &in, double *q) {
   using C = cplx<R>;
-  if constexpr (MODE == RED_SOBG) {
-    // w = S(W psi) becomes the Sobolev gradient S(-Lap psi + W psi) =
-    // S(W psi) + psi - S psi (S = 1/(1 + alpha k^2), so S alpha k^2 = 1 - S),
-    // then Re<psi, G>, Re<psi, S psi>, <psi, psi>
-    const double2 p = to_d<R>(in.v), ps = to_d<R>(in.c);
-    double2 g = to_d<R>(in.b);
-    g.x += p.x - ps.x;
-    g.y += p.y - ps.y;
-    a.w[l] = g;
-    q[0] += p.x * g.x + p.y * g.y;
-    q[1] += p.x * ps.x + p.y * ps.y;
-    q[2] += p.x * p.x + p.y * p.y;
-  } else if constexpr (MODE == RED_PROJ) {  // Project_Sobolev_Gradient and the norm of the result in one pass
-    const double fak = a.fq[0] / a.fq[1];
-    double2 v = to_d<R>(in.b);
-    const double2 u = to_d<R>(in.c);
-    v.x -= fak * u.x;
-    v.y -= fak * u.y;
-    a.w[l] = v;
-    q[0] += v.x * v.x + v.y * v.y;
-  } else {
-    const C v = in.v;
-    const double den = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
-    if constexpr (MODE == RED_NORM) q[0] += den;
-    if constexpr (MODE == RED_POS || MODE == RED_MOM || MODE == RED_RABI) {
-      int ijk[3];
-      idx3(a.g, l, ijk[0], ijk[1], ijk[2]);
-      double x[3];
+  const C v = in.v;
+  const double den = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
+  if constexpr (MODE == RED_NORM) q[0] += den;
+  if constexpr (MODE == RED_POS || MODE == RED_MOM || MODE == RED_RABI) {
+    int ijk[3];
+    idx3(a.g, l, ijk[0], ijk[1], ijk[2]);
+    double x[3];
+    #pragma unroll
+    for (int ax = 0; ax < 3; ax++) {  // axis lengths are powers of two (unused axes: one point)
+      const int t = (MODE == RED_POS) ? ijk[ax] : ((ijk[ax] + a.shift[ax]) & (a.n[ax] - 1));
+      x[ax] = (double)(t - a.shift[ax]) * ((MODE == RED_POS) ? a.d[ax] : a.dk[ax]);
+    }
+    if constexpr (MODE != RED_RABI) {
       #pragma unroll
-      for (int ax = 0; ax < 3; ax++) {  // axis lengths are powers of two (unused axes: one point)
-        const int t = (MODE == RED_POS) ? ijk[ax] : ((ijk[ax] + a.shift[ax]) & (a.n[ax] - 1));
-        x[ax] = (double)(t - a.shift[ax]) * ((MODE == RED_POS) ? a.d[ax] : a.dk[ax]);
-      }
-      if constexpr (MODE != RED_RABI) {
-        #pragma unroll
-        for (int ax = 0; ax < 3; ax++) q[ax] += x[ax] * den;
-      } else {
-        red_balls<3>(a.k0, a.nq, a.thr, x, den, q);
+      for (int ax = 0; ax < 3; ax++) q[ax] += x[ax] * den;
+    } else {
+      red_balls<3>(a.k0, a.nq, a.thr, x, den, q);
+    }
+  }
+  if constexpr (MODE == RED_DOT2) {  // Re<a,b>, Re<a,c>, <a,a>
+    q[0] += (double)v.x * (double)in.b.x + (double)v.y * (double)in.b.y;
+    q[1] += (double)v.x * (double)in.c.x + (double)v.y * (double)in.c.y;
+    q[2] += den;
+  }
+  if constexpr (MODE == RED_MU) {  // a = psi_i, b = Lap psi_i
+    double nl = 0;
+    #pragma unroll
+    for (int j = 0; j < MAXC; j++) {
+      if (j < a.ncomp) {
+        const C pj = ((const C *)a.psi_all[j])[l];
+        nl += a.gs[a.comp * MAXC + j] * ((double)pj.x * (double)pj.x + (double)pj.y * (double)pj.y);
       }
     }
-    if constexpr (MODE == RED_DOT2) {  // Re<a,b>, Re<a,c> (and <a,a> when nq is 3)
-      q[0] += (double)v.x * (double)in.b.x + (double)v.y * (double)in.b.y;
-      q[1] += (double)v.x * (double)in.c.x + (double)v.y * (double)in.c.y;
-      q[2] += den;
-    }
-    if constexpr (MODE == RED_MU) {  // a = psi_i, b = Lap psi_i
-      double nl = 0;
-      #pragma unroll
-      for (int j = 0; j < MAXC; j++) {
-        if (j < a.ncomp) {
-          const C pj = ((const C *)a.psi_all[j])[l];
-          nl += a.gs[a.comp * MAXC + j] * ((double)pj.x * (double)pj.x + (double)pj.y * (double)pj.y);
-        }
-      }
-      q[0] += -((double)v.x * (double)in.b.x + (double)v.y * (double)in.b.y) + (in.pot + nl) * den;
-    }
+    q[0] += -((double)v.x * (double)in.b.x + (double)v.y * (double)in.b.y) + (in.pot + nl) * den;
   }
 }
 
@@ -1175,8 +1158,9 @@ __device__ __forceinline__ void red_point(const RedArgs &a, int64_t l, const Red
 // Measured against a second launch whose one thread per quantity added 592
 // rows: that launch took 25-29 us by itself, of 50 us for a reduction over
 // 2^21 points.
+// Returns true in every thread of that last block.
 template <int NT>
-__device__ __forceinline__ void red_finish(double *q, int nq, double *partial, unsigned *count, double *out) {
+__device__ __forceinline__ bool red_finish(double *q, int nq, double *partial, unsigned *count, double *out) {
   static_assert(NT % 32 == 0 && NT >= 4 * RED_MAXQ, "whole warps, several rows per quantity");
   constexpr int NW = NT / 32, ROWS = NT / RED_MAXQ;
   __shared__ double sh[NT];
@@ -1203,7 +1187,7 @@ __device__ __forceinline__ void red_finish(double *q, int nq, double *partial, u
   __syncthreads();
   if (tid == 0) last = (atomicAdd(count, 1u) == gridDim.x - 1);
   __syncthreads();
-  if (!last) return;
+  if (!last) return false;
   __threadfence();
   const int i = tid % RED_MAXQ, r0 = tid / RED_MAXQ;
   double v = 0;
@@ -1219,6 +1203,7 @@ __device__ __forceinline__ void red_finish(double *q, int nq, double *partial, u
     out[tid] = v;
   }
   if (tid == 0) *count = 0;
+  return true;
 }
 
 // Points a thread loads before it uses the first: with 32 warps on an SM

@@ -299,7 +299,7 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   const int64_t work = a.per_comp ? ntiles * ctx->ncomp : ntiles;
   const int64_t slots = (int64_t)nsm * resident;
   unsigned grid = (unsigned)(work < slots ? work : slots);
-  if (MODE == M2_KIN_RABI && grid > RED_BLOCKS) grid = RED_BLOCKS;  // one partial row per CTA
+  if ((MODE == M2_KIN_RABI || MODE == M2_INV_SOB) && grid > RED_ROWS) grid = RED_ROWS;  // one row of sums per CTA
   pass2_kernel<R, N, TC, MODE, STRIDED><<<grid, Cfg::NT, smem, ctx->stream>>>(a);
   LAUNCHED(ctx);
   return ATUS_OK;
@@ -364,7 +364,7 @@ static inline int launch_pass2_n(atus_ctx *ctx, PassArgs &a, int axis) {
     case 256: return launch_pass2_t<R, 256, TC, MODE, STRIDED>(ctx, a, axis);
     default: break;
   }
-  if constexpr (MODE != M2_KIN_RABI) {
+  if constexpr (MODE != M2_KIN_RABI && MODE != M2_FWD_SOB && MODE != M2_INV_SOB) {
     switch (ctx->n[axis]) {
       case 512: return launch_pass3_t<R, 512, TC, MODE, STRIDED>(ctx, a, axis);
       case 1024: return launch_pass3_t<R, 1024, TC, MODE, STRIDED>(ctx, a, axis);

@@ -27,3 +27,6 @@ int launch_pass2_d_kr(atus_ctx *ctx, PassArgs &a, int axis);
 int launch_pass2_f_kr(atus_ctx *ctx, PassArgs &a, int axis);
 int launch_pass2_d_nl(atus_ctx *ctx, PassArgs &a, int axis, int tc);
 int launch_pass2_f_nl(atus_ctx *ctx, PassArgs &a, int axis, int tc);
+// _sob: first (M2_FWD_SOB) and last (M2_INV_SOB) pass of a Sobolev iteration,
+// along the contiguous axis (32..256 points)
+int launch_pass2_d_sob(atus_ctx *ctx, PassArgs &a, int axis, int mode);

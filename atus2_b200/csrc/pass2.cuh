@@ -28,6 +28,11 @@ template <typename R> struct Tile2;
 template <> struct Tile2<double> { static constexpr int E = 2048, NT = 128, MINB = 5; };
 template <> struct Tile2<float> { static constexpr int E = 4096, NT = 256, MINB = 3; };
 
+// CTAs per SM the register budget is sized for: the passes at the ends of a
+// Sobolev iteration hold a thread's 16 potential values beside its 16 points.
+template <typename R, int MODE>
+constexpr int p2_minb = (MODE == M2_FWD_SOB || MODE == M2_INV_SOB) ? 4 : Tile2<R>::MINB;
+
 template <typename R, int N, int TC>
 struct P2Cfg {
   static constexpr int R2 = N / 16;        // stage-2 radix
@@ -149,6 +154,19 @@ __device__ __forceinline__ void p2_rabi(const PassArgs &a, int ci, const int *p0
   }
 }
 
+// sum_j g_j |psi_j|^2 at grid index l (several components).
+__device__ __forceinline__ double sob_interaction(const PassArgs &a, int64_t l) {
+  double nl = 0;
+  #pragma unroll
+  for (int c = 0; c < MAXC; c++) {
+    if (c < a.sob_ncomp) {
+      const double2 p = a.sob_psi[c][l];
+      nl += a.sob_gs[c] * (p.x * p.x + p.y * p.y);
+    }
+  }
+  return nl;
+}
+
 // After-load hook of p2_item (the TMA kernel refills the tile buffer there).
 struct P2NoHook {
   __device__ __forceinline__ void operator()() const {}
@@ -219,15 +237,66 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
     #pragma unroll
     for (int r = 0; r < 16; r++) v[r] = p2_tile_at<R, B>(tile, j + R2 * r, b);
     hook();
+  } else if constexpr (MODE == M2_FWD_SOB) {
+    // item component 0: psi, 1: W psi, W = V + sum_j g_j |psi_j|^2
+    const double2 *const own = pick(a.sob_psi, a.sob_comp) + lb + (int64_t)j * a.sa;
+    const double *const Vp = a.nl.V[0];
+    #pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = live ? own[r * step] : mk<R>(0, 0);
+    if (live && g.comp0 == 1) {
+      #pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const int64_t l = lb + (int64_t)(j + R2 * r) * a.sa;
+        double W = Vp ? __ldg(&Vp[l]) : 0.0;
+        W += a.sob_ncomp == 1 ? a.sob_gs[0] * (v[r].x * v[r].x + v[r].y * v[r].y) : sob_interaction(a, l);
+        v[r].x *= W;
+        v[r].y *= W;
+      }
+    }
   } else {
     #pragma unroll
     for (int r = 0; r < 16; r++) v[r] = live ? src[r * step] : mk<R>(0, 0);
   }
 
-  if constexpr (MODE == M2_FWD) {
+  if constexpr (MODE == M2_FWD || MODE == M2_FWD_SOB) {
     p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
   } else if constexpr (MODE == M2_INV) {
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
+  } else if constexpr (MODE == M2_INV_SOB) {
+    p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
+    // Item component 0 (v = S psi) takes every product of the iteration:
+    // rq = <S psi, W psi> (= <psi, S(W psi)>, S being self-adjoint),
+    // <psi, S psi>, <psi, psi>.  psi arrives in the pencil's exchange rows by
+    // cp.async, all 16 points of a thread in flight without registers (two
+    // 128^3 fields: 43 us; loads into registers, four at a time, 52 us; the
+    // plain inverse pass and a reduction over three fields 19 + 22 us plus a
+    // launch, and a sweep that forms the gradient).
+    if (g.comp0 == 0) {
+      const double2 *const own = pick(a.sob_psi, a.sob_comp) + lb + (int64_t)j * a.sa;
+      const double *const Vp = a.nl.V[0];
+      __syncwarp();  // the pencil's stage-2 reads are done
+      #pragma unroll
+      for (int m = 0; m < 16; m++)
+        if (live) cp_async(&my[ex_at(j, m)], own + m * step, double2{});
+      cp_commit();
+      double W[16];
+      #pragma unroll
+      for (int m = 0; m < 16; m++) W[m] = (live && Vp) ? __ldg(&Vp[lb + (int64_t)(j + R2 * m) * a.sa]) : 0.0;
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      if (live) {
+        #pragma unroll
+        for (int m = 0; m < 16; m++) {
+          const double2 p = my[ex_at(j, m)];
+          const double pv = p.x * v[m].x + p.y * v[m].y, pp = p.x * p.x + p.y * p.y;
+          const double w = W[m] + (a.sob_ncomp == 1
+                                       ? a.sob_gs[0] * pp
+                                       : sob_interaction(a, lb + (int64_t)(j + R2 * m) * a.sa));
+          rq[0] += w * pv;
+          rq[1] += pv;
+          rq[2] += pp;
+        }
+      }
+    }
   } else if constexpr (MODE == M2_KIN || MODE == M2_KIN_RABI) {
     p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
     int p0[3];
@@ -272,20 +341,43 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         v[m] = from_d<R>(u);
       }
     } else if (a.op == OP_FILT) {
+      // alpha k^2 of the pencil's two fixed axes, and of the point's own
+      auto ak2 = [&](int ax, int ii) {
+        const int sh = a.n[ax] >> 1;  // lengths are powers of two
+        const double k = a.dk[ax] * (double)(((ii + sh) & (a.n[ax] - 1)) - sh);
+        return (k * a.filt_alpha) * k;
+      };
+      double rest = 0;
       #pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const int i = j + R2 * m;
-        double phi = 0;
+      for (int ax = 0; ax < 3; ax++)
+        if (ax != a.axis) rest += ak2(ax, p0[ax]);
+      if (a.filt_mode == FILT_SOBOLEV && a.filt_batch) {
+        // 1 / (1 + alpha k^2) of four points from one division (with the
+        // axis indices wrapped by masks instead of integer division: 46 ->
+        // 29 us for two 128^3 fields)
         #pragma unroll
-        for (int ax = 0; ax < 3; ax++) {
-          const int ii = (ax == a.axis) ? i : p0[ax];
-          const int t = (ii + a.n[ax] / 2) % a.n[ax];
-          const double k = a.dk[ax] * (double)(t - a.n[ax] / 2);
-          phi += (k * a.filt_alpha) * k;
+        for (int m0 = 0; m0 < 16; m0 += 4) {
+          double d[4];
+          #pragma unroll
+          for (int u = 0; u < 4; u++) d[u] = 1.0 + (ak2(a.axis, j + R2 * (m0 + u)) + rest);
+          const double d01 = d[0] * d[1], d23 = d[2] * d[3];
+          const double inv = a.filt_scale / (d01 * d23);
+          const double i01 = inv * d23, i23 = inv * d01;
+          const double f[4] = {i01 * d[1], i01 * d[0], i23 * d[3], i23 * d[2]};
+          #pragma unroll
+          for (int u = 0; u < 4; u++) {
+            v[m0 + u].x = (R)((double)v[m0 + u].x * f[u]);
+            v[m0 + u].y = (R)((double)v[m0 + u].y * f[u]);
+          }
         }
-        const double fk = (a.filt_mode == FILT_SOBOLEV ? 1.0 / (1.0 + phi) : -phi) * a.filt_scale;
-        v[m].x = (R)((double)v[m].x * fk);
-        v[m].y = (R)((double)v[m].y * fk);
+      } else {
+        #pragma unroll
+        for (int m = 0; m < 16; m++) {
+          const double phi = ak2(a.axis, j + R2 * m) + rest;
+          const double fk = (a.filt_mode == FILT_SOBOLEV ? 1.0 / (1.0 + phi) : -phi) * a.filt_scale;
+          v[m].x = (R)((double)v[m].x * fk);
+          v[m].y = (R)((double)v[m].y * fk);
+        }
       }
     }
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
@@ -389,24 +481,26 @@ __device__ __forceinline__ void p2_prefetch_l2(const PassArgs &a, const TileGeo 
 }
 
 template <typename R, int N, int TC, int MODE, bool STRIDED>
-__global__ void __launch_bounds__(Tile2<R>::NT, Tile2<R>::MINB) pass2_kernel(PassArgs a) {
+__global__ void __launch_bounds__(Tile2<R>::NT, p2_minb<R, MODE>) pass2_kernel(PassArgs a) {
   using Cfg = P2Cfg<R, N, TC>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_om[Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];
   const bool kt_shared = p2_setup<R, N, TC, MODE>(a, smem_raw);
   __syncthreads();  // twiddle rows and kinetic factors visible to every warp
   const int64_t W = a.per_comp ? a.ntiles * a.ncomp_grid : a.ntiles;
-  double rq[MODE == M2_KIN_RABI ? RED_MAXQ : 1];
+  constexpr bool SUMS = (MODE == M2_KIN_RABI || MODE == M2_INV_SOB);
+  double rq[SUMS ? RED_MAXQ : 1];
   #pragma unroll
-  for (int q = 0; q < (MODE == M2_KIN_RABI ? RED_MAXQ : 1); q++) rq[q] = 0.0;
+  for (int q = 0; q < (SUMS ? RED_MAXQ : 1); q++) rq[q] = 0.0;
   for (int64_t w = blockIdx.x; w < W; w += gridDim.x) {
     if (STRIDED && w + gridDim.x < W) p2_prefetch_l2<R, N, TC>(a, tile_geo<Cfg::B, N>(a, w + gridDim.x));
     p2_item<R, N, TC, MODE, STRIDED>(a, tile_geo<Cfg::B, N>(a, w), smem_raw, kt_shared, s_om, s_ec, s_es, rq);
   }
-  if constexpr (MODE == M2_KIN_RABI) {
+  if constexpr (SUMS) {
     // the tiles of a CTA are fixed by the grid size, so the result does not
     // depend on scheduling
-    red_finish<Cfg::NT>(rq, a.rabi_ncomp * a.rabi_n, a.rabi_partial, a.rabi_count, a.rabi_out);
+    red_finish<Cfg::NT>(rq, MODE == M2_INV_SOB ? 3 : a.rabi_ncomp * a.rabi_n, a.rabi_partial, a.rabi_count,
+                        a.rabi_out);
   }
 }
 

@@ -218,8 +218,8 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
         #pragma unroll
         for (int ax = 0; ax < 3; ax++) {
           const int ii = (ax == a.axis) ? i : p0[ax];
-          const int tt = (ii + a.n[ax] / 2) % a.n[ax];
-          const double k = a.dk[ax] * (double)(tt - a.n[ax] / 2);
+          const int sh = a.n[ax] >> 1;  // lengths are powers of two
+          const double k = a.dk[ax] * (double)(((ii + sh) & (a.n[ax] - 1)) - sh);
           phi += (k * a.filt_alpha) * k;
         }
         const double fk = (a.filt_mode == FILT_SOBOLEV ? 1.0 / (1.0 + phi) : -phi) * a.filt_scale;
