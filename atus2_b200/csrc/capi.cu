@@ -82,8 +82,11 @@ static int build_kinetic(atus_ctx *ctx) {
             const double k = ctx->dk[ax] * (double)wrapped(i, n);
             phi = (-ctx->dt) * ((k * ctx->alpha[c][ax]) * k);
           }
-          tab[i].x = (hf == 0) ? cos(0.5 * phi) : cos(phi);
-          tab[i].y = (hf == 0) ? sin(0.5 * phi) : sin(phi);
+          // a long 1D axis: wavenumber k1 + n1 k2 at k1 n2 + k2, where the
+          // four-step spectrum holds it
+          const int64_t at = (ctx->fs_tw && ax == 0) ? (i % ctx->fs_n1) * ctx->fs_n2 + i / ctx->fs_n1 : i;
+          tab[at].x = (hf == 0) ? cos(0.5 * phi) : cos(phi);
+          tab[at].y = (hf == 0) ? sin(0.5 * phi) : sin(phi);
         }
         if (!ctx->kt[hf][c][ax]) CK(cudaMalloc(&ctx->kt[hf][c][ax], sizeof(double2) * n));
         CK(cudaMemcpyAsync(ctx->kt[hf][c][ax], tab.data(), sizeof(double2) * n, cudaMemcpyHostToDevice, ctx->stream));
@@ -235,34 +238,22 @@ static int grid_blocks(int64_t n, int threads) {
 // (r' the transformed index), transform along c; element (k1, k2) then holds
 // X[k1 + n1 k2].  Inverse: the same steps backwards with conjugate twiddles.
 template <typename R>
-__global__ void fs_twiddle_kernel(void *psi, const double2 *tw, int64_t n2c, int64_t N, int conj_) {
+__global__ void fs_twiddle_kernel(void *psi, const double2 *tw, int64_t N, int conj_) {
   cplx<R> *p = static_cast<cplx<R> *>(psi);
   for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < N; l += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = l / n2c, c = l % n2c;
-    double2 w = tw[(r * c) % N];
+    double2 w = tw[l];
     if (conj_) w.y = -w.y;
     p[l] = from_d<R>(cmul(to_d<R>(p[l]), w));
   }
 }
 
-// Kinetic factor of the four-step spectrum: element (k1, k2) is wavenumber
-// index k1 + n1 k2 of the 1D table, with the transform scales applied as in
-// the passes: ((u s_f) K) s_b in FP64.
+// Kinetic factor of the four-step spectrum (the table is in its order), with
+// the transform scales applied as in the passes: ((u s_f) K) s_b in FP64.
 template <typename R>
-__global__ void fs_kin_kernel(void *psi, const double2 *kt, int64_t n1, int64_t n2c, double s_f, double s_b) {
+__global__ void fs_kin_kernel(void *psi, const double2 *kt, int64_t N, double s_f, double s_b) {
   cplx<R> *p = static_cast<cplx<R> *>(psi);
-  const int64_t N = n1 * n2c;
-  for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < N; l += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k1 = l / n2c, k2 = l % n2c;
-    const double2 K = kt[k1 + n1 * k2];
-    double2 u = to_d<R>(p[l]);
-    u.x *= s_f;
-    u.y *= s_f;
-    u = cmul(u, K);
-    u.x *= s_b;
-    u.y *= s_b;
-    p[l] = from_d<R>(u);
-  }
+  for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < N; l += (int64_t)gridDim.x * blockDim.x)
+    p[l] = kin_mul<R>(p[l], kt[l], s_f, s_b);
 }
 
 // Four-step spectrum <-> natural wavenumber order, FP64 buffers:
@@ -307,24 +298,49 @@ struct FsView {
 static int fs_twiddle(atus_ctx *ctx, void *const *f, int nf, int conj_, bool fp64) {
   for (int i = 0; i < nf; i++) {
     if (fp64)
-      fs_twiddle_kernel<double><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(f[i], ctx->fs_tw, ctx->fs_n2,
-                                                                                       ctx->npts, conj_);
+      fs_twiddle_kernel<double><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(f[i], ctx->fs_tw, ctx->npts, conj_);
     else
-      fs_twiddle_kernel<float><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(f[i], ctx->fs_tw, ctx->fs_n2,
-                                                                                      ctx->npts, conj_);
+      fs_twiddle_kernel<float><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(f[i], ctx->fs_tw, ctx->npts, conj_);
     LAUNCHED(ctx);
   }
   return ATUS_OK;
 }
 
+// One fused four-step pass (M2_FS_*) over nf fields; half: which kinetic
+// table.  ATUS_E_UNSUPPORTED, nothing launched, where a view axis is longer
+// than the register-staged passes (N >= 2^23) or tc > 2.
+static int fs_pass(atus_ctx *ctx, int mode, void *const *f, int nf, int half, const NLArgs *nl) {
+  if (!ctx->use_pass2 || ctx->fs_n2 > 2048 || (mode == M2_FS_NL && nf > 2)) return ATUS_E_UNSUPPORTED;
+  PassArgs a;
+  memset(&a, 0, sizeof(a));
+  for (int c = 0; c < nf; c++) a.psi[c] = f[c];
+  for (int c = 0; c < nf && c < ctx->ncomp; c++) a.kt[c][0] = ctx->kt[half ? 0 : 1][c][0];
+  a.per_comp = (mode != M2_FS_NL) ? 1 : 0;
+  a.nc = a.per_comp ? 1 : nf;
+  a.s_f = scale_fak(ctx->dim, ctx->d);
+  a.s_b = scale_fak(ctx->dim, ctx->dk);
+  a.fs_tw = ctx->fs_tw;
+  if (nl) a.nl = *nl;
+  FsView v(ctx);
+  const int saved = ctx->ncomp;
+  ctx->ncomp = nf;
+  const int r = (ctx->prec == ATUS_PREC_FP64) ? launch_fs_d(ctx, a, mode, nf) : launch_fs_f(ctx, a, mode, nf);
+  ctx->ncomp = saved;
+  return r;
+}
+
 // Unscaled forward / inverse transform of nf fields (four-step order in k).
 static int fs_forward(atus_ctx *ctx, void *const *f, int nf) {
   const bool fp64 = ctx->prec == ATUS_PREC_FP64;
-  {
-    FsView v(ctx);
-    RUN(run_pass(ctx, 0, T_FWD, OP_NONE, T_NONE, nullptr, 0, f, nf));
+  int r = fs_pass(ctx, M2_FS_FWD, f, nf, 0, nullptr);
+  if (r == ATUS_E_UNSUPPORTED) {
+    {
+      FsView v(ctx);
+      RUN(run_pass(ctx, 0, T_FWD, OP_NONE, T_NONE, nullptr, 0, f, nf));
+    }
+    r = fs_twiddle(ctx, f, nf, 0, fp64);
   }
-  RUN(fs_twiddle(ctx, f, nf, 0, fp64));
+  RUN(r);
   FsView v(ctx);
   return run_pass(ctx, 1, T_FWD, OP_NONE, T_NONE, nullptr, 0, f, nf);
 }
@@ -355,16 +371,21 @@ static int fs_reorder(atus_ctx *ctx, void *&buf, int to_natural) {
 // four-step transforms around the factor of each wavenumber).
 static int kinetic_pass(atus_ctx *ctx, int half) {
   if (ctx->fs_tw) {
+    int r = fs_pass(ctx, M2_FS_FWD, ctx->psi, ctx->ncomp, half, nullptr);
+    if (r == ATUS_OK) {
+      RUN(fs_pass(ctx, M2_FS_KIN, ctx->psi, ctx->ncomp, half, nullptr));
+      FsView v(ctx);
+      return run_pass(ctx, 0, T_INV, OP_NONE, T_NONE, nullptr, 0);
+    }
+    if (r != ATUS_E_UNSUPPORTED) return r;
     RUN(fs_forward(ctx, ctx->psi, ctx->ncomp));
     const double s_f = scale_fak(ctx->dim, ctx->d), s_b = scale_fak(ctx->dim, ctx->dk);
     for (int c = 0; c < ctx->ncomp; c++) {
       const double2 *kt = ctx->kt[half ? 0 : 1][c][0];
       if (ctx->prec == ATUS_PREC_FP64)
-        fs_kin_kernel<double><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(ctx->psi[c], kt, ctx->fs_n1,
-                                                                                    ctx->fs_n2, s_f, s_b);
+        fs_kin_kernel<double><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(ctx->psi[c], kt, ctx->npts, s_f, s_b);
       else
-        fs_kin_kernel<float><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(ctx->psi[c], kt, ctx->fs_n1,
-                                                                                   ctx->fs_n2, s_f, s_b);
+        fs_kin_kernel<float><<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>(ctx->psi[c], kt, ctx->npts, s_f, s_b);
       LAUNCHED(ctx);
     }
     return fs_inverse(ctx, ctx->psi, ctx->ncomp);
@@ -625,11 +646,16 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
     ctx->fs_n2 = ctx->n[0] / ctx->fs_n1;
     std::vector<double2> t(ctx->n[0]);
     const long double two_pi = 6.283185307179586476925286766559005768L;
+    std::vector<double2> w(ctx->n[0]);
     for (int64_t m = 0; m < ctx->n[0]; m++) {
       const long double th = two_pi * (long double)m / (long double)ctx->n[0];
-      t[m].x = (double)cosl(th);
-      t[m].y = (double)(-sinl(th));
+      w[m].x = (double)cosl(th);
+      w[m].y = (double)(-sinl(th));
     }
+    // in the order of the field, r n2 + c holding W_N^{r c}: the passes read
+    // it with their own points instead of gathering
+    for (int64_t r = 0; r < ctx->fs_n1; r++)
+      for (int64_t c = 0; c < ctx->fs_n2; c++) t[r * ctx->fs_n2 + c] = w[(r * c) % ctx->n[0]];
     ok = cudaMalloc(&ctx->fs_tw, sizeof(double2) * ctx->n[0]) == cudaSuccess &&
          cudaMemcpy(ctx->fs_tw, t.data(), sizeof(double2) * ctx->n[0], cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok) {
@@ -1120,6 +1146,29 @@ static int strang_block(atus_ctx *ctx, int nk, int kind, const double *F, const 
     // field too long for one CTA); the per-step passes below run the block
     if (r != ATUS_E_UNSUPPORTED) return r;
     ctx->err.clear();
+  }
+  if (ctx->fs_tw && ctx->ncomp <= 2) {
+    // long 1D axis: two passes over the fields per step, the strided one
+    // around the potential step and the contiguous one around the kinetic
+    // factor, twiddles in registers.  2^20 points, one FP64 component with a
+    // potential: 132 us per step as separate transforms, twiddle, kinetic and
+    // potential kernels (eight sweeps), 38 us as these two (22 + 16; FP64 issue
+    // bound: ~175 FP64 instructions a point in the strided pass).
+    int r = fs_pass(ctx, M2_FS_FWD, ctx->psi, ctx->ncomp, 1, nullptr);
+    if (r == ATUS_OK) {
+      RUN(fs_pass(ctx, M2_FS_KIN, ctx->psi, ctx->ncomp, 1, nullptr));
+      ctx->t += 0.5 * dt;
+      for (int j = 0; j < nk; j++) {
+        const bool last = (j == nk - 1);
+        const NLArgs nl = nl_args(ctx, kind, ctx->t + 0.5 * dt, F ? F[j] : 1.0);
+        RUN(fs_pass(ctx, M2_FS_NL, ctx->psi, ctx->ncomp, 0, &nl));
+        RUN(fs_pass(ctx, M2_FS_KIN, ctx->psi, ctx->ncomp, last ? 1 : 0, nullptr));
+        ctx->t += last ? 0.5 * dt : dt;
+      }
+      FsView v(ctx);
+      return run_pass(ctx, 0, T_INV, OP_NONE, T_NONE, nullptr, 0);
+    }
+    if (r != ATUS_E_UNSUPPORTED) return r;
   }
   if (ctx->dim == 1) {
     // more components or points than the resident 1D kernel holds, or a step

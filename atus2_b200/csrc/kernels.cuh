@@ -48,7 +48,13 @@ enum { K_NL = 0, K_NL_IF = 1, K_BRAGG = 2, K_DBRAGG = 3, K_NL_IF2 = 4, K_BRAGG_D
 // M2_FWD_SOB, M2_INV_SOB: the first and the last pass of a Sobolev iteration
 // (the transform of psi and W psi straight from psi; the inverse transform of
 // S psi and S(W psi) with their products with psi).
-enum { M2_FWD = 0, M2_INV = 1, M2_KIN = 2, M2_NL = 3, M2_KIN_RABI = 4, M2_FWD_SOB = 5, M2_INV_SOB = 6 };
+// M2_FS_*: the passes of a long 1D axis seen as n1 x n2 points (four-step
+// transforms), the twiddles W_N^{r c} applied in registers:
+//   M2_FS_FWD  strided axis: FFT, twiddles
+//   M2_FS_NL   strided axis: IFFT, potential step, FFT, twiddles
+//   M2_FS_KIN  contiguous axis: FFT, kinetic factor, IFFT, conjugate twiddles
+enum { M2_FWD = 0, M2_INV = 1, M2_KIN = 2, M2_NL = 3, M2_KIN_RABI = 4, M2_FWD_SOB = 5, M2_INV_SOB = 6,
+       M2_FS_FWD = 7, M2_FS_NL = 8, M2_FS_KIN = 9 };
 
 struct LaserD {
   double beta0, DeltaL[MAXC], Amp0, laser_k0, laser_dk0, laser_domh0, phase0, chirp_rate0, chirp;
@@ -102,6 +108,7 @@ struct PassArgs {
   NLArgs nl;
   int x_along;              // 1 when the pencil runs along axis 0 (x varies inside a pencil)
   int axis;                 // axis the pencils run along
+  const double2 *fs_tw;     // M2_FS_*: W_N^{r c} at grid index r n2 + c
   // OP_FILT: real k-space filter of CSOB_Base (include/CSOB_Base.h:228-248):
   // 1/(1 + alpha k^2) or -alpha k^2, times the transform scale.
   int filt_mode;
@@ -127,6 +134,15 @@ struct PassArgs {
   long wait_limit;       // try_wait rounds before a TMA tile counts as lost
   int drop_copies;       // issue no tile copies, so every wait runs out (error-path tests; 0)
 };
+
+// kt[c][0] without an indexed copy of the parameter array.
+__device__ __forceinline__ const double2 *pick_kt0(const PassArgs &a, int c) {
+  const double2 *k = a.kt[0][0];
+  #pragma unroll
+  for (int i = 1; i < MAXC; i++)
+    if (c == i) k = a.kt[i][0];
+  return k;
+}
 
 __device__ __forceinline__ void idx3(const Geo &g, int64_t l, int &ix, int &iy, int &iz) {
   ix = (int)(l >> (g.lg[1] + g.lg[2]));
@@ -639,6 +655,22 @@ __device__ __forceinline__ void bragg_coupling(const NLArgs &a, double x0, doubl
   Omega = a.F * a.L.Amp0 *
           cos(a.L.laser_k0 * x0 - (a.L.laser_domh0 + a.L.chirp * t1 + a.L.chirp_rate0 * t1) * t1 + a.L.phase0 / 2);
   sincos(-0.5 * (a.L.laser_dk0 * x0), &es, &ec);
+}
+
+// v times a twiddle (DIR > 0: its conjugate), in FP64 for both precisions.
+template <typename R, int DIR> __device__ __forceinline__ cplx<R> fs_mul(cplx<R> v, double2 w) {
+  return from_d<R>(DIR < 0 ? cmul(to_d<R>(v), w) : cmulc(to_d<R>(v), w));
+}
+
+// psi^ <- ((psi^ s_f) K) s_b in FP64.
+template <typename R> __device__ __forceinline__ cplx<R> kin_mul(cplx<R> v, double2 K, double s_f, double s_b) {
+  double2 u = to_d<R>(v);
+  u.x *= s_f;
+  u.y *= s_f;
+  u = cmul(u, K);
+  u.x *= s_b;
+  u.y *= s_b;
+  return from_d<R>(u);
 }
 
 // ------------------------------------------------------------ kinetic step

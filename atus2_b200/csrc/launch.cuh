@@ -375,3 +375,25 @@ static inline int launch_pass2_n(atus_ctx *ctx, PassArgs &a, int axis) {
   return ATUS_E_UNSUPPORTED;
 }
 
+// The four-step passes of one mode (ctx viewed as n1 x n2).
+template <typename R, int TC, int MODE, bool STRIDED>
+static inline int launch_fs_n(atus_ctx *ctx, PassArgs &a) {
+  constexpr int axis = STRIDED ? 0 : 1;
+  switch (ctx->n[axis]) {
+    case 128: return launch_pass2_t<R, 128, TC, MODE, STRIDED>(ctx, a, axis);
+    case 256: return launch_pass2_t<R, 256, TC, MODE, STRIDED>(ctx, a, axis);
+    case 512: return launch_pass3_t<R, 512, TC, MODE, STRIDED>(ctx, a, axis);
+    case 1024: return launch_pass3_t<R, 1024, TC, MODE, STRIDED>(ctx, a, axis);
+    case 2048: return launch_pass3_t<R, 2048, TC, MODE, STRIDED>(ctx, a, axis);
+    default: return ATUS_E_UNSUPPORTED;
+  }
+}
+
+template <typename R>
+static inline int launch_fs(atus_ctx *ctx, PassArgs &a, int mode, int tc) {
+  if (mode == M2_FS_FWD) return launch_fs_n<R, 1, M2_FS_FWD, true>(ctx, a);
+  if (mode == M2_FS_KIN) return launch_fs_n<R, 1, M2_FS_KIN, false>(ctx, a);
+  if (mode == M2_FS_NL && tc == 1) return launch_fs_n<R, 1, M2_FS_NL, true>(ctx, a);
+  if (mode == M2_FS_NL && tc == 2) return launch_fs_n<R, 2, M2_FS_NL, true>(ctx, a);
+  return ATUS_E_UNSUPPORTED;
+}

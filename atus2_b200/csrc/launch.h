@@ -30,3 +30,7 @@ int launch_pass2_f_nl(atus_ctx *ctx, PassArgs &a, int axis, int tc);
 // _sob: first (M2_FWD_SOB) and last (M2_INV_SOB) pass of a Sobolev iteration,
 // along the contiguous axis (32..256 points)
 int launch_pass2_d_sob(atus_ctx *ctx, PassArgs &a, int axis, int mode);
+// _fs: the passes of a long 1D axis seen as n1 x n2 points (M2_FS_*), axes of
+// 128..2048 points; tc: components of M2_FS_NL (1 or 2)
+int launch_fs_d(atus_ctx *ctx, PassArgs &a, int mode, int tc);
+int launch_fs_f(atus_ctx *ctx, PassArgs &a, int mode, int tc);

@@ -19,6 +19,8 @@
 // pencils (the inner grid index), so one warp-wide load covers whole 128-byte
 // rows; along the contiguous axis consecutive threads take consecutive points.
 #pragma once
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace atus {
@@ -29,9 +31,10 @@ template <> struct Tile2<double> { static constexpr int E = 2048, NT = 128, MINB
 template <> struct Tile2<float> { static constexpr int E = 4096, NT = 256, MINB = 3; };
 
 // CTAs per SM the register budget is sized for: the passes at the ends of a
-// Sobolev iteration hold a thread's 16 potential values beside its 16 points.
+// Sobolev iteration and the four-step passes hold potential values or
+// twiddles beside a thread's 16 points.
 template <typename R, int MODE>
-constexpr int p2_minb = (MODE == M2_FWD_SOB || MODE == M2_INV_SOB) ? 4 : Tile2<R>::MINB;
+constexpr int p2_minb = (MODE >= M2_FWD_SOB && sizeof(R) == 8) ? 4 : Tile2<R>::MINB;
 
 template <typename R, int N, int TC>
 struct P2Cfg {
@@ -258,7 +261,27 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
     for (int r = 0; r < 16; r++) v[r] = live ? src[r * step] : mk<R>(0, 0);
   }
 
-  if constexpr (MODE == M2_FWD || MODE == M2_FWD_SOB) {
+  // outputs times W_N^{r c} or its conjugate (four-step passes)
+  auto fs_twiddle = [&](auto dir) {
+    constexpr int DIR = decltype(dir)::value;
+    const double2 *const T = a.fs_tw + lb + (int64_t)j * a.sa;
+    if (live) {
+      #pragma unroll
+      for (int m = 0; m < 16; m++) v[m] = fs_mul<R, DIR>(v[m], __ldg(&T[m * step]));
+    }
+  };
+
+  if constexpr (MODE == M2_FS_FWD) {
+    p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
+    fs_twiddle(std::integral_constant<int, -1>());
+  } else if constexpr (MODE == M2_FS_KIN) {
+    p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
+    const double2 *const K = pick_kt0(a, g.comp0) + lb + j;
+    #pragma unroll
+    for (int m = 0; m < 16; m++) v[m] = kin_mul<R>(v[m], __ldg(&K[R2 * m]), a.s_f, a.s_b);
+    p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
+    fs_twiddle(std::integral_constant<int, 1>());
+  } else if constexpr (MODE == M2_FWD || MODE == M2_FWD_SOB) {
     p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
   } else if constexpr (MODE == M2_INV) {
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
@@ -381,7 +404,8 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
       }
     }
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
-  } else {  // M2_NL: IFFT -> potential step -> FFT
+  } else {  // M2_NL, M2_FS_NL: IFFT -> potential step -> FFT
+    constexpr bool FS = (MODE == M2_FS_NL);  // axis 0 is the whole grid index
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
     if constexpr (TC == 1) {
       int p0[3];
@@ -400,7 +424,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         if (m + AHEAD < 16) load_v(m + AHEAD);
         const int i = j + R2 * m;
         const int64_t l = lb + (int64_t)i * a.sa;
-        const int ix = (a.axis == 0) ? i : p0[0];
+        const int ix = FS ? (int)l : (a.axis == 0) ? i : p0[0];
         const double x0 = (double)(ix - a.nl.shift0) * a.nl.dx0;
         double om = 0, ec = 1, es = 0;
         if (a.nl.kind == K_BRAGG) bragg_coupling(a.nl, x0, om, ec, es);
@@ -429,7 +453,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
           const int64_t l = g.base0 + pb * g.pstride + (int64_t)i * a.sa;
           int ix, iy, iz;
           idx3(a.g, l, ix, iy, iz);
-          const double x0 = (double)(ix - a.nl.shift0) * a.nl.dx0;
+          const double x0 = (double)((FS ? (int)l : ix) - a.nl.shift0) * a.nl.dx0;
           double om = 0, ec = 1, es = 0;
           if (bragg) {
             if (a.axis == 0) bragg_coupling(a.nl, x0, om, ec, es);
@@ -451,6 +475,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
       }
     }
     p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
+    if constexpr (FS) fs_twiddle(std::integral_constant<int, -1>());
   }
 
   if (live) {

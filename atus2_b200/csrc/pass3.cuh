@@ -37,7 +37,8 @@ struct P3Cfg {
   static constexpr int M = N / 16;   // stage-1 butterflies: threads per pencil-component
   static constexpr int R3 = M / 16;  // radix of stage 3
   static constexpr int T3 = 16 / R3; // stage-3 butterflies per thread
-  static constexpr int BMIN = STRIDED ? ((sizeof(R) == 8 && M * TC * 8 > 512) ? 4 : 8) : 1;
+  static constexpr int BCAP = (sizeof(R) == 8 ? 512 : 1024) / (M * TC);  // pencils that fit the register file
+  static constexpr int BMIN = STRIDED ? (BCAP < 8 ? BCAP : 8) : 1;
   static constexpr int NT_MIN = M * TC * BMIN;
   static constexpr int NT = (NT_MIN > Tile3<R>::NT) ? NT_MIN : Tile3<R>::NT;
   static constexpr int NPC = NT / M; // pencil-components per tile
@@ -164,14 +165,34 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
   // the inverse transform (behind the per-point branches each load would
   // wait on its own)
   const double *const Vp = a.nl.V[0];
-  const bool preV = MODE == M2_NL && TC == 1 && a.nl.kind == K_NL && Vp != nullptr && live;
+  const bool preV = (MODE == M2_NL || MODE == M2_FS_NL) && TC == 1 && a.nl.kind == K_NL && Vp != nullptr && live;
   if (preV) {
     #pragma unroll
     for (int m = 0; m < 16; m++)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(Vp + lb + (int64_t)(t + M * m) * a.sa));
   }
 
-  if constexpr (MODE == M2_FWD) {
+  // outputs times W_N^{r c} or its conjugate (four-step passes)
+  auto fs_twiddle = [&](auto dir) {
+    constexpr int DIR = decltype(dir)::value;
+    const double2 *const T = a.fs_tw + lb + (int64_t)t * a.sa;
+    if (live) {
+      #pragma unroll
+      for (int m = 0; m < 16; m++) v[m] = fs_mul<R, DIR>(v[m], __ldg(&T[m * step]));
+    }
+  };
+
+  if constexpr (MODE == M2_FS_FWD) {
+    p3_transform<R, N, -1>(v, my, twN, twM, t);
+    fs_twiddle(std::integral_constant<int, -1>());
+  } else if constexpr (MODE == M2_FS_KIN) {
+    p3_transform<R, N, -1>(v, my, twN, twM, t);
+    const double2 *const K = pick_kt0(a, g.comp0) + lb + t;
+    #pragma unroll
+    for (int m = 0; m < 16; m++) v[m] = kin_mul<R>(v[m], __ldg(&K[M * m]), a.s_f, a.s_b);
+    p3_transform<R, N, +1>(v, my, twN, twM, t);
+    fs_twiddle(std::integral_constant<int, 1>());
+  } else if constexpr (MODE == M2_FWD) {
     p3_transform<R, N, -1>(v, my, twN, twM, t);
   } else if constexpr (MODE == M2_INV) {
     p3_transform<R, N, +1>(v, my, twN, twM, t);
@@ -228,7 +249,8 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
       }
     }
     p3_transform<R, N, +1>(v, my, twN, twM, t);
-  } else {  // M2_NL: IFFT -> potential step -> FFT
+  } else {  // M2_NL, M2_FS_NL: IFFT -> potential step -> FFT
+    constexpr bool FS = (MODE == M2_FS_NL);  // axis 0 is the whole grid index
     p3_transform<R, N, +1>(v, my, twN, twM, t);
     if constexpr (TC == 1) {
       int p0[3];
@@ -243,7 +265,7 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
         if (m + AHEAD < 16) load_v(m + AHEAD);
         const int i = t + M * m;
         const int64_t l = lb + (int64_t)i * a.sa;
-        const int ix = (a.axis == 0) ? i : p0[0];
+        const int ix = FS ? (int)l : (a.axis == 0) ? i : p0[0];
         const double x0 = (double)(ix - a.nl.shift0) * a.nl.dx0;
         double om = 0, ec = 1, es = 0;
         if (a.nl.kind == K_BRAGG) bragg_coupling(a.nl, x0, om, ec, es);
@@ -272,7 +294,7 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
           const int64_t l = g.base0 + pb * g.pstride + (int64_t)i * a.sa;
           int ix, iy, iz;
           idx3(a.g, l, ix, iy, iz);
-          const double x0 = (double)(ix - a.nl.shift0) * a.nl.dx0;
+          const double x0 = (double)((FS ? (int)l : ix) - a.nl.shift0) * a.nl.dx0;
           double om = 0, ec = 1, es = 0;
           if (bragg) {
             if (a.axis == 0) bragg_coupling(a.nl, x0, om, ec, es);
@@ -294,6 +316,7 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
       }
     }
     p3_transform<R, N, -1>(v, my, twN, twM, t);
+    if constexpr (FS) fs_twiddle(std::integral_constant<int, -1>());
   }
 
   if (live) {
