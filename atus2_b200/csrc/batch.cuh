@@ -252,8 +252,13 @@ __global__ void __launch_bounds__(Tile2<R>::NT, Tile2<R>::MINB) batch_pass2_kern
       setup = true;
       __syncthreads();  // twiddle rows visible to every warp before the first exchange
     }
-    p2_item<R, N, TC, MODE, STRIDED>(sa, tile_geo<Cfg::B, N>(sa, w % bp.items), smem_raw, false, s_om, s_ec,
-                                            s_es);
+    const TileGeo g = tile_geo<Cfg::B, N>(sa, w % bp.items);
+    if constexpr (p2_pair<TC, MODE, STRIDED>) {
+      if (threadIdx.x < Cfg::B)
+        p2_coupling(sa, g, threadIdx.x, s_om[threadIdx.x], s_ec[threadIdx.x], s_es[threadIdx.x]);
+      __syncthreads();
+    }
+    p2_item<R, N, TC, MODE, STRIDED>(sa, g, smem_raw, false, s_om, s_ec, s_es);
     __syncthreads();  // sa is rewritten by the next item
   }
 }

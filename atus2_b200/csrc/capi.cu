@@ -602,14 +602,20 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
     if (ok) ok = cudaMemset(ctx->psi[c], 0, ctx->csize * ctx->npts) == cudaSuccess;
   }
   if (ok) ok = cudaMalloc(&ctx->scratch, 16 * ctx->npts) == cudaSuccess;
-  if (ok) ok = cudaMallocHost(&ctx->err_word, sizeof(int)) == cudaSuccess;
-  if (ok) *ctx->err_word = 0;
   if (ok) ok = cudaMalloc(&ctx->red_partial, sizeof(double) * RED_ROWS * RED_MAXQ) == cudaSuccess;
   if (ok)
     ok = cudaMalloc(&ctx->red_count, sizeof(unsigned)) == cudaSuccess &&
          cudaMemset(ctx->red_count, 0, sizeof(unsigned)) == cudaSuccess;
-  if (ok) ok = cudaMallocHost(&ctx->h_red, sizeof(double) * RED_MAXQ) == cudaSuccess;
-  if (ok) ok = cudaMallocHost(&ctx->h_sob, sizeof(SobDev)) == cudaSuccess;
+  if (ok) {  // one pinned block: reduction totals, the descent's scalars, the error word
+    constexpr size_t red = sizeof(double) * RED_MAXQ, sob = (sizeof(SobDev) + 15) / 16 * 16;
+    ok = cudaMallocHost(&ctx->pinned, red + sob + sizeof(int)) == cudaSuccess;
+    if (ok) {
+      ctx->h_red = static_cast<double *>(ctx->pinned);
+      ctx->h_sob = static_cast<char *>(ctx->pinned) + red;
+      ctx->err_word = reinterpret_cast<int *>(static_cast<char *>(ctx->pinned) + red + sob);
+      *ctx->err_word = 0;
+    }
+  }
   if (ok) {
     ok = cudaMalloc(&ctx->tw64, 16 * TWN) == cudaSuccess;
     if (ok) {
@@ -691,16 +697,14 @@ void atus_destroy(atus_ctx *ctx) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   cudaFree(ctx->fs_tw);
   cudaFree(ctx->fs_tmp);
-  if (ctx->err_word) cudaFreeHost(ctx->err_word);
   cudaFree(ctx->scratch);
   cudaFree(ctx->sob_dev);
   if (ctx->sob_graph) cudaGraphExecDestroy(ctx->sob_graph);
-  if (ctx->h_sob) cudaFreeHost(ctx->h_sob);
   if (ctx->tw != ctx->tw64) cudaFree(ctx->tw);
   cudaFree(ctx->tw64);
   cudaFree(ctx->red_partial);
   cudaFree(ctx->red_count);
-  if (ctx->h_red) cudaFreeHost(ctx->h_red);
+  if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
 }

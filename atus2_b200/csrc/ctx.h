@@ -32,13 +32,14 @@ struct atus_ctx {
   double2 *kt[2][MAXC][3] = {}; // kinetic phase factors [half=0/full=1][comp][axis], FP64
   double *red_partial = nullptr;  // block sums of the reductions
   unsigned *red_count = nullptr;  // blocks done; zero between launches
-  double *h_red = nullptr;        // their totals (pinned host memory, written by the device)
+  void *pinned = nullptr;         // host memory mapped into the device: h_red, h_sob, err_word
+  double *h_red = nullptr;        // totals of a reduction, written by the device
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int64_t launches = 0;
   bool use_pass2 = true;        // register-staged passes for pencils of 32..256 points
   bool use_cluster1d = true;    // 1D blocks of 2048..8192 points on a 16-CTA cluster
   bool use_tma = false;         // strided 256-point passes fed by TMA tile copies
-  int *err_word = nullptr;      // error word of bounded waits, pinned host memory (0: none)
+  int *err_word = nullptr;      // error word of bounded waits (0: none)
   bool err_armed = false;       // a kernel that can set it ran since the last check
   long wait_limit = 1L << 22;   // TMA tile waits: try_wait rounds (atus_set_wait_limits)
   int drop_copies = 0;          // TMA passes issue no copies (error-path tests)

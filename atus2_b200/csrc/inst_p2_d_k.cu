@@ -2,5 +2,6 @@
 #include "launch.cuh"
 
 int launch_pass2_d_k(atus_ctx *ctx, PassArgs &a, int axis) {
-  return launch_pass2_n<double, 1, M2_KIN, true>(ctx, a, axis);
+  return a.op == OP_FILT ? launch_pass2_n<double, 1, M2_FILT, true>(ctx, a, axis)
+                         : launch_pass2_n<double, 1, M2_KIN, true>(ctx, a, axis);
 }

@@ -48,13 +48,15 @@ enum { K_NL = 0, K_NL_IF = 1, K_BRAGG = 2, K_DBRAGG = 3, K_NL_IF2 = 4, K_BRAGG_D
 // M2_FWD_SOB, M2_INV_SOB: the first and the last pass of a Sobolev iteration
 // (the transform of psi and W psi straight from psi; the inverse transform of
 // S psi and S(W psi) with their products with psi).
+// M2_FILT: FFT, Sobolev or Laplace filter, IFFT (apart from M2_KIN, whose
+// complex64 x pass went from 160 to 170 us on 256^3 x 2 with both in one).
 // M2_FS_*: the passes of a long 1D axis seen as n1 x n2 points (four-step
 // transforms), the twiddles W_N^{r c} applied in registers:
 //   M2_FS_FWD  strided axis: FFT, twiddles
 //   M2_FS_NL   strided axis: IFFT, potential step, FFT, twiddles
 //   M2_FS_KIN  contiguous axis: FFT, kinetic factor, IFFT, conjugate twiddles
 enum { M2_FWD = 0, M2_INV = 1, M2_KIN = 2, M2_NL = 3, M2_KIN_RABI = 4, M2_FWD_SOB = 5, M2_INV_SOB = 6,
-       M2_FS_FWD = 7, M2_FS_NL = 8, M2_FS_KIN = 9 };
+       M2_FS_FWD = 7, M2_FS_NL = 8, M2_FS_KIN = 9, M2_FILT = 10 };
 
 struct LaserD {
   double beta0, DeltaL[MAXC], Amp0, laser_k0, laser_dk0, laser_domh0, phase0, chirp_rate0, chirp;
@@ -161,26 +163,38 @@ __device__ __forceinline__ double reduce_2pi(double a) {
   return fma(-q, P3, r);
 }
 
+// sincos() out of line: the step kernels call it from 8 or 16 places each, for
+// arguments that a resolved time step rarely has, and its inlined copies cost
+// the common path registers.
+static __device__ __noinline__ double2 sincos_far(double x) {
+  double s, c;
+  sincos(x, &s, &c);
+  return make_double2(c, s);
+}
+
 // sin and cos of an FP64 argument.  The phases of a time step are small
-// (|dt V| << 1 in practice), so |x| <= 1/32 takes the Taylor polynomials
-//   sin x = x (1 - x^2/3! + x^4/5! - x^6/7! + x^8/9!)
-//   cos x = 1 - x^2/2! + x^4/4! - x^6/6! + x^8/8! - x^10/10!
-// whose truncation errors (x^11/11!, x^12/12!) are below 2^-70 there, in
-// Horner form on x^2; larger arguments call sincos().
+// (|dt V| << 1 in practice), so |x| <= 1/32 takes the series; larger
+// arguments call sincos().
+// (cos, sin) by Taylor series to x^8 (cos) and x^7 (sin): the first omitted
+// terms, x^10/10! and x^9/9!, are below 2.5e-22 and 2.5e-18 x for |x| <= 1/32.
+__device__ __forceinline__ double2 expi_series(double x) {
+  const double x2 = x * x;
+  double ps = fma(x2, -1.0 / 5040.0, 1.0 / 120.0);
+  ps = fma(ps, x2, -1.0 / 6.0);
+  double pc = fma(x2, 1.0 / 40320.0, -1.0 / 720.0);
+  pc = fma(pc, x2, 1.0 / 24.0);
+  pc = fma(pc, x2, -0.5);
+  return make_double2(fma(pc, x2, 1.0), fma(ps * x2, x, x));
+}
 __device__ __forceinline__ void sincos_step(double x, double *s, double *c) {
   if (fabs(x) <= 0.03125) {
-    // Taylor series to x^7 (sin) and x^8 (cos): the first omitted terms,
-    // x^9/9! and x^10/10!, are below 2.5e-18 x and 2.5e-22 for |x| <= 1/32
-    const double x2 = x * x;
-    double ps = fma(x2, -1.0 / 5040.0, 1.0 / 120.0);
-    ps = fma(ps, x2, -1.0 / 6.0);
-    *s = fma(ps * x2, x, x);
-    double pc = fma(x2, 1.0 / 40320.0, -1.0 / 720.0);
-    pc = fma(pc, x2, 1.0 / 24.0);
-    pc = fma(pc, x2, -0.5);
-    *c = fma(pc, x2, 1.0);
+    const double2 e = expi_series(x);
+    *c = e.x;
+    *s = e.y;
   } else {
-    sincos(x, s, c);
+    const double2 e = sincos_far(x);
+    *c = e.x;
+    *s = e.y;
   }
 }
 
@@ -205,17 +219,20 @@ template <> __device__ __forceinline__ double2 expi<double>(double phi) {
   sincos_step(phi, &s, &c);
   return make_double2(c, s);
 }
+static __device__ __noinline__ double2 expi_far_mixed(double phi) {
+  float s, c;
+  sincosf((float)reduce_2pi(phi), &s, &c);
+  const double cd = c, sd = s;
+  const double inv = rsqrt(cd * cd + sd * sd);
+  return make_double2(cd * inv, sd * inv);
+}
 template <> __device__ __forceinline__ double2 expi<float>(double phi) {
   if (fabs(phi) <= 0.03125) {  // the usual phase of one time step: FP64 Taylor, |e| = 1 to FP64
     double sd, cd;
     sincos_step(phi, &sd, &cd);
     return make_double2(cd, sd);
   }
-  float s, c;
-  sincosf((float)reduce_2pi(phi), &s, &c);
-  const double cd = c, sd = s;
-  const double inv = rsqrt(cd * cd + sd * sd);
-  return make_double2(cd * inv, sd * inv);
+  return expi_far_mixed(phi);
 }
 
 // ------------------------------------------------------------ three-level Bragg step
@@ -302,57 +319,64 @@ __device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_
 
 // ------------------------------------------------------------ two-level exponential
 // exp(-i dt [[V11, Omega eta], [Omega conj(eta), V22]]) applied to (p1, p2).
-// FP64 and not `stable`: the reference's eigenvalue form (bragg.cpp:226-302,
-// bragg_ds.cpp:215-248): E+- = (V11 + V22 +- sqrt((V11 - V22)^2 + 4 Omega^2))/2,
-// gamma+- = e^{-i dt E+-} / |(V11 - E+-)^2 + Omega^2|, pure phases when
-// Omega == 0.  Otherwise the eigenvalue-free form
-//   U = e^{-i dt m} [cos(r dt) I - i sin(r dt)/r [[d, W], [W, -d]]],
-// m = (V11+V22)/2, d = (V11-V22)/2, W = Omega, r = sqrt(d^2 + W^2), built in
-// FP64 from unit (cos, sin) pairs, so it is unitary to FP64 accuracy for every
-// Omega (the eigenvalue form divides by (V11 - E)^2 + Omega^2, which loses
-// unitarity once Omega is below the spacing of V and divides by zero once
-// Omega^2 underflows).
+// With m = (V11+V22)/2, d = (V11-V22)/2, r = sqrt(d^2 + Omega^2), x = r dt:
+//   U = e^{-i dt m} [cos x I - i dt (sin x / x) [[d, Omega eta], [Omega conj(eta), -d]]].
+// cos x and sin x / x are even in x, so for x <= 1/32 -- a time step that
+// resolves the coupling -- they are short Taylor series in x^2 and the step
+// needs no square root and no division.  Truncation below 2.5e-22 (cos, to
+// x^8) and 2.6e-23 (sin x / x, to x^8).
+//
+// FP64 and not `stable` follows the reference's eigenvalue form (bragg.cpp:
+// 226-302, bragg_ds.cpp:215-248), in bragg_pair_eigen below, which divides by
+// (V11 - E+-)^2 + Omega^2 and so carries an error of about 2^-53 |V| / |Omega|
+// (and no unitarity at all once Omega^2 underflows).  Where that error is
+// below 2^-41 (Omega^2 >= 2^-24 (V11^2 + V22^2)) the two forms are the same
+// map to 4.5e-13 and the series serves; below that line, and for longer
+// steps, the reference's operations stay.  Complex64 fields and `stable`
+// always take the eigenvalue-free form.
+// swapped: states 1 and 2 exchanged throughout (V11 with V22, eta with its
+// conjugate, q1 with q2) -- the same step for a thread that holds state 2.
+// 256^3, two components, z pass (components meeting in shared memory):
+// eigenvalue form everywhere 0.368 ms, series 0.337 ms, no exponential 0.283.
 template <typename R>
-__device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, double V22, double Omega, double eta_c,
-                                           double eta_s, cplx<R> &q1, cplx<R> &q2) {
-  if constexpr (sizeof(R) == 8) {
-    if (!stable) {
-      double re1, im1;
-      if (Omega == 0.0) {
-        sincos_step(-dt * V11, &im1, &re1);
-        q1 = cmul(q1, make_double2(re1, im1));
-        sincos_step(-dt * V22, &im1, &re1);
-        q2 = cmul(q2, make_double2(re1, im1));
-        return;
-      }
-      double tmp1 = sqrt((V11 - V22) * (V11 - V22) + 4.0 * Omega * Omega);
-      const double Ep = 0.5 * (V11 + V22 + tmp1);
-      const double Em = 0.5 * (V11 + V22 - tmp1);
-      double2 gp, gm;
-      // the reference's 1 / |(V11 - E+-)^2 + Omega^2| (sums of squares, so
-      // |.| is the identity) from one division: 1/A = B/(AB), 1/B = A/(AB)
-      const double Ap = (V11 - Ep) * (V11 - Ep) + Omega * Omega;
-      const double Am = (V11 - Em) * (V11 - Em) + Omega * Omega;
-      const double inv = 1.0 / (Ap * Am);
-      sincos_step(-dt * Ep, &im1, &re1);
-      tmp1 = Am * inv;
-      gp = make_double2(tmp1 * re1, tmp1 * im1);
-      sincos_step(-dt * Em, &im1, &re1);
-      tmp1 = Ap * inv;
-      gm = make_double2(tmp1 * re1, tmp1 * im1);
-      const double O2 = Omega * Omega;
-      const double2 O11 = make_double2(O2 * (gp.x + gm.x), O2 * (gp.y + gm.y));
-      const double a1 = V11 - Ep, a2 = V11 - Em;
-      const double2 O22 = make_double2(a1 * a1 * gp.x + a2 * a2 * gm.x, a1 * a1 * gp.y + a2 * a2 * gm.y);
-      const double2 Os = make_double2(-Omega * (a1 * gp.x + a2 * gm.x), -Omega * (a1 * gp.y + a2 * gm.y));
-      const double2 eta = make_double2(eta_c, eta_s);
-      const double2 O12 = cmul(Os, eta);   // eta * O12
-      const double2 O21 = cmulc(Os, eta);  // conj(eta) * O21
-      const double2 p1 = q1, p2 = q2;
-      q1 = cadd(cmul(O11, p1), cmul(O12, p2));
-      q2 = cadd(cmul(O21, p1), cmul(O22, p2));
+__device__ __noinline__ void bragg_pair_general(int stable, double dt, double V11, double V22, double Omega,
+                                                double eta_c, double eta_s, double2 p1, double2 p2, double2 *o1,
+                                                double2 *o2) {
+  const double2 eta = make_double2(eta_c, eta_s);
+  if (sizeof(R) == 8 && !stable) {
+    double re1, im1;
+    if (Omega == 0.0) {
+      sincos_step(-dt * V11, &im1, &re1);
+      *o1 = cmul(p1, make_double2(re1, im1));
+      sincos_step(-dt * V22, &im1, &re1);
+      *o2 = cmul(p2, make_double2(re1, im1));
       return;
     }
+    double tmp1 = sqrt((V11 - V22) * (V11 - V22) + 4.0 * Omega * Omega);
+    const double Ep = 0.5 * (V11 + V22 + tmp1);
+    const double Em = 0.5 * (V11 + V22 - tmp1);
+    double2 gp, gm;
+    // the reference's 1 / |(V11 - E+-)^2 + Omega^2| (sums of squares, so
+    // |.| is the identity) from one division: 1/A = B/(AB), 1/B = A/(AB)
+    const double Ap = (V11 - Ep) * (V11 - Ep) + Omega * Omega;
+    const double Am = (V11 - Em) * (V11 - Em) + Omega * Omega;
+    const double inv = 1.0 / (Ap * Am);
+    sincos_step(-dt * Ep, &im1, &re1);
+    tmp1 = Am * inv;
+    gp = make_double2(tmp1 * re1, tmp1 * im1);
+    sincos_step(-dt * Em, &im1, &re1);
+    tmp1 = Ap * inv;
+    gm = make_double2(tmp1 * re1, tmp1 * im1);
+    const double O2 = Omega * Omega;
+    const double2 O11 = make_double2(O2 * (gp.x + gm.x), O2 * (gp.y + gm.y));
+    const double a1 = V11 - Ep, a2 = V11 - Em;
+    const double2 O22 = make_double2(a1 * a1 * gp.x + a2 * a2 * gm.x, a1 * a1 * gp.y + a2 * a2 * gm.y);
+    const double2 Os = make_double2(-Omega * (a1 * gp.x + a2 * gm.x), -Omega * (a1 * gp.y + a2 * gm.y));
+    const double2 O12 = cmul(Os, eta);   // eta * O12
+    const double2 O21 = cmulc(Os, eta);  // conj(eta) * O21
+    *o1 = cadd(cmul(O11, p1), cmul(O12, p2));
+    *o2 = cadd(cmul(O21, p1), cmul(O22, p2));
+    return;
   }
   const double m = 0.5 * (V11 + V22), d = 0.5 * (V11 - V22);
   const double r = sqrt(d * d + Omega * Omega);
@@ -375,11 +399,50 @@ __device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, do
   const double2 U11 = cmul(e, make_double2(rr.x, -fd));
   const double2 U22 = cmul(e, make_double2(rr.x, fd));
   const double2 Uo = cmul(e, make_double2(0.0, -fw));
-  const double2 et = make_double2(eta_c, eta_s);
-  const double2 U12 = cmul(Uo, et), U21 = cmulc(Uo, et);
+  const double2 U12 = cmul(Uo, eta), U21 = cmulc(Uo, eta);
+  *o1 = cadd(cmul(U11, p1), cmul(U12, p2));
+  *o2 = cadd(cmul(U21, p1), cmul(U22, p2));
+}
+
+// The series form for x^2 = x2 (<= 2^-10), e = e^{-i dt m}.
+template <typename R>
+__device__ __forceinline__ void bragg_series(double dt, double x2, double d, double Omega, double2 e, double eta_c,
+                                             double eta_s, cplx<R> &q1, cplx<R> &q2) {
   const double2 p1 = to_d<R>(q1), p2 = to_d<R>(q2);
-  q1 = from_d<R>(cadd(cmul(U11, p1), cmul(U12, p2)));
-  q2 = from_d<R>(cadd(cmul(U21, p1), cmul(U22, p2)));
+  double ps = fma(x2, 1.0 / 362880.0, -1.0 / 5040.0);
+  ps = fma(ps, x2, 1.0 / 120.0);
+  ps = fma(ps, x2, -1.0 / 6.0);
+  const double s = dt * fma(ps, x2, 1.0);  // sin(x) / r
+  double pc = fma(x2, 1.0 / 40320.0, -1.0 / 720.0);
+  pc = fma(pc, x2, 1.0 / 24.0);
+  pc = fma(pc, x2, -0.5);
+  const double c = fma(pc, x2, 1.0);
+  const double fd = s * d, so = s * Omega;
+  const double2 w = make_double2(so * eta_c, so * eta_s);
+  // (c - i fd) p1 - i w p2 and (c + i fd) p2 - i conj(w) p1
+  const double2 a = make_double2(c * p1.x + fd * p1.y + (w.x * p2.y + w.y * p2.x),
+                                 c * p1.y - fd * p1.x - (w.x * p2.x - w.y * p2.y));
+  const double2 b = make_double2(c * p2.x - fd * p2.y + (w.x * p1.y - w.y * p1.x),
+                                 c * p2.y + fd * p2.x - (w.x * p1.x + w.y * p1.y));
+  q1 = from_d<R>(cmul(e, a));
+  q2 = from_d<R>(cmul(e, b));
+}
+
+template <typename R>
+__device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, double V22, double Omega, double eta_c,
+                                           double eta_s, cplx<R> &q1, cplx<R> &q2, bool swapped = false) {
+  const double m = 0.5 * (V11 + V22), d = 0.5 * (V11 - V22), O2 = Omega * Omega;
+  const double x2 = (dt * dt) * (d * d + O2);
+  if (x2 <= 0x1p-10 && (sizeof(R) == 4 || stable || O2 >= 0x1p-24 * (V11 * V11 + V22 * V22))) {
+    bragg_series<R>(dt, x2, d, Omega, expi<R>(-dt * m), eta_c, eta_s, q1, q2);
+    return;
+  }
+  const double2 p1 = to_d<R>(q1), p2 = to_d<R>(q2);
+  double2 o1, o2;
+  if (swapped) bragg_pair_general<R>(stable, dt, V22, V11, Omega, eta_c, -eta_s, p2, p1, &o2, &o1);
+  else bragg_pair_general<R>(stable, dt, V11, V22, Omega, eta_c, eta_s, p1, p2, &o1, &o2);
+  q1 = from_d<R>(o1);
+  q2 = from_d<R>(o2);
 }
 
 // ------------------------------------------------------------ two-species Bragg step
@@ -571,6 +634,165 @@ __device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, d
     if (j < n) v[j] = from_d<R>(p[j]);
 }
 
+
+// v with its sign bits flipped by mask sg (0 or 0x80000000).
+__device__ __forceinline__ double flip1(double x, int sg) {
+  return __hiloint2double(__double2hiint(x) ^ sg, __double2loint(x));
+}
+__device__ __forceinline__ float flip1(float x, int sg) { return __int_as_float(__float_as_int(x) ^ sg); }
+template <typename C> __device__ __forceinline__ C flip(C v, int sg) {
+  v.x = flip1(v.x, sg);
+  v.y = flip1(v.y, sg);
+  return v;
+}
+template <typename C> __device__ __forceinline__ C shfl_xor_c(C v, int mask) {
+  v.x = __shfl_xor_sync(0xffffffffu, v.x, mask);
+  v.y = __shfl_xor_sync(0xffffffffu, v.y, mask);
+  return v;
+}
+
+// Potential step of two components on 16 points a thread, the components of a
+// point in two lanes of a warp (partner = lane ^ mask).  Thread c (0 or 1)
+// holds its component's points in the order m ^ 8c, m < 16, so registers
+// m < 8 are the points it steps for both components, and registers m + 8
+// those its partner does: one shuffle brings the partner's value of a point,
+// one returns the result, with no shared memory, no barrier and no register
+// selection.  Point of register m: grid index l0 + dl (m ^ 8c).  x0, om, ec, es
+// belong to the pencil; live: it is inside the grid.
+//
+// nl_pair16_any takes every step kind and size of phase, on a copy in local
+// memory: with its calls inlined eight or sixteen times the common path lost
+// its registers to spills (z pass of 256^3 FP64: 0.35 ms).
+template <typename R>
+__device__ __noinline__ void nl_pair16_any(const NLArgs &a, cplx<R> *v, int c, int mask, bool live, double x0,
+                                           double om, double ec, double es, int64_t l0, int dl) {
+  using C = cplx<R>;
+  if (a.kind == K_BRAGG || a.kind == K_NUM_BRAGG) {
+    const double bx = a.L.beta0 * x0, bd = bx - a.L.DeltaL[1];
+    #pragma unroll 1
+    for (int m = 0; m < 8; m++) {
+      C own = v[m], oth = shfl_xor_c(v[m + 8], mask);
+      if (a.kind == K_BRAGG) {
+        const double ro = (double)own.x * (double)own.x + (double)own.y * (double)own.y;
+        const double rt = (double)oth.x * (double)oth.x + (double)oth.y * (double)oth.y;
+        const double Vo = a.gs[c * (MAXC + 1)] * ro + a.gs[c ? MAXC : 1] * rt + (c ? bd : bx);
+        const double Vt = a.gs[c ? 1 : MAXC] * ro + a.gs[c ? 0 : MAXC + 1] * rt + (c ? bx : bd);
+        bragg_pair<R>(a.stable, a.dt, Vo, Vt, om, ec, c ? -es : es, own, oth, c != 0);
+      } else {
+        C w[2] = {c ? oth : own, c ? own : oth};
+        num_point<R, 2>(a, w, l0 + (int64_t)dl * (m ^ (8 * c)), x0);
+        own = c ? w[1] : w[0];
+        oth = c ? w[0] : w[1];
+      }
+      v[m] = own;
+      v[m + 8] = shfl_xor_c(oth, mask);
+    }
+    return;
+  }
+  // pure phases: a point needs only the partner's density
+  const double *const Vp = (a.kind == K_NL && live) ? (c ? a.V[1] : a.V[0]) : nullptr;
+  const double b = (a.kind == K_NL_IF2 && c) ? a.L2.beta0 : a.L.beta0;
+  const double off = (a.kind == K_NL) ? 0.0 : b * x0 - (c ? a.L.DeltaL[1] : a.L.DeltaL[0]);
+  #pragma unroll 2
+  for (int m = 0; m < 8; m++) {  // registers m and m + 8 together: their densities cross over
+    const C v0 = v[m], v1 = v[m + 8];
+    const double w0 = Vp ? __ldg(&Vp[l0 + (int64_t)dl * (m ^ (8 * c))]) : 0.0;
+    const double w1 = Vp ? __ldg(&Vp[l0 + (int64_t)dl * ((m + 8) ^ (8 * c))]) : 0.0;
+    const double r0 = (double)v0.x * (double)v0.x + (double)v0.y * (double)v0.y;
+    const double r1 = (double)v1.x * (double)v1.x + (double)v1.y * (double)v1.y;
+    const double t0 = __shfl_xor_sync(0xffffffffu, r1, mask), t1 = __shfl_xor_sync(0xffffffffu, r0, mask);
+    const double g_oo = a.gs[c * (MAXC + 1)], g_ot = a.gs[c ? MAXC : 1];
+    v[m] = from_d<R>(cmul(to_d<R>(v0), expi<R>((w0 + (g_oo * r0 + g_ot * t0 + off)) * a.mdt)));
+    v[m + 8] = from_d<R>(cmul(to_d<R>(v1), expi<R>((w1 + (g_oo * r1 + g_ot * t1 + off)) * a.mdt)));
+  }
+}
+
+// Largest |re| or |im| of v[0..16), rounded up.
+__device__ __forceinline__ double abs_bound(const double2 *v) {
+  int h = 0;
+  #pragma unroll
+  for (int m = 0; m < 16; m++)
+    h = max(h, max(__double2hiint(v[m].x) & 0x7fffffff, __double2hiint(v[m].y) & 0x7fffffff));
+  return __hiloint2double(h + 1, 0);  // NaN and infinity stay above every bound
+}
+__device__ __forceinline__ double abs_bound(const float2 *v) {
+  int h = 0;
+  #pragma unroll
+  for (int m = 0; m < 16; m++)
+    h = max(h, max(__float_as_int(v[m].x) & 0x7fffffff, __float_as_int(v[m].y) & 0x7fffffff));
+  return (double)__int_as_float(h);
+}
+
+// BRAGG: a.kind is K_BRAGG (else it is not); apart, each keeps its registers.
+template <typename R, bool BRAGG>
+__device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, int mask, bool live, double x0, double om,
+                                          double ec, double es, int64_t l0, int dl) {
+  using C = cplx<R>;
+  // The series serve every point of the warp if they do for the largest
+  // potential that its points allow: |V| <= G rho + |off| + max |V_c|, with
+  // rho <= 2 max(|re|, |im|)^2 over the pencil and G the larger row sum of |g|.
+  const double bx = a.L.beta0 * x0, bd = bx - a.L.DeltaL[1];
+  const double m1 = abs_bound(v), mx = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, mask));
+  const double G = fmax(fabs(a.gs[0]) + fabs(a.gs[1]), fabs(a.gs[MAXC]) + fabs(a.gs[MAXC + 1]));
+  const double Vrho = 2.0 * G * (mx * mx);
+  const double *const Vp = (a.kind == K_NL && live) ? (c ? a.V[1] : a.V[0]) : nullptr;
+  // pure phases: the constant part of the component's potential
+  const double off = (a.kind == K_NL) ? 0.0
+                                      : ((a.kind == K_NL_IF2 && c) ? a.L2.beta0 : a.L.beta0) * x0 -
+                                            (c ? a.L.DeltaL[1] : a.L.DeltaL[0]);
+  bool small = false;
+  if constexpr (BRAGG) {
+    const double V = Vrho + fmax(fabs(bx), fabs(bd)), O2 = om * om;
+    small = fabs(a.dt) * V <= 0.03125 && (a.dt * a.dt) * (V * V + O2) <= 0x1p-10 &&
+            (sizeof(R) == 4 || a.stable || O2 >= 0x1p-23 * (V * V));
+  } else if (a.kind != K_NUM_BRAGG) {
+    int h = 0;
+    if (Vp) {
+      #pragma unroll
+      for (int m = 0; m < 16; m++) h = max(h, __double2hiint(__ldg(&Vp[l0 + (int64_t)dl * m])) & 0x7fffffff);
+      h++;
+    }
+    small = fabs(a.dt) * (Vrho + fabs(off) + __hiloint2double(h, 0)) <= 0.03125;
+  }
+  if (!__all_sync(0xffffffffu, small)) {
+    C w[16];
+    #pragma unroll
+    for (int m = 0; m < 16; m++) w[m] = v[m];
+    nl_pair16_any<R>(a, w, c, mask, live, x0, om, ec, es, l0, dl);
+    #pragma unroll
+    for (int m = 0; m < 16; m++) v[m] = w[m];
+    return;
+  }
+  if constexpr (!BRAGG) {  // a point needs only the partner's density
+    const double s_oo = a.gs[c * (MAXC + 1)], s_ot = a.gs[c ? MAXC : 1];
+    #pragma unroll
+    for (int m = 0; m < 8; m++) {  // registers m and m + 8 together: their densities cross over
+      const C v0 = v[m], v1 = v[m + 8];
+      const double w0 = Vp ? __ldg(&Vp[l0 + (int64_t)dl * (m ^ (8 * c))]) : 0.0;
+      const double w1 = Vp ? __ldg(&Vp[l0 + (int64_t)dl * ((m + 8) ^ (8 * c))]) : 0.0;
+      const double r0 = (double)v0.x * (double)v0.x + (double)v0.y * (double)v0.y;
+      const double r1 = (double)v1.x * (double)v1.x + (double)v1.y * (double)v1.y;
+      const double t0 = __shfl_xor_sync(0xffffffffu, r1, mask), t1 = __shfl_xor_sync(0xffffffffu, r0, mask);
+      v[m] = from_d<R>(cmul(to_d<R>(v0), expi_series((w0 + (s_oo * r0 + s_ot * t0 + off)) * a.mdt)));
+      v[m + 8] = from_d<R>(cmul(to_d<R>(v1), expi_series((w1 + (s_oo * r1 + s_ot * t1 + off)) * a.mdt)));
+    }
+    return;
+  }
+  const double g_oo = a.gs[c * (MAXC + 1)], g_ot = a.gs[c ? MAXC : 1];
+  const double g_to = a.gs[c ? 1 : MAXC], g_tt = a.gs[c ? 0 : MAXC + 1];
+  const double off_o = c ? bd : bx, off_t = c ? bx : bd, se = c ? -es : es, dt2 = a.dt * a.dt, O2 = om * om;
+  #pragma unroll
+  for (int m = 0; m < 8; m++) {
+    C own = v[m], oth = shfl_xor_c(v[m + 8], mask);
+    const double ro = (double)own.x * (double)own.x + (double)own.y * (double)own.y;
+    const double rt = (double)oth.x * (double)oth.x + (double)oth.y * (double)oth.y;
+    const double Vo = g_oo * ro + g_ot * rt + off_o, Vt = g_to * ro + g_tt * rt + off_t;
+    const double d = 0.5 * (Vo - Vt);
+    bragg_series<R>(a.dt, dt2 * (d * d + O2), d, om, expi_series(a.mdt * (0.5 * (Vo + Vt))), ec, se, own, oth);
+    v[m] = own;
+    v[m + 8] = shfl_xor_c(oth, mask);
+  }
+}
 
 // ------------------------------------------------------------ potential step
 // Point-wise potential step on the ncomp values v[] at grid index l.

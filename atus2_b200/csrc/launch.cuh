@@ -7,6 +7,7 @@
 #include "ctx.h"
 #include "cluster1d.cuh"
 #include "pass2.cuh"
+#include "pass2_pair.cuh"
 #include "pass2_tma.cuh"
 #include "pass3.cuh"
 
@@ -246,6 +247,34 @@ static inline int launch_pass2_tma_t(atus_ctx *ctx, PassArgs &a, int axis) {
   return ATUS_OK;
 }
 
+// IFFT -> potential step -> FFT of two components along the contiguous axis.
+template <typename R, int N, bool BRAGG>
+static inline int launch_pair_t(atus_ctx *ctx, PassArgs &a, int axis) {
+  using Cfg = PairCfg<R, N>;
+  static int resident = 0;
+  static int nsm = 0;
+  if (!resident) {
+    CK(cudaFuncSetAttribute(pass2_pair_kernel<R, N, BRAGG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
+    CK(cudaFuncSetAttribute(pass2_pair_kernel<R, N, BRAGG>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                            cudaSharedmemCarveoutMaxShared));
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pass2_pair_kernel<R, N, BRAGG>, Cfg::NT, Cfg::smem));
+    if (resident < 1) return fail(ctx, ATUS_E_UNSUPPORTED, "pass kernel does not fit on an SM");
+  }
+  a.sa = 1;
+  a.npencils = ctx->npts / N;
+  a.axis = axis;
+  a.g = geo(ctx);
+  a.tw = (sizeof(R) == 8) ? ctx->tw64 : ctx->tw;
+  const int64_t ctas = (a.npencils + Cfg::PW * Cfg::WPC - 1) / (Cfg::PW * Cfg::WPC);
+  const int64_t slots = (int64_t)nsm * resident;
+  pass2_pair_kernel<R, N, BRAGG><<<(unsigned)(ctas < slots ? ctas : slots), Cfg::NT, Cfg::smem, ctx->stream>>>(a);
+  LAUNCHED(ctx);
+  return ATUS_OK;
+}
+
 template <typename R, int N, int TC, int MODE, bool STRIDED>
 static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   // 256-point pencils only: on 128-point pencils (the 128^3 Sobolev
@@ -257,6 +286,9 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
       if (r != ATUS_E_UNSUPPORTED) return r;
     }
   }
+  if constexpr (MODE == M2_NL && TC == 2 && !STRIDED) {
+    return a.nl.kind == K_BRAGG ? launch_pair_t<R, N, true>(ctx, a, axis) : launch_pair_t<R, N, false>(ctx, a, axis);
+  } else {
   using Cfg = P2Cfg<R, N, TC>;
   constexpr size_t smem = ((MODE == M2_KIN || MODE == M2_KIN_RABI) && Cfg::kin_smem) ? Cfg::smem_kin : Cfg::smem;
   static int resident = 0;
@@ -303,6 +335,7 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   pass2_kernel<R, N, TC, MODE, STRIDED><<<grid, Cfg::NT, smem, ctx->stream>>>(a);
   LAUNCHED(ctx);
   return ATUS_OK;
+  }
 }
 
 // Launch of pass3_kernel (pencils of 512..2048 points); as launch_pass2_t.

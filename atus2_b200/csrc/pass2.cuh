@@ -31,10 +31,16 @@ template <> struct Tile2<double> { static constexpr int E = 2048, NT = 128, MINB
 template <> struct Tile2<float> { static constexpr int E = 4096, NT = 256, MINB = 3; };
 
 // CTAs per SM the register budget is sized for: the passes at the ends of a
-// Sobolev iteration and the four-step passes hold potential values or
-// twiddles beside a thread's 16 points.
+// Sobolev iteration, the potential passes and the four-step passes hold
+// potential values or twiddles beside a thread's 16 points (256^3, one
+// component, z pass: 5 CTAs with spills 207 us, 4 without 178 us).
 template <typename R, int MODE>
-constexpr int p2_minb = (MODE >= M2_FWD_SOB && sizeof(R) == 8) ? 4 : Tile2<R>::MINB;
+constexpr int p2_minb =
+    (((MODE >= M2_FWD_SOB && MODE != M2_FILT) || MODE == M2_NL) && sizeof(R) == 8) ? 4 : Tile2<R>::MINB;
+
+// Passes whose two components meet inside a warp (the batched passes; a
+// single grid's run in pass2_pair.cuh).
+template <int TC, int MODE, bool STRIDED> constexpr bool p2_pair = (MODE == M2_NL && TC == 2 && !STRIDED);
 
 template <typename R, int N, int TC>
 struct P2Cfg {
@@ -68,8 +74,11 @@ __device__ __forceinline__ int ex_at(int row, int col) { return 17 * row + col; 
 // Twiddle W_N^{r k} is entry r of row k (pitch R2 + 1, odd): the eight threads
 // of a quarter warp, which hold eight different k on the contiguous axis, hit
 // eight different bank groups.
-template <typename R, int N, int DIR>
-__device__ __forceinline__ void p2_stage2(const cplx<R> *ex, const typename TwTab<R>::type *twS, int j, cplx<R> *o) {
+// sg (0 or the sign bit): with the odd inputs of every radix-R2 DFT negated its
+// outputs come out rotated by R2 / 2, so o[m] is point j + R2 (m ^ 8).
+template <typename R, int N, int DIR, bool FLIP = false>
+__device__ __forceinline__ void p2_stage2(const cplx<R> *ex, const typename TwTab<R>::type *twS, int j, cplx<R> *o,
+                                          int sg = 0) {
   using C = cplx<R>;
   constexpr int R2 = N / 16, T2 = 16 / R2;
   #pragma unroll
@@ -80,6 +89,10 @@ __device__ __forceinline__ void p2_stage2(const cplx<R> *ex, const typename TwTa
     for (int r = 0; r < R2; r++) u[r] = ex[ex_at(r, k)];
     #pragma unroll
     for (int r = 1; r < R2; r++) u[r] = twmul<DIR>(u[r], twS[k * (R2 + 1) + r]);
+    if constexpr (FLIP) {
+      #pragma unroll
+      for (int r = 1; r < R2; r += 2) u[r] = flip(u[r], sg);
+    }
     dftR<R2, DIR>(u);
     #pragma unroll
     for (int r = 0; r < R2; r++) o[t + T2 * r] = u[r];
@@ -91,15 +104,22 @@ __device__ __forceinline__ void p2_stage2(const cplx<R> *ex, const typename TwTa
 // that other threads may still be reading from the previous use.  WARP: the
 // R2 threads of each pencil are consecutive lanes of one warp (the contiguous
 // mapping), so the exchange needs only a warp barrier; the strided mapping
-// spreads a pencil over the CTA's warps and needs the CTA barrier.
-template <typename R, int N, int DIR, bool WARP = false>
-__device__ __forceinline__ void p2_transform(cplx<R> *v, cplx<R> *ex, const typename TwTab<R>::type *twS, int j) {
+// spreads a pencil over the CTA's warps and needs the CTA barrier.  FLIP (in
+// or out: 1 or 2) with sg set: the 16 values come in, or go out, in the order
+// m ^ 8 (inputs rotated by 8 negate the odd outputs of a 16-point DFT).
+template <typename R, int N, int DIR, bool WARP = false, int FLIP = 0>
+__device__ __forceinline__ void p2_transform(cplx<R> *v, cplx<R> *ex, const typename TwTab<R>::type *twS, int j,
+                                             int sg = 0) {
   dft16<DIR>(v);
+  if constexpr (FLIP == 1) {
+    #pragma unroll
+    for (int q = 1; q < 16; q += 2) v[q] = flip(v[q], sg);
+  }
   if constexpr (WARP) __syncwarp(); else __syncthreads();
   #pragma unroll
   for (int q = 0; q < 16; q++) ex[ex_at(j, q)] = v[q];
   if constexpr (WARP) __syncwarp(); else __syncthreads();
-  p2_stage2<R, N, DIR>(ex, twS, j, v);
+  p2_stage2<R, N, DIR, FLIP == 2>(ex, twS, j, v, sg);
 }
 
 // Shared-memory set-up of a CTA, once per launch: the twiddle rows and, for
@@ -121,7 +141,7 @@ __device__ __forceinline__ bool p2_setup(const PassArgs &a, unsigned char *smem_
   }
   // k-space passes: along-axis kinetic factors of components 0 and 1
   double2 *const s_kt = reinterpret_cast<double2 *>(smem_raw + Cfg::smem);
-  const bool kt_shared = (MODE == M2_KIN || MODE == M2_KIN_RABI) && Cfg::kin_smem && a.op == OP_KIN && a.ncomp_grid <= 2;
+  const bool kt_shared = (MODE == M2_KIN || MODE == M2_KIN_RABI) && Cfg::kin_smem && a.ncomp_grid <= 2;
   if (kt_shared) {
     for (int e = tid; e < a.ncomp_grid * N; e += NT) {
       const int cc = e / N, i = e % N;
@@ -133,7 +153,6 @@ __device__ __forceinline__ bool p2_setup(const PassArgs &a, unsigned char *smem_
   return kt_shared;
 }
 
-// One work item: the tile g of the pass described by a.
 // Rabi sums of one thread's 16 values (k-space points j + R2 m of the pencil
 // whose point 0 has axis indices p0) into rq, with the ball rule of
 // compute_rabi_integrals (include/CRT_Base_IF.h:231-257): a point inside a
@@ -168,6 +187,19 @@ __device__ __forceinline__ double sob_interaction(const PassArgs &a, int64_t l) 
     }
   }
   return nl;
+}
+
+// Bragg coupling of pencil b of tile g (contiguous axis).
+__device__ __forceinline__ void p2_coupling(const PassArgs &a, const TileGeo &g, int b, double &om, double &ec,
+                                            double &es) {
+  om = 0;
+  ec = 1;
+  es = 0;
+  if (b < g.nb) {
+    int ix, iy, iz;
+    idx3(a.g, g.base0 + b * g.pstride, ix, iy, iz);
+    bragg_coupling(a.nl, (double)(ix - a.nl.shift0) * a.nl.dx0, om, ec, es);
+  }
 }
 
 // After-load hook of p2_item (the TMA kernel refills the tile buffer there).
@@ -208,10 +240,15 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
   const TW *const twS = reinterpret_cast<const TW *>(smem_raw + Cfg::smem_ex);
   const double2 *const s_kt = reinterpret_cast<const double2 *>(smem_raw + Cfg::smem);
   const int tid = threadIdx.x;
+  // PAIR: the two components of a pencil in one warp, so that the potential
+  // step meets through shuffles (nl_pair16); exchange rows (b, c) at a pitch
+  // of 17 R2, which spreads the lanes of a bank group over the banks
+  constexpr bool PAIR = p2_pair<TC, MODE, STRIDED>;
   int b, j, c;
   if (STRIDED) { b = tid % B; j = (tid / B) % R2; c = tid / (B * R2); }
+  else if (PAIR) { j = tid % R2; c = (tid / R2) & 1; b = tid / (2 * R2); }
   else { j = tid % R2; b = (tid / R2) % B; c = tid / (R2 * B); }
-  C *const my = ex + (c * B + b) * PB;
+  C *const my = PAIR ? ex + (2 * b + c) * (17 * R2) : ex + (c * B + b) * PB;
   const int nc = a.per_comp ? 1 : a.nc;
   const bool live = (b < g.nb) && (c < nc);
   C *const f = (C *)pick(a.psi, g.comp0 + c);
@@ -219,7 +256,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
   const int64_t step = (int64_t)R2 * a.sa;     // distance of points j + R2 m and j + R2 (m+1)
   const C *src = live ? f + lb + (int64_t)j * a.sa : nullptr;
 
-  if constexpr (MODE == M2_NL && TC > 1) {
+  if constexpr (MODE == M2_NL && TC > 1 && !PAIR) {
     // coupling of each pencil (x is constant along it); read after the
     // barriers of the first transform
     if (a.nl.kind == K_BRAGG && a.axis != 0)
@@ -320,7 +357,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         }
       }
     }
-  } else if constexpr (MODE == M2_KIN || MODE == M2_KIN_RABI) {
+  } else if constexpr (MODE == M2_KIN || MODE == M2_KIN_RABI || MODE == M2_FILT) {
     p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
     int p0[3];
     idx3(a.g, lb, p0[0], p0[1], p0[2]);
@@ -330,40 +367,42 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         if (a.rabi_comp[c] == g.comp0) ci = c;
       if (live && ci >= 0) p2_rabi<R, N>(a, ci, p0, j, v, rq);
     }
-    if (a.op == OP_KIN) {
-      // psi^ <- ((psi^ s_f) K) s_b in FP64, K = K_along (product of the other
-      // two axis factors, x before y before z); complex64 fields take the
-      // scales folded into K
-      const double2 *kx = a.kt[0][0], *ky = a.kt[0][1], *kz = a.kt[0][2];
-      #pragma unroll
-      for (int cc = 1; cc < MAXC; cc++)
-        if (g.comp0 == cc) { kx = a.kt[cc][0]; ky = a.kt[cc][1]; kz = a.kt[cc][2]; }
-      const double2 KX = __ldg(&kx[p0[0]]), KY = __ldg(&ky[p0[1]]), KZ = __ldg(&kz[p0[2]]);
-      double2 Kp = (a.axis == 0) ? cmul(KY, KZ) : (a.axis == 1) ? cmul(KX, KZ) : cmul(KX, KY);
-      const double2 *along = (a.axis == 0) ? kx : (a.axis == 1) ? ky : kz;
-      const double2 *sk = s_kt + (g.comp0 == 1 ? N : 0);
-      if (sizeof(R) == 4) {
-        const double sc = a.s_f * a.s_b;
-        Kp.x *= sc;
-        Kp.y *= sc;
-      }
-      #pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const int i = j + R2 * m;
-        const double2 K = cmul(kt_shared ? sk[i] : __ldg(&along[i]), Kp);
-        double2 u = to_d<R>(v[m]);
-        if (sizeof(R) == 8) {
-          u.x *= a.s_f;
-          u.y *= a.s_f;
+    if constexpr (MODE != M2_FILT) {
+      if (a.op == OP_KIN) {  // always: a branch keeps the factors' loads out of the transform above
+        // psi^ <- ((psi^ s_f) K) s_b in FP64, K = K_along (product of the other
+        // two axis factors, x before y before z); complex64 fields take the
+        // scales folded into K
+        const double2 *kx = a.kt[0][0], *ky = a.kt[0][1], *kz = a.kt[0][2];
+        #pragma unroll
+        for (int cc = 1; cc < MAXC; cc++)
+          if (g.comp0 == cc) { kx = a.kt[cc][0]; ky = a.kt[cc][1]; kz = a.kt[cc][2]; }
+        const double2 KX = __ldg(&kx[p0[0]]), KY = __ldg(&ky[p0[1]]), KZ = __ldg(&kz[p0[2]]);
+        double2 Kp = (a.axis == 0) ? cmul(KY, KZ) : (a.axis == 1) ? cmul(KX, KZ) : cmul(KX, KY);
+        const double2 *along = (a.axis == 0) ? kx : (a.axis == 1) ? ky : kz;
+        const double2 *sk = s_kt + (g.comp0 == 1 ? N : 0);
+        if (sizeof(R) == 4) {
+          const double sc = a.s_f * a.s_b;
+          Kp.x *= sc;
+          Kp.y *= sc;
         }
-        u = cmul(u, K);
-        if (sizeof(R) == 8) {
-          u.x *= a.s_b;
-          u.y *= a.s_b;
+        #pragma unroll
+        for (int m = 0; m < 16; m++) {
+          const int i = j + R2 * m;
+          const double2 K = cmul(kt_shared ? sk[i] : __ldg(&along[i]), Kp);
+          double2 u = to_d<R>(v[m]);
+          if (sizeof(R) == 8) {
+            u.x *= a.s_f;
+            u.y *= a.s_f;
+          }
+          u = cmul(u, K);
+          if (sizeof(R) == 8) {
+            u.x *= a.s_b;
+            u.y *= a.s_b;
+          }
+          v[m] = from_d<R>(u);
         }
-        v[m] = from_d<R>(u);
       }
-    } else if (a.op == OP_FILT) {
+    } else {
       // alpha k^2 of the pencil's two fixed axes, and of the point's own
       auto ak2 = [&](int ax, int ii) {
         const int sh = a.n[ax] >> 1;  // lengths are powers of two
@@ -406,8 +445,15 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
   } else {  // M2_NL, M2_FS_NL: IFFT -> potential step -> FFT
     constexpr bool FS = (MODE == M2_FS_NL);  // axis 0 is the whole grid index
-    p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
-    if constexpr (TC == 1) {
+    const int sg = (PAIR && c) ? (int)0x80000000 : 0;
+    p2_transform<R, N, +1, !STRIDED, PAIR ? 2 : 0>(v, my, twS, j, sg);
+    if constexpr (PAIR) {
+      int p0[3];
+      idx3(a.g, lb, p0[0], p0[1], p0[2]);
+      const double x0 = (double)(p0[0] - a.nl.shift0) * a.nl.dx0;
+      if (a.nl.kind == K_BRAGG) nl_pair16<R, true>(a.nl, v, c, R2, live, x0, s_om[b], s_ec[b], s_es[b], lb + j, R2);
+      else nl_pair16<R, false>(a.nl, v, c, R2, live, x0, 0.0, 1.0, 0.0, lb + j, R2);
+    } else if constexpr (TC == 1) {
       int p0[3];
       idx3(a.g, lb, p0[0], p0[1], p0[2]);
       // the potential, loaded four points ahead of its use (behind the
@@ -474,7 +520,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         v[r] = my[ex_at(i >> 4, i & 15)];
       }
     }
-    p2_transform<R, N, -1, !STRIDED>(v, my, twS, j);
+    p2_transform<R, N, -1, !STRIDED, PAIR ? 1 : 0>(v, my, twS, j, sg);
     if constexpr (FS) fs_twiddle(std::integral_constant<int, -1>());
   }
 

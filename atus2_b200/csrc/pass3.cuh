@@ -49,7 +49,8 @@ struct P3Cfg {
   // PB = G / B (mod G) puts them on G distinct banks (the rows' own offsets
   // are t mod G, 17 M = 0 mod G).  Contiguous tiles: a group is one pencil.
   static constexpr int G = 128 / (int)sizeof(cplx<R>);
-  static constexpr int PB = 17 * M + ((STRIDED && B < G) ? G / B : 1);
+  // Contiguous tiles of two components: G / 2 consecutive t of both.
+  static constexpr int PB = 17 * M + ((STRIDED && B < G) ? G / B : (!STRIDED && TC == 2) ? G / 2 : 1);
   static constexpr size_t smem_ex = sizeof(cplx<R>) * NPC * PB;
   // W_N^{t q} (row q, column t) and W_M^{j2 q2} (row q2, column j2)
   static constexpr int TWN_N = 16 * M, TWN_M = 16 * R3;
@@ -63,13 +64,18 @@ struct P3Cfg {
 
 // One transform of the thread's 16 values v (inputs t + M r on entry, points
 // t + M r on return).  ex: the pencil-component's exchange rows.
-template <typename R, int N, int DIR>
+// FLIP (1: in, 2: out) with sg set: order m ^ 8, as in p2_transform.
+template <typename R, int N, int DIR, int FLIP = 0>
 __device__ __forceinline__ void p3_transform(cplx<R> *v, cplx<R> *ex, const typename TwTab<R>::type *twN,
-                                             const typename TwTab<R>::type *twM, int t) {
+                                             const typename TwTab<R>::type *twM, int t, int sg = 0) {
   using C = cplx<R>;
   constexpr int M = N / 16, R3 = M / 16, T3 = 16 / R3;
   // stage 1: radix 16 over r, twiddles W_N^{t q}
   dft16<DIR>(v);
+  if constexpr (FLIP == 1) {
+    #pragma unroll
+    for (int q = 1; q < 16; q += 2) v[q] = flip(v[q], sg);
+  }
   #pragma unroll
   for (int q = 1; q < 16; q++) v[q] = twmul<DIR>(v[q], twN[q * M + t]);
   __syncthreads();
@@ -94,6 +100,10 @@ __device__ __forceinline__ void p3_transform(cplx<R> *v, cplx<R> *ex, const type
     C u[R3];
     #pragma unroll
     for (int jj = 0; jj < R3; jj++) u[jj] = ex[qa + 16 * (jj + R3 * (q2p + R3 * s))];
+    if constexpr (FLIP == 2) {
+      #pragma unroll
+      for (int jj = 1; jj < R3; jj += 2) u[jj] = flip(u[jj], sg);
+    }
     dftR<R3, DIR>(u);
     #pragma unroll
     for (int k3 = 0; k3 < R3; k3++) v[s + T3 * k3] = u[k3];
@@ -132,10 +142,14 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
   const TW *const twN = reinterpret_cast<const TW *>(smem_raw + Cfg::smem_ex);
   const TW *const twM = twN + Cfg::TWN_N;
   const int tid = threadIdx.x;
+  // PAIR: the components of a pencil on alternate lanes, so that the
+  // potential step meets through shuffles (nl_pair16)
+  constexpr bool PAIR = p2_pair<TC, MODE, STRIDED>;
   int b, t, c;
   if (STRIDED) { b = tid % B; t = (tid / B) % M; c = tid / (B * M); }
+  else if (PAIR) { c = tid & 1; t = (tid >> 1) % M; b = tid / (2 * M); }
   else { t = tid % M; b = (tid / M) % B; c = tid / (M * B); }
-  C *const my = ex + (c * B + b) * PB;
+  C *const my = ex + (PAIR ? 2 * b + c : c * B + b) * PB;
   const int nc = a.per_comp ? 1 : a.nc;
   const bool live = (b < g.nb) && (c < nc);
   C *const f = (C *)pick(a.psi, g.comp0 + c);
@@ -196,42 +210,44 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
     p3_transform<R, N, -1>(v, my, twN, twM, t);
   } else if constexpr (MODE == M2_INV) {
     p3_transform<R, N, +1>(v, my, twN, twM, t);
-  } else if constexpr (MODE == M2_KIN) {
+  } else if constexpr (MODE == M2_KIN || MODE == M2_FILT) {
     p3_transform<R, N, -1>(v, my, twN, twM, t);
     int p0[3];
     idx3(a.g, lb, p0[0], p0[1], p0[2]);
-    if (a.op == OP_KIN) {
-      // psi^ <- ((psi^ s_f) K) s_b in FP64 (complex64 fields: the scales
-      // folded into K), K = K_along x the product of the other axis factors
-      const double2 *kx = a.kt[0][0], *ky = a.kt[0][1], *kz = a.kt[0][2];
-      #pragma unroll
-      for (int cc = 1; cc < MAXC; cc++)
-        if (g.comp0 == cc) { kx = a.kt[cc][0]; ky = a.kt[cc][1]; kz = a.kt[cc][2]; }
-      const double2 KX = __ldg(&kx[p0[0]]), KY = __ldg(&ky[p0[1]]), KZ = __ldg(&kz[p0[2]]);
-      double2 Kp = (a.axis == 0) ? cmul(KY, KZ) : (a.axis == 1) ? cmul(KX, KZ) : cmul(KX, KY);
-      const double2 *along = (a.axis == 0) ? kx : (a.axis == 1) ? ky : kz;
-      if (sizeof(R) == 4) {
-        const double sc = a.s_f * a.s_b;
-        Kp.x *= sc;
-        Kp.y *= sc;
-      }
-      #pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const int i = t + M * m;
-        const double2 K = cmul(__ldg(&along[i]), Kp);
-        double2 u = to_d<R>(v[m]);
-        if (sizeof(R) == 8) {
-          u.x *= a.s_f;
-          u.y *= a.s_f;
+    if constexpr (MODE == M2_KIN) {
+      if (a.op == OP_KIN) {  // always: a branch keeps the factors' loads out of the transform above
+        // psi^ <- ((psi^ s_f) K) s_b in FP64 (complex64 fields: the scales
+        // folded into K), K = K_along x the product of the other axis factors
+        const double2 *kx = a.kt[0][0], *ky = a.kt[0][1], *kz = a.kt[0][2];
+        #pragma unroll
+        for (int cc = 1; cc < MAXC; cc++)
+          if (g.comp0 == cc) { kx = a.kt[cc][0]; ky = a.kt[cc][1]; kz = a.kt[cc][2]; }
+        const double2 KX = __ldg(&kx[p0[0]]), KY = __ldg(&ky[p0[1]]), KZ = __ldg(&kz[p0[2]]);
+        double2 Kp = (a.axis == 0) ? cmul(KY, KZ) : (a.axis == 1) ? cmul(KX, KZ) : cmul(KX, KY);
+        const double2 *along = (a.axis == 0) ? kx : (a.axis == 1) ? ky : kz;
+        if (sizeof(R) == 4) {
+          const double sc = a.s_f * a.s_b;
+          Kp.x *= sc;
+          Kp.y *= sc;
         }
-        u = cmul(u, K);
-        if (sizeof(R) == 8) {
-          u.x *= a.s_b;
-          u.y *= a.s_b;
+        #pragma unroll
+        for (int m = 0; m < 16; m++) {
+          const int i = t + M * m;
+          const double2 K = cmul(__ldg(&along[i]), Kp);
+          double2 u = to_d<R>(v[m]);
+          if (sizeof(R) == 8) {
+            u.x *= a.s_f;
+            u.y *= a.s_f;
+          }
+          u = cmul(u, K);
+          if (sizeof(R) == 8) {
+            u.x *= a.s_b;
+            u.y *= a.s_b;
+          }
+          v[m] = from_d<R>(u);
         }
-        v[m] = from_d<R>(u);
       }
-    } else if (a.op == OP_FILT) {
+    } else {
       #pragma unroll
       for (int m = 0; m < 16; m++) {
         const int i = t + M * m;
@@ -251,8 +267,15 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
     p3_transform<R, N, +1>(v, my, twN, twM, t);
   } else {  // M2_NL, M2_FS_NL: IFFT -> potential step -> FFT
     constexpr bool FS = (MODE == M2_FS_NL);  // axis 0 is the whole grid index
-    p3_transform<R, N, +1>(v, my, twN, twM, t);
-    if constexpr (TC == 1) {
+    const int sg = (PAIR && c) ? (int)0x80000000 : 0;
+    p3_transform<R, N, +1, PAIR ? 2 : 0>(v, my, twN, twM, t, sg);
+    if constexpr (PAIR) {
+      int p0[3];
+      idx3(a.g, lb, p0[0], p0[1], p0[2]);
+      const double x0 = (double)(p0[0] - a.nl.shift0) * a.nl.dx0;
+      if (a.nl.kind == K_BRAGG) nl_pair16<R, true>(a.nl, v, c, 1, live, x0, s_om[b], s_ec[b], s_es[b], lb + t, M);
+      else nl_pair16<R, false>(a.nl, v, c, 1, live, x0, 0.0, 1.0, 0.0, lb + t, M);
+    } else if constexpr (TC == 1) {
       int p0[3];
       idx3(a.g, lb, p0[0], p0[1], p0[2]);
       constexpr int AHEAD = 8;  // potential loads in flight
@@ -315,7 +338,7 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
         v[m] = my[ex_at(i >> 4, i & 15)];
       }
     }
-    p3_transform<R, N, -1>(v, my, twN, twM, t);
+    p3_transform<R, N, -1, PAIR ? 1 : 0>(v, my, twN, twM, t, sg);
     if constexpr (FS) fs_twiddle(std::integral_constant<int, -1>());
   }
 
