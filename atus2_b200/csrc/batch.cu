@@ -23,8 +23,8 @@
 
 using namespace atus;
 
-bool batch1d_info_f(int N, int NT, int RES, BKernel *k);
-bool batch1d_info_d(int N, int NT, int RES, BKernel *k);
+bool batch1d_info_f(int N, int C, BKernel *k);
+bool batch1d_info_d(int N, int C, BKernel *k);
 bool batch2d_p2_info_f(int N, int mode, BKernel *k);
 bool batch2d_p2_info_d(int N, int mode, BKernel *k);
 bool batch2d_tile_info_f(int N, int mode, BKernel *k);
@@ -36,7 +36,7 @@ namespace {
 enum { P_FWD = 0, P_INV = 1, P_KH = 2, P_KF = 3, P_POT = 4, NPASS = 5 };
 
 struct Variant {
-  int a = 0, b = 0;  // 1D: threads, resident components; 2D: BV_P2 / BV_TILE
+  int a = 0;  // 1D: CTAs an instance runs on; 2D: BV_P2 / BV_P5 / BV_TILE
 };
 
 struct Class {
@@ -73,7 +73,7 @@ struct atus_batch {
   std::vector<double> t;           // header times
   std::vector<void *> psi[2];
   std::vector<double2 *> kt[2][2]; // [half/full][axis] per instance
-  BInst1 *d_b1 = nullptr;          // per batch index (1D entries used)
+  LineInst *d_b1 = nullptr;          // per batch index (1D entries used)
   Pulse *d_pulse = nullptr;
   double *d_t0 = nullptr, *h_t0 = nullptr;
   void *tw = nullptr;              // twiddles in the field precision
@@ -107,7 +107,7 @@ int64_t npts(const atus_batch_instance &in) {
 }
 
 bool info1d(const atus_batch *b, int N, const Variant &v, BKernel *k) {
-  return b->prec == ATUS_PREC_FP64 ? batch1d_info_d(N, v.a, v.b, k) : batch1d_info_f(N, v.a, v.b, k);
+  return b->prec == ATUS_PREC_FP64 ? batch1d_info_d(N, v.a, k) : batch1d_info_f(N, v.a, k);
 }
 bool info2d(const atus_batch *b, int N, int variant, int mode, BKernel *k) {
   if (variant == BV_P2)
@@ -206,26 +206,51 @@ int build_2d_args(atus_batch *b, Class &c) {
   return ATUS_OK;
 }
 
+cudaLaunchConfig_t cluster_config(const BKernel &k, int grid, cudaStream_t s, cudaLaunchAttribute *attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(k.nt);
+  cfg.dynamicSmemBytes = k.smem;
+  cfg.stream = s;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = k.cluster;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = k.cluster > 1 ? 1 : 0;
+  return cfg;
+}
+
 // Shared-memory attribute and occupancy of a kernel, set up once outside
 // any stream capture.
 int prepare(atus_batch *b, const BKernel &k) {
   if (b->resident.count(k.fn)) return ATUS_OK;
   BCK(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
   int res = 0;
-  BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, k.fn, k.nt, k.smem));
+  if (k.cluster > 1) {  // clusters the device holds at once
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = cluster_config(k, k.cluster, nullptr, &attr);
+    BCK(cudaOccupancyMaxActiveClusters(&res, k.fn, &cfg));
+  } else {
+    BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, k.fn, k.nt, k.smem));
+  }
   if (res < 1) return fail(b, ATUS_E_UNSUPPORTED, "batch kernel does not fit on an SM");
   b->resident[k.fn] = res;
   return ATUS_OK;
 }
 
 int launch(atus_batch *b, const BKernel &k, int grid, void **args, cudaStream_t s) {
-  BCK(cudaLaunchKernel(k.fn, dim3(grid), dim3(k.nt), args, k.smem, s));
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = cluster_config(k, grid, s, &attr);
+  BCK(cudaLaunchKernelExC(&cfg, k.fn, args));
   return ATUS_OK;
 }
 
 int grid_for(atus_batch *b, const BKernel &k, int64_t work) {
   auto it = b->resident.find(k.fn);
   const int res = it == b->resident.end() ? 1 : it->second;
+  // a cluster kernel's work items and slots are clusters
+  if (k.cluster > 1) return k.cluster * (int)std::max<int64_t>(1, std::min<int64_t>(work, res));
   const int64_t slots = (int64_t)b->nsm * res;
   return (int)std::max<int64_t>(1, std::min<int64_t>(work, slots));
 }
@@ -236,13 +261,13 @@ int enqueue_class(atus_batch *b, Class &c, int nk, cudaStream_t s) {
   if (c.dim == 1) {
     BKernel k;
     if (!info1d(b, c.n, c.v, &k)) return fail(b, ATUS_E_UNSUPPORTED, "no 1D batch kernel for this variant");
-    const BInst1 *insts = b->d_b1;
+    const LineInst *insts = b->d_b1;
     const int *order = c.d_ids;
     const double *t0 = b->d_t0;
     int ninst = m;
     const void *tw = b->tw;
     void *args[] = {(void *)&insts, (void *)&order, (void *)&t0, (void *)&ninst, (void *)&nk, (void *)&tw};
-    // one CTA per instance: the whole block of an instance runs in one CTA
+    // the whole block of an instance runs in one CTA or one cluster
     return launch(b, k, grid_for(b, k, m), args, s);
   }
   auto pass = [&](int p, int step) -> int {
@@ -277,7 +302,7 @@ void drop_graphs(atus_batch *b) {
 
 std::string variant_name(const Class &c, const Variant &v) {
   char buf[64];
-  if (c.dim == 1) snprintf(buf, sizeof(buf), "%d threads, %d resident", v.a, v.b);
+  if (c.dim == 1) snprintf(buf, sizeof(buf), "%d CTA%s per instance", v.a, v.a > 1 ? "s" : "");
   else snprintf(buf, sizeof(buf), "%s", v.a == BV_P2 ? "register-staged passes" : v.a == BV_P5 ? "register-staged 512-point passes" : "shared-memory tile passes");
   return buf;
 }
@@ -349,7 +374,7 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
   for (int c = 0; c < 2; c++) b->psi[c].assign(count, nullptr);
   for (int h = 0; h < 2; h++)
     for (int ax = 0; ax < 2; ax++) b->kt[h][ax].assign(count, nullptr);
-  std::vector<BInst1> b1(count);
+  std::vector<LineInst> b1(count);
   std::vector<Pulse> pulse(count);
   for (int i = 0; i < count; i++) {
     const atus_batch_instance &in = inst[i];
@@ -374,11 +399,13 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     }
     pulse[i].tc = in.pulse_tc;
     pulse[i].two_sigma2 = in.pulse_sigma > 0 ? 2.0 * in.pulse_sigma * in.pulse_sigma : 0.0;
-    memset(&b1[i], 0, sizeof(BInst1));
+    memset(&b1[i], 0, sizeof(LineInst));
     b1[i].psi[0] = b->psi[0][i];
     b1[i].psi[1] = b->psi[1][i];
-    b1[i].kh = b->kt[0][0][i];
-    b1[i].kf = b->kt[1][0][i];
+    for (int c = 0; c < 2; c++) {
+      b1[i].kh[c] = b->kt[0][0][i];
+      b1[i].kf[c] = b->kt[1][0][i];
+    }
     b1[i].s_f = scale_fak(1, in.grid.d);
     b1[i].s_b = scale_fak(1, in.grid.dk);
     b1[i].pulse = pulse[i];
@@ -389,12 +416,12 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     if (cudaMalloc(&b->unit, sizeof(double2)) != cudaSuccess) return bail(ATUS_E_NOMEM);
     cudaMemcpy(b->unit, &one, sizeof(double2), cudaMemcpyHostToDevice);
   }
-  if (cudaMalloc(&b->d_b1, sizeof(BInst1) * count) != cudaSuccess ||
+  if (cudaMalloc(&b->d_b1, sizeof(LineInst) * count) != cudaSuccess ||
       cudaMalloc(&b->d_pulse, sizeof(Pulse) * count) != cudaSuccess ||
       cudaMalloc(&b->d_t0, sizeof(double) * count) != cudaSuccess ||
       cudaMallocHost(&b->h_t0, sizeof(double) * count) != cudaSuccess)
     return bail(ATUS_E_NOMEM);
-  cudaMemcpy(b->d_b1, b1.data(), sizeof(BInst1) * count, cudaMemcpyHostToDevice);
+  cudaMemcpy(b->d_b1, b1.data(), sizeof(LineInst) * count, cudaMemcpyHostToDevice);
   cudaMemcpy(b->d_pulse, pulse.data(), sizeof(Pulse) * count, cudaMemcpyHostToDevice);
   // size classes, instances longest run first (equal here) in batch order
   std::map<std::pair<int, int>, int> key;
@@ -414,13 +441,14 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     cudaMemcpy(c.d_ids, c.ids.data(), sizeof(int) * c.ids.size(), cudaMemcpyHostToDevice);
     BKernel k;
     if (c.dim == 1) {
-      for (int res : {2, 1})
-        for (int nt : {256, 512}) {
-          Variant v;
-          v.a = nt;
-          v.b = res;
-          if (info1d(b, c.n, v, &k)) c.cands.push_back(v);
-        }
+      for (int ctas : {1, 2, 4, 8}) {
+        Variant v;
+        v.a = ctas;
+        if (!info1d(b, c.n, v, &k)) continue;
+        const int r = prepare(b, k);
+        if (r == ATUS_OK) c.cands.push_back(v);
+        else if (ctas == 1 || b->err.find("does not fit") == std::string::npos) return bail(ATUS_E_CUDA);
+      }
     } else {
       for (int var : {BV_P2, BV_P5, BV_TILE}) {
         Variant v;
@@ -430,9 +458,7 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     }
     if (c.cands.empty()) return bail(fail(b, ATUS_E_UNSUPPORTED, "no batch kernel for a size class"));
     for (const Variant &v : c.cands) {
-      if (c.dim == 1) {
-        if (info1d(b, c.n, v, &k) && prepare(b, k) != ATUS_OK) return bail(ATUS_E_CUDA);
-      } else {
+      if (c.dim == 2) {
         for (int mode : {M2_FWD, M2_INV, M2_KIN, M2_NL})
           if (info2d(b, c.n, v.a, mode, &k) && prepare(b, k) != ATUS_OK) return bail(ATUS_E_CUDA);
       }

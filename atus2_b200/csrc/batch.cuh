@@ -2,32 +2,21 @@
 // Bragg instances (parameter sweeps over pulse area, detuning, interaction
 // strength and pulse length) with uneven grids.
 //
-// 1D instances: batch1d_kernel, one CTA per instance, persistent over the
-//   instances of one grid length and over the whole Strang block
-//   half, (V, full)^(nk-1), V, half  (include/CRT_Base_IF.h:779-789 with the
-//   Bragg step of source/interferometry/src/bragg.cpp:185-304).  RES = 2 keeps
-//   both components in shared memory; RES = 1 keeps one and parks the other
-//   in global memory (L2), swapping them around each kinetic step -- for
-//   grids whose two components do not fit (16384 complex64 points).  The
-//   Gaussian pulse envelope F(t) is evaluated on the device.
+// 1D instances: line1d_batch_kernel (line1d.cuh), one CTA or one cluster of
+//   CTAs per instance, persistent over the instances of one grid length and
+//   over the whole Strang block half, (V, full)^(nk-1), V, half
+//   (include/CRT_Base_IF.h:779-789 with the Bragg step of
+//   source/interferometry/src/bragg.cpp:185-304), both components on chip.
+//   The Gaussian pulse envelope F(t) is evaluated on the device.
 // 2D instances: batch_pass2_kernel / batch_tile_kernel run one pass (the
 //   same passes as a single 2D context) over the tiles of every instance of a
 //   size class; the tile of work item w belongs to instance w / tiles.
 #pragma once
+#include "line1d.cuh"
 #include "pass2.cuh"
 #include "pass512.cuh"
 
 namespace atus {
-
-// Gaussian pulse envelope exp(-(t - tc)^2 / (2 sigma^2)); two_sigma2 <= 0: 1.
-struct Pulse {
-  double tc, two_sigma2;
-};
-__device__ __forceinline__ double pulse_at(const Pulse &p, double t) {
-  if (p.two_sigma2 <= 0.0) return 1.0;
-  const double u = t - p.tc;
-  return exp(-(u * u) / p.two_sigma2);
-}
 
 // Bragg coupling of complex64 instances: FP64 phase arguments reduced modulo
 // 2 pi, FP32 cos / sincos -- coupling accurate to FP32 for FP32 fields.  FP64
@@ -48,159 +37,6 @@ template <typename R>
 __device__ __forceinline__ void coupling_at(const NLArgs &a, double x0, double &om, double &ec, double &es) {
   if constexpr (sizeof(R) == 8) bragg_coupling(a, x0, om, ec, es);
   else bragg_coupling_mixed(a, x0, om, ec, es);
-}
-
-// ------------------------------------------------------------------ 1D
-struct BInst1 {
-  void *psi[2];            // device fields of the instance
-  const double2 *kh, *kf;  // half / full kinetic factors (FP64, N entries)
-  double s_f, s_b;         // transform scales
-  Pulse pulse;
-  NLArgs nl;               // Bragg step parameters (kind K_BRAGG, ncomp 2)
-};
-
-// psi^ <- ((psi^ s_f) K) s_b, K in FP64 (as kin_1d).
-template <typename R, int N, int NT>
-__device__ __forceinline__ void b1_kin(cplx<R> *s, const double2 *tab, double s_f, double s_b) {
-  for (int i = threadIdx.x; i < N; i += NT) {
-    const int si = Pad<N>::idx(0, i);
-    double2 v = to_d<R>(s[si]);
-    v.x *= s_f;
-    v.y *= s_f;
-    v = cmul(v, __ldg(&tab[i]));
-    v.x *= s_b;
-    v.y *= s_b;
-    s[si] = from_d<R>(v);
-  }
-  __syncthreads();
-}
-
-// One kinetic step of the component held in s.
-template <typename R, int N, int NT>
-__device__ __forceinline__ void b1_kinetic(cplx<R> *s, const typename TwTab<R>::type *tw, const double2 *tab,
-                                           double s_f, double s_b) {
-  fft_tile<R, N, 1, NT, -1, TWN>(s, tw);
-  b1_kin<R, N, NT>(s, tab, s_f, s_b);
-  fft_tile<R, N, 1, NT, +1, TWN>(s, tw);
-}
-
-template <typename R, int N, int NT, int RES>
-__device__ __forceinline__ void b1_load(cplx<R> *s, const cplx<R> *src) {
-  for (int i = threadIdx.x; i < N; i += NT) s[Pad<N>::idx(0, i)] = src[i];
-}
-template <typename R, int N, int NT, int RES>
-__device__ __forceinline__ void b1_store(const cplx<R> *s, cplx<R> *dst) {
-  for (int i = threadIdx.x; i < N; i += NT) dst[i] = s[Pad<N>::idx(0, i)];
-}
-
-template <typename R, int N, int NT, int RES>
-__global__ void __launch_bounds__(NT) batch1d_kernel(const BInst1 *__restrict__ insts, const int *__restrict__ order,
-                                                     const double *__restrict__ t0, int ninst, int nk, const void *twv) {
-  // insts and t0 are indexed by batch index; order lists the class's instances
-  using C = cplx<R>;
-  constexpr int NP = Pad<N>::NP;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *const s = reinterpret_cast<C *>(smem_raw);
-  const typename TwTab<R>::type *tw = (const typename TwTab<R>::type *)twv;
-  // the instance's Bragg parameters live in shared memory (thread 0 sets the
-  // step's time and pulse amplitude): a per-thread copy of the ~0.5 KB block
-  // sat in local memory
-  __shared__ NLArgs s_nl;
-  const NLArgs &nl = s_nl;
-  for (int k = blockIdx.x; k < ninst; k += gridDim.x) {
-    const int id = order[k];
-    const BInst1 &in = insts[id];
-    C *fld[2] = {(C *)in.psi[0], (C *)in.psi[1]};
-    {
-      static_assert(sizeof(NLArgs) % 8 == 0, "NLArgs is copied in 8-byte words");
-      const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&in.nl);
-      unsigned long long *dst = reinterpret_cast<unsigned long long *>(&s_nl);
-      for (int e = threadIdx.x; e < (int)(sizeof(NLArgs) / 8); e += NT) dst[e] = src[e];
-    }
-    __syncthreads();
-    const double dt = nl.dt;
-    double t = t0[id];
-    if constexpr (RES == 2) {
-      b1_load<R, N, NT, RES>(s, fld[0]);
-      b1_load<R, N, NT, RES>(s + NP, fld[1]);
-      __syncthreads();
-      b1_kinetic<R, N, NT>(s, tw, in.kh, in.s_f, in.s_b);
-      b1_kinetic<R, N, NT>(s + NP, tw, in.kh, in.s_f, in.s_b);
-      t += 0.5 * dt;
-      for (int j = 0; j < nk; j++) {
-        if (threadIdx.x == 0) {
-          s_nl.t1 = t + 0.5 * dt;
-          s_nl.F = pulse_at(in.pulse, s_nl.t1);
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < N; i += NT) {
-          const double x0 = (double)(i - nl.shift0) * nl.dx0;
-          double om, ec, es;
-          coupling_at<R>(nl, x0, om, ec, es);
-          C v[MAXC];
-          v[0] = s[Pad<N>::idx(0, i)];
-          v[1] = s[NP + Pad<N>::idx(0, i)];
-          nl_point<R, 2>(nl, v, i, x0, om, ec, es);
-          s[Pad<N>::idx(0, i)] = v[0];
-          s[NP + Pad<N>::idx(0, i)] = v[1];
-        }
-        __syncthreads();
-        const bool last = (j == nk - 1);
-        const double2 *tab = last ? in.kh : in.kf;
-        b1_kinetic<R, N, NT>(s, tw, tab, in.s_f, in.s_b);
-        b1_kinetic<R, N, NT>(s + NP, tw, tab, in.s_f, in.s_b);
-        t += last ? 0.5 * dt : dt;
-      }
-      b1_store<R, N, NT, RES>(s, fld[0]);
-      b1_store<R, N, NT, RES>(s + NP, fld[1]);
-    } else {
-      // one component resident (index rc), the other in global memory
-      int rc = 0;
-      b1_load<R, N, NT, RES>(s, fld[0]);
-      __syncthreads();
-      b1_kinetic<R, N, NT>(s, tw, in.kh, in.s_f, in.s_b);
-      b1_store<R, N, NT, RES>(s, fld[0]);
-      __syncthreads();
-      b1_load<R, N, NT, RES>(s, fld[1]);
-      rc = 1;
-      __syncthreads();
-      b1_kinetic<R, N, NT>(s, tw, in.kh, in.s_f, in.s_b);
-      t += 0.5 * dt;
-      for (int j = 0; j < nk; j++) {
-        if (threadIdx.x == 0) {
-          s_nl.t1 = t + 0.5 * dt;
-          s_nl.F = pulse_at(in.pulse, s_nl.t1);
-        }
-        __syncthreads();
-        C *other = fld[rc ^ 1];
-        for (int i = threadIdx.x; i < N; i += NT) {
-          const double x0 = (double)(i - nl.shift0) * nl.dx0;
-          double om, ec, es;
-          coupling_at<R>(nl, x0, om, ec, es);
-          const C res = s[Pad<N>::idx(0, i)], oth = other[i];
-          C v[MAXC];
-          v[0] = rc ? oth : res;
-          v[1] = rc ? res : oth;
-          nl_point<R, 2>(nl, v, i, x0, om, ec, es);
-          s[Pad<N>::idx(0, i)] = rc ? v[1] : v[0];
-          other[i] = rc ? v[0] : v[1];
-        }
-        __syncthreads();
-        const bool last = (j == nk - 1);
-        const double2 *tab = last ? in.kh : in.kf;
-        b1_kinetic<R, N, NT>(s, tw, tab, in.s_f, in.s_b);
-        b1_store<R, N, NT, RES>(s, fld[rc]);
-        __syncthreads();
-        rc ^= 1;
-        b1_load<R, N, NT, RES>(s, fld[rc]);
-        __syncthreads();
-        b1_kinetic<R, N, NT>(s, tw, tab, in.s_f, in.s_b);
-        t += last ? 0.5 * dt : dt;
-      }
-      b1_store<R, N, NT, RES>(s, fld[rc]);
-    }
-    __syncthreads();  // shared memory is reused by the next instance
-  }
 }
 
 // ------------------------------------------------------------------ 2D
@@ -418,6 +254,7 @@ __global__ void __launch_bounds__(Tile<R>::NT) batch_tile_kernel(BPass bp) {
 // of one kernel instantiation, for the host's generic launches.
 struct BKernel {
   const void *fn;
+  int cluster = 1;  // CTAs a launch groups into a cluster
   int nt;
   size_t smem;
   int B;

@@ -1,25 +1,41 @@
-// Batched 1D Strang-block kernels, double fields: every (length, threads,
-// resident components) combination the autotuner may pick.
+// Batched 1D Strang-block kernels, double fields: every (length, CTAs a run)
+// combination the autotuner may pick.
 #include "batch.cuh"
 
 using namespace atus;
 
-template <int N, int NT, int RES>
+template <int N, int C>
 static bool k1(BKernel *k) {
-  k->fn = (const void *)batch1d_kernel<double, N, NT, RES>;
-  k->nt = NT;
-  k->smem = sizeof(cplx<double>) * Pad<N>::NP * RES;
-  k->B = 0;
-  return true;
+  using Cfg = LineCfg<double, N, 2, C>;
+  if constexpr (Cfg::fits) {
+    k->fn = (const void *)line1d_batch_kernel<double, N, C>;
+    k->nt = Cfg::NT;
+    k->smem = Cfg::smem;
+    k->B = 0;
+    k->cluster = C;
+    return true;
+  } else {
+    return false;
+  }
+}
+template <int N>
+static bool k1c(int C, BKernel *k) {
+  switch (C) {
+    case 1: return k1<N, 1>(k);
+    case 2: return k1<N, 2>(k);
+    case 4: return k1<N, 4>(k);
+    case 8: return k1<N, 8>(k);
+    default: return false;
+  }
 }
 
-bool batch1d_info_d(int N, int NT, int RES, BKernel *k) {
-  if (N == 1024 && NT == 256 && RES == 2) return k1<1024, 256, 2>(k);
-  if (N == 1024 && NT == 256 && RES == 1) return k1<1024, 256, 1>(k);
-  if (N == 2048 && NT == 256 && RES == 2) return k1<2048, 256, 2>(k);
-  if (N == 2048 && NT == 256 && RES == 1) return k1<2048, 256, 1>(k);
-  if (N == 4096 && NT == 256 && RES == 2) return k1<4096, 256, 2>(k);
-  if (N == 4096 && NT == 256 && RES == 1) return k1<4096, 256, 1>(k);
-  if (N == 8192 && NT == 256 && RES == 1) return k1<8192, 256, 1>(k);
-  return false;
+bool batch1d_info_d(int N, int C, BKernel *k) {
+  switch (N) {
+    case 1024: return k1c<1024>(C, k);
+    case 2048: return k1c<2048>(C, k);
+    case 4096: return k1c<4096>(C, k);
+    case 8192: return k1c<8192>(C, k);
+    case 16384: return k1c<16384>(C, k);
+    default: return false;
+  }
 }

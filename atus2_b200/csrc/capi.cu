@@ -697,6 +697,7 @@ void atus_destroy(atus_ctx *ctx) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   cudaFree(ctx->fs_tw);
   cudaFree(ctx->fs_tmp);
+  cudaFree(ctx->blk_F);
   cudaFree(ctx->scratch);
   cudaFree(ctx->sob_dev);
   if (ctx->sob_graph) cudaGraphExecDestroy(ctx->sob_graph);
@@ -1098,47 +1099,75 @@ int atus_strang_block_rabi(atus_ctx *ctx, int nk, int kind, const double *F, int
   return ATUS_OK;
 }
 
+// A 1D block with the field on chip: line1d.cuh (256..16384 points) or
+// block1d_kernel (2..128).  ATUS_E_UNSUPPORTED, nothing launched, where the
+// field does not fit.
+static int resident_block(atus_ctx *ctx, int nk, int kind, const double *F) {
+  const bool fp64 = ctx->prec == ATUS_PREC_FP64;
+  const bool line = ctx->n[0] >= 256, inlined = F && line && nk <= LINE_F_INLINE;
+  if (F && !inlined) {  // amplitudes in a buffer the context keeps, at most as long as its longest block
+    if (ctx->blk_F_n < nk) {
+      CK(cudaStreamSynchronize(ctx->stream));  // an earlier block may still read the old one
+      cudaFree(ctx->blk_F);
+      ctx->blk_F = nullptr;
+      ctx->blk_F_n = 0;
+      CK(cudaMalloc(&ctx->blk_F, sizeof(double) * nk));
+      ctx->blk_F_n = nk;
+    }
+    CK(cudaMemcpyAsync(ctx->blk_F, F, sizeof(double) * nk, cudaMemcpyHostToDevice, ctx->stream));
+  }
+  if (line) {
+    LineArgs a;
+    memset(&a, 0, sizeof(a));
+    for (int c = 0; c < ctx->ncomp; c++) {
+      a.in.psi[c] = ctx->psi[c];
+      a.in.kh[c] = ctx->kt[0][c][0];
+      a.in.kf[c] = ctx->kt[1][c][0];
+    }
+    a.in.s_f = scale_fak(ctx->dim, ctx->d);
+    a.in.s_b = scale_fak(ctx->dim, ctx->dk);
+    a.in.nl = nl_args(ctx, kind, 0.0, 1.0);
+    if (ctx->fs_tw) {  // the kinetic tables of a long axis are in four-step order
+      a.in.fs_lg1 = ilog2(ctx->fs_n1);
+      a.in.fs_lg2 = ilog2(ctx->fs_n2);
+    }
+    a.tw = ctx->tw;
+    a.nk = nk;
+    a.t0 = ctx->t;
+    if (inlined) {
+      memcpy(a.f, F, sizeof(double) * nk);
+      a.nf = nk;
+    } else if (F) {
+      a.F = ctx->blk_F;
+    }
+    if (ctx->ncomp == 1) return fp64 ? launch_line_d1(ctx, a) : launch_line_f1(ctx, a);
+    return fp64 ? launch_line_d2(ctx, a, kind == K_BRAGG) : launch_line_f2(ctx, a, kind == K_BRAGG);
+  }
+  Block1DArgs a;
+  memset(&a, 0, sizeof(a));
+  for (int c = 0; c < ctx->ncomp; c++) {
+    a.psi[c] = ctx->psi[c];
+    a.kh[c] = ctx->kt[0][c][0];
+    a.kf[c] = ctx->kt[1][c][0];
+  }
+  a.s_f = scale_fak(ctx->dim, ctx->d);
+  a.s_b = scale_fak(ctx->dim, ctx->dk);
+  a.tw = ctx->tw;
+  a.nl = nl_args(ctx, kind, 0.0, 1.0);
+  a.nk = nk;
+  a.t0 = ctx->t;
+  a.F = F ? ctx->blk_F : nullptr;
+  if (fp64) return ctx->ncomp == 1 ? launch_block1d_d1(ctx, a) : launch_block1d_d2(ctx, a);
+  return ctx->ncomp == 1 ? launch_block1d_f1(ctx, a) : launch_block1d_f2(ctx, a);
+}
+
 static int strang_block(atus_ctx *ctx, int nk, int kind, const double *F, const RabiReq *rr, double *sums,
                         bool *fused) {
   if (!ctx || nk < 1) return ATUS_E_ARG;
   RUN(check_kind(ctx, kind));
   const double dt = ctx->dt;
-  // shared memory of the resident 1D kernel (padded pencils, Pad<N>)
-  const int64_t n0 = ctx->n[0];
-  const int64_t np1d = ((n0 >= 16) ? (n0 + n0 / 16) : n0) | 1;
-  const bool on_cluster = ctx->use_cluster1d && n0 >= 2048 && n0 <= 8192;  // cluster1d.cuh
-  const bool fits1d = on_cluster || (int64_t)ctx->csize * tc_for(ctx->ncomp) * np1d <= 227 * 1024;
-  if (ctx->dim == 1 && ctx->ncomp <= 2 && kind != K_NUM_BRAGG && !ctx->fs_tw && fits1d) {
-    Block1DArgs a;
-    memset(&a, 0, sizeof(a));
-    for (int c = 0; c < MAXC; c++) {
-      a.psi[c] = ctx->psi[c];
-      a.kh[c] = (c < ctx->ncomp) ? ctx->kt[0][c][0] : nullptr;
-      a.kf[c] = (c < ctx->ncomp) ? ctx->kt[1][c][0] : nullptr;
-    }
-    a.s_f = scale_fak(ctx->dim, ctx->d);
-    a.s_b = scale_fak(ctx->dim, ctx->dk);
-    a.tw = ctx->tw;
-    a.nl = nl_args(ctx, kind, 0.0, 1.0);
-    a.nk = nk;
-    a.t0 = ctx->t;
-    double *dF = nullptr;
-    if (F) {
-      CK(cudaMalloc(&dF, sizeof(double) * nk));
-      CK(cudaMemcpyAsync(dF, F, sizeof(double) * nk, cudaMemcpyHostToDevice, ctx->stream));
-    }
-    a.F = dF;
-    const int tc = tc_for(ctx->ncomp);
-    int r;
-    if (tc > 2) return fail(ctx, ATUS_E_UNSUPPORTED, "1D blocks take at most two components");
-    if (ctx->prec == ATUS_PREC_FP64)
-      r = tc == 1 ? launch_block1d_d1(ctx, a) : launch_block1d_d2(ctx, a);
-    else
-      r = tc == 1 ? launch_block1d_f1(ctx, a) : launch_block1d_f2(ctx, a);
-    if (dF) {
-      cudaStreamSynchronize(ctx->stream);
-      cudaFree(dF);
-    }
+  if (ctx->dim == 1 && ctx->ncomp <= 2 && kind != K_NUM_BRAGG && ctx->n[0] <= 16384) {
+    const int r = resident_block(ctx, nk, kind, F);
     if (r == ATUS_OK) {
       // replay the header-time additions of the reference
       double t = ctx->t + 0.5 * dt;

@@ -37,7 +37,7 @@ struct atus_ctx {
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int64_t launches = 0;
   bool use_pass2 = true;        // register-staged passes for pencils of 32..256 points
-  bool use_cluster1d = true;    // 1D blocks of 2048..8192 points on a 16-CTA cluster
+  bool use_cluster1d = true;    // 1D blocks on a cluster of CTAs where that is faster
   bool use_tma = false;         // strided 256-point passes fed by TMA tile copies
   int *err_word = nullptr;      // error word of bounded waits (0: none)
   bool err_armed = false;       // a kernel that can set it ran since the last check
@@ -60,6 +60,8 @@ struct atus_ctx {
   int64_t fs_n1 = 0, fs_n2 = 0;
   double2 *fs_tw = nullptr;
   void *fs_tmp = nullptr;
+  double *blk_F = nullptr;              // pulse amplitudes of a 1D block (blk_F_n doubles)
+  int blk_F_n = 0;
   // asynchronous output snapshots
   void *snap = nullptr;                 // ncomp x N complex128 staging copy
   cudaStream_t copy_stream = nullptr;   // its device->host copies

@@ -5,7 +5,7 @@
 #include <cstring>
 
 #include "ctx.h"
-#include "cluster1d.cuh"
+#include "line1d.cuh"
 #include "pass2.cuh"
 #include "pass2_pair.cuh"
 #include "pass2_tma.cuh"
@@ -96,49 +96,72 @@ static inline int launch_block1d_t(atus_ctx *ctx, Block1DArgs &a) {
   return ATUS_OK;
 }
 
-// A 1D block on one cluster of CTAs (cluster1d.cuh).
-// ATUS_E_UNSUPPORTED (nothing launched) where the device cannot place such a
-// cluster (then the caller takes the one-CTA kernel or the per-step passes).
-template <typename R, int N, int TC>
-static inline int launch_cluster1d_t(atus_ctx *ctx, Block1DArgs &a) {
-  using Cfg = C1Cfg<R, N, TC>;
-  static int placeable = -1;  // clusters of this kernel the device can hold at once
-  if (placeable < 0) {
-    CK(cudaFuncSetAttribute(cluster1d_kernel<R, N, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
-    if (Cfg::C > 8) CK(cudaFuncSetAttribute(cluster1d_kernel<R, N, TC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+// A 1D block of 256..16384 points on one CTA or one cluster of C CTAs
+// (line1d.cuh).  ATUS_E_UNSUPPORTED, nothing launched, where the device cannot
+// place such a cluster.
+template <typename R, int N, int TC, int C, bool BRAGG>
+static inline int launch_line_t(atus_ctx *ctx, const LineArgs &a) {
+  using Cfg = LineCfg<R, N, TC, C>;
+  if constexpr (!Cfg::fits) {
+    return ATUS_E_UNSUPPORTED;
+  } else {
+    const auto kernel = line1d_kernel<R, N, TC, C, BRAGG>;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(Cfg::C);
+    cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(Cfg::NT);
     cfg.dynamicSmemBytes = Cfg::smem;
+    cfg.stream = ctx->stream;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = Cfg::C;
+    attr.val.clusterDim.x = C;
     attr.val.clusterDim.y = 1;
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    placeable = (cudaOccupancyMaxActiveClusters(&n, cluster1d_kernel<R, N, TC>, &cfg) == cudaSuccess) ? n : 0;
-    cudaGetLastError();  // a refused query leaves no sticky error
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    static int placeable = -1;  // clusters of this kernel the device can hold at once
+    if (placeable < 0) {
+      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
+      int n = 1;
+      if (C > 1 && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
+      placeable = n;
+      cudaGetLastError();  // a refused query leaves no sticky error
+    }
+    if (placeable < 1) return ATUS_E_UNSUPPORTED;
+    CK(cudaLaunchKernelEx(&cfg, kernel, a));
+    LAUNCHED(ctx);
+    return ATUS_OK;
   }
-  if (placeable < 1) return ATUS_E_UNSUPPORTED;
-  cluster1d_kernel<R, N, TC><<<Cfg::C, Cfg::NT, Cfg::smem, ctx->stream>>>(a);
-  LAUNCHED(ctx);
-  return ATUS_OK;
 }
 
+// CTAs a block runs on: line_ctas (line1d.cuh); ATUS_CLUSTER1D=0 asks for one.
+template <typename R, int N, int TC, bool BRAGG>
+static inline int launch_line_c(atus_ctx *ctx, const LineArgs &a) {
+  int r = ATUS_E_UNSUPPORTED;
+  constexpr int C = line_ctas<R, N, TC>;
+  if (ctx->use_cluster1d) r = launch_line_t<R, N, TC, C, BRAGG>(ctx, a);
+  if constexpr (C > 1) {
+    if (r == ATUS_E_UNSUPPORTED) r = launch_line_t<R, N, TC, 1, BRAGG>(ctx, a);
+  }
+  return r;
+}
+
+template <typename R, int TC, bool BRAGG>
+static inline int launch_line_n(atus_ctx *ctx, const LineArgs &a) {
+  switch (ctx->n[0]) {
+    case 256: return launch_line_c<R, 256, TC, BRAGG>(ctx, a);
+    case 512: return launch_line_c<R, 512, TC, BRAGG>(ctx, a);
+    case 1024: return launch_line_c<R, 1024, TC, BRAGG>(ctx, a);
+    case 2048: return launch_line_c<R, 2048, TC, BRAGG>(ctx, a);
+    case 4096: return launch_line_c<R, 4096, TC, BRAGG>(ctx, a);
+    case 8192: return launch_line_c<R, 8192, TC, BRAGG>(ctx, a);
+    case 16384: return launch_line_c<R, 16384, TC, BRAGG>(ctx, a);
+    default: return ATUS_E_UNSUPPORTED;
+  }
+}
+
+// 2..128 points: block1d.
 template <typename R, int TC>
 static inline int launch_block1d_n(atus_ctx *ctx, Block1DArgs &a) {
-  if (ctx->use_cluster1d) {
-    int r = ATUS_E_UNSUPPORTED;
-    switch (ctx->n[0]) {
-      case 2048: r = launch_cluster1d_t<R, 2048, TC>(ctx, a); break;
-      case 4096: r = launch_cluster1d_t<R, 4096, TC>(ctx, a); break;
-      case 8192: r = launch_cluster1d_t<R, 8192, TC>(ctx, a); break;
-      default: break;
-    }
-    if (r != ATUS_E_UNSUPPORTED) return r;
-  }
   switch (ctx->n[0]) {
     case 2: return launch_block1d_t<R, 2, TC>(ctx, a);
     case 4: return launch_block1d_t<R, 4, TC>(ctx, a);
@@ -147,16 +170,9 @@ static inline int launch_block1d_n(atus_ctx *ctx, Block1DArgs &a) {
     case 32: return launch_block1d_t<R, 32, TC>(ctx, a);
     case 64: return launch_block1d_t<R, 64, TC>(ctx, a);
     case 128: return launch_block1d_t<R, 128, TC>(ctx, a);
-    case 256: return launch_block1d_t<R, 256, TC>(ctx, a);
-    case 512: return launch_block1d_t<R, 512, TC>(ctx, a);
-    case 1024: return launch_block1d_t<R, 1024, TC>(ctx, a);
-    case 2048: return launch_block1d_t<R, 2048, TC>(ctx, a);
-    case 4096: return launch_block1d_t<R, 4096, TC>(ctx, a);
-    case 8192: return launch_block1d_t<R, 8192, TC>(ctx, a);
-    default: return fail(ctx, ATUS_E_UNSUPPORTED, "axis length must be a power of two in [2, 8192]");
+    default: return ATUS_E_UNSUPPORTED;
   }
 }
-
 
 // ------------------------------------------------------------ register-staged passes
 // Launch of pass2_kernel (pencils of 32..256 points); ATUS_E_UNSUPPORTED,

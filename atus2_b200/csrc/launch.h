@@ -1,6 +1,7 @@
 // launch.h -- exported launchers, one per precision and tile component count.
 #pragma once
 #include "ctx.h"
+#include "line1d.cuh"
 #include "pass2.cuh"
 
 int launch_pass_d1(atus_ctx *ctx, PassArgs &a, int axis);
@@ -9,6 +10,13 @@ int launch_pass_d4(atus_ctx *ctx, PassArgs &a, int axis);
 int launch_pass_f1(atus_ctx *ctx, PassArgs &a, int axis);
 int launch_pass_f2(atus_ctx *ctx, PassArgs &a, int axis);
 int launch_pass_f4(atus_ctx *ctx, PassArgs &a, int axis);
+// A 1D block with the field on chip.  _line: 256..16384 points (bragg: two
+// components, kind K_BRAGG; else pure phases); _block1d: 2..128 points.
+// ATUS_E_UNSUPPORTED, nothing launched, where the field does not fit.
+int launch_line_d1(atus_ctx *ctx, const LineArgs &a);
+int launch_line_d2(atus_ctx *ctx, const LineArgs &a, bool bragg);
+int launch_line_f1(atus_ctx *ctx, const LineArgs &a);
+int launch_line_f2(atus_ctx *ctx, const LineArgs &a, bool bragg);
 int launch_block1d_d1(atus_ctx *ctx, Block1DArgs &a);
 int launch_block1d_d2(atus_ctx *ctx, Block1DArgs &a);
 int launch_block1d_f1(atus_ctx *ctx, Block1DArgs &a);
