@@ -162,6 +162,10 @@ static int dispatch_pass(atus_ctx *ctx, PassArgs &a, int axis, int tc) {
       r = dbl ? launch_pass2_d_t(ctx, a, axis, mode, strided) : launch_pass2_f_t(ctx, a, axis, mode, strided);
     } else if ((a.op == OP_KIN || a.op == OP_FILT) && a.t1 == T_FWD && a.t2 == T_INV && strided) {
       r = dbl ? launch_pass2_d_k(ctx, a, axis) : launch_pass2_f_k(ctx, a, axis);
+    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 3) {
+      r = dbl ? launch_pass2_d_nl3(ctx, a, axis) : launch_pass2_f_nl3(ctx, a, axis);
+    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 4) {
+      r = dbl ? launch_pass2_d_nl4(ctx, a, axis) : launch_pass2_f_nl4(ctx, a, axis);
     } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && tc <= 2) {
       r = dbl ? launch_pass2_d_nl(ctx, a, axis, tc) : launch_pass2_f_nl(ctx, a, axis, tc);
     }

@@ -235,6 +235,45 @@ template <> __device__ __forceinline__ double2 expi<float>(double phi) {
   return expi_far_mixed(phi);
 }
 
+// ------------------------------------------------------------ couplings
+// What a step's coupling takes from x alone (and the step's time): the same
+// for every point of a pencil that does not run along x, so the passes
+// evaluate it once a pencil instead of once a point.
+//   K_DBRAGG    Omega_+, Omega_-, cos, sin of -dk x / 2
+//   K_BRAGG_DS  per species Omega_s, cos, sin of -(dk_s x + phase_s) / 2
+//   K_RAMAN     cos, sin of k x
+//   K_NUM_BRAGG per upper state cos, sin of (-domh + rate_i t) t + k_i x - phase / 2
+constexpr int NCPL = 6;
+__device__ __forceinline__ void coupling_x(const NLArgs &a, double x0, double *cp) {
+  const double t1 = a.t1;
+  if (a.kind == K_DBRAGG) {
+    const double F = a.F < 0 ? 0.0 : a.F;
+    double dw = a.L.laser_domh0 + a.L.chirp_rate0 * t1;
+    cp[0] = F * a.L.Amp0 * cos(a.L.laser_k0 * x0 - dw * t1 - a.L.phase0 / 2);
+    dw = a.L.laser_domh0 - a.L.chirp_rate0 * t1;
+    cp[1] = F * a.L.Amp0 * cos(-a.L.laser_k0 * x0 - dw * t1 - a.L.phase0 / 2);
+    sincos(-0.5 * a.L.laser_dk0 * x0, &cp[3], &cp[2]);
+  } else if (a.kind == K_BRAGG_DS) {
+    #pragma unroll
+    for (int s = 0; s < 2; s++) {
+      const LaserD &L = s ? a.L2 : a.L;
+      cp[3 * s] = (s ? a.F2 : a.F) * L.Amp0 *
+                  cos(L.laser_k0 * x0 - (L.laser_domh0 + L.chirp_rate0 * t1) * t1 + L.phase0 / 2);
+      sincos(-0.5 * (L.laser_dk0 * x0 + L.phase0), &cp[3 * s + 2], &cp[3 * s + 1]);
+    }
+  } else if (a.kind == K_RAMAN) {
+    sincos(a.L.laser_k0 * x0, &cp[1], &cp[0]);
+  } else if (a.kind == K_NUM_BRAGG) {
+    const double th = a.th;
+    #pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const double k = i == 0 ? a.L.laser_k0 : -a.L.laser_k0;
+      const double rate = i == 0 ? a.L.chirp_rate0 : -a.L.chirp_rate0;
+      sincos((-a.L.laser_domh0 + rate * th) * th + k * x0 - 0.5 * a.L.phase0, &cp[2 * i + 1], &cp[2 * i]);
+    }
+  }
+}
+
 // ------------------------------------------------------------ three-level Bragg step
 // Bragg_double::Do_Double_Bragg_ad (source/interferometry/src/double_bragg.cpp:
 // 123-256) at grid index l: state 1 (component 0) couples to states 2 and 3
@@ -243,8 +282,9 @@ template <> __device__ __forceinline__ double2 expi<float>(double phi) {
 // V includes beta . x over all axes.  The reference's operation order,
 // including its O32 update that reads the already-updated O23 imaginary part
 // (double_bragg.cpp:233).  FP64 arithmetic for both field precisions.
+// cp: Omega_+, Omega_-, cos and sin of -dk x / 2 (coupling_x).
 template <typename R>
-__device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0) {
+__device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, const double *cp) {
   double bx = a.L.beta0 * x0;
   if (a.lg1 > 0) {
     const int iy = (int)((l >> a.lg2) & ((1 << a.lg1) - 1));
@@ -261,12 +301,7 @@ __device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_
   const double *gs = a.gs;  // padded rows: g_ij at i * MAXC + j
   const double V11 = gs[0] * tmp1 + gs[1] * tmp2 + gs[2] * tmp3 + bx;
   const double V22 = gs[MAXC] * tmp1 + gs[MAXC + 1] * tmp2 + gs[MAXC + 2] * tmp3 - a.L.DeltaL[1] + bx;
-  const double t1 = a.t1, dt = a.dt;
-  const double F = a.F < 0 ? 0.0 : a.F;
-  double dw = a.L.laser_domh0 + a.L.chirp_rate0 * t1;
-  const double Op = F * a.L.Amp0 * cos(a.L.laser_k0 * x0 - dw * t1 - a.L.phase0 / 2);
-  dw = a.L.laser_domh0 - a.L.chirp_rate0 * t1;
-  const double Om = F * a.L.Amp0 * cos(-a.L.laser_k0 * x0 - dw * t1 - a.L.phase0 / 2);
+  const double dt = a.dt, Op = cp[0], Om = cp[1];
   double re1, im1;
   if (Om == 0.0 && Op == 0.0) {
     sincos_step(-dt * V11, &im1, &re1);
@@ -276,8 +311,7 @@ __device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_
     v[2] = from_d<R>(cmul(p3, make_double2(re1, im1)));
     return;
   }
-  double e0, e1;
-  sincos(-0.5 * a.L.laser_dk0 * x0, &e1, &e0);
+  const double e0 = cp[2], e1 = cp[3];
   const double OO = Op * Op + Om * Om;
   tmp1 = sqrt((V11 - V22) * (V11 - V22) + 4.0 * OO);
   const double E1 = 0.5 * (V11 + V22 + tmp1);
@@ -453,8 +487,9 @@ __device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, do
 // with Omega_s = F_s Amp_s cos(k_s x - (domh_s + rate_s t1) t1 + phase_s/2),
 // eta_s = e^{-i (dk_s x + phase_s)/2}.  F_s is 0 outside the species' pulse
 // window (bragg_ds.cpp:117-127), set on the host.
+// cp: Omega_s, cos and sin of -(dk_s x + phase_s) / 2 per species (coupling_x).
 template <typename R>
-__device__ __forceinline__ void bragg_ds_point(const NLArgs &a, cplx<R> *v, double x0) {
+__device__ __forceinline__ void bragg_ds_point(const NLArgs &a, cplx<R> *v, double x0, const double *cp) {
   double rho[MAXC];
   #pragma unroll
   for (int j = 0; j < MAXC; j++) rho[j] = (double)v[j].x * (double)v[j].x + (double)v[j].y * (double)v[j].y;
@@ -466,16 +501,10 @@ __device__ __forceinline__ void bragg_ds_point(const NLArgs &a, cplx<R> *v, doub
     for (int j = 1; j < MAXC; j++) p += a.gs[i * MAXC + j] * rho[j];
     phi[i] = p + (((i < 2) ? a.L.beta0 : a.L2.beta0) * x0 - a.L.DeltaL[i]);
   }
-  const double t1 = a.t1, dt = a.dt;
   #pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const LaserD &L = s ? a.L2 : a.L;
-    const double Omega = (s ? a.F2 : a.F) * L.Amp0 *
-                         cos(L.laser_k0 * x0 - (L.laser_domh0 + L.chirp_rate0 * t1) * t1 + L.phase0 / 2);
-    double es, ec;
-    sincos(-0.5 * (L.laser_dk0 * x0 + L.phase0), &es, &ec);
-    bragg_pair<R>(a.stable, dt, phi[2 * s], phi[2 * s + 1], Omega, ec, es, v[2 * s], v[2 * s + 1]);
-  }
+  for (int s = 0; s < 2; s++)
+    bragg_pair<R>(a.stable, a.dt, phi[2 * s], phi[2 * s + 1], cp[3 * s], cp[3 * s + 1], cp[3 * s + 2], v[2 * s],
+                  v[2 * s + 1]);
 }
 
 // ------------------------------------------------------------ numerical n-state steps
@@ -578,7 +607,7 @@ __device__ __forceinline__ double beta_dot_x(const NLArgs &a, int64_t l, double 
 // Not inlined: the pass kernels that carry it keep their register budget for
 // the common steps.
 template <typename R, int TC>
-__device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0) {
+__device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, const double *cp) {
   constexpr int NC = TC < 3 ? TC : 3;
   const int n = a.ncomp;
   const double bx = beta_dot_x(a, l, x0);
@@ -606,8 +635,7 @@ __device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, d
   if (a.kind == K_RAMAN) {
     if constexpr (NC >= 3) {
       A[2][2].x += a.L.laser_domh0;
-      double sn, cs;
-      sincos(a.L.laser_k0 * x0, &sn, &cs);
+      const double cs = cp[0], sn = cp[1];
       const double h0 = a.L.Amp0 / 2, h1 = a.L.Amp1 / 2;
       A[0][2] = make_double2(h0 * cs, h0 * sn);
       A[2][0] = make_double2(h0 * cs, -h0 * sn);
@@ -615,14 +643,10 @@ __device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, d
       A[2][1] = make_double2(h1 * cs, h1 * sn);
     }
   } else {
-    const double t1 = a.th;
     #pragma unroll
     for (int i = 0; i + 1 < NC; i++) {
       if (i + 1 >= n) break;
-      const double k = i == 0 ? a.L.laser_k0 : -a.L.laser_k0;
-      const double rate = i == 0 ? a.L.chirp_rate0 : -a.L.chirp_rate0;
-      double sn, cs;
-      sincos((-a.L.laser_domh0 + rate * t1) * t1 + k * x0 - 0.5 * a.L.phase0, &sn, &cs);
+      const double cs = cp[2 * i], sn = cp[2 * i + 1];
       const double er = a.L.Amp0 * cs / 2 + a.L.Amp1 * cs / 2, ei = a.L.Amp0 * sn / 2 - a.L.Amp1 * sn / 2;
       A[i + 1][0] = make_double2(er, ei);
       A[0][i + 1] = make_double2(er, -ei);
@@ -669,6 +693,8 @@ __device__ __noinline__ void nl_pair16_any(const NLArgs &a, cplx<R> *v, int c, i
   using C = cplx<R>;
   if (a.kind == K_BRAGG || a.kind == K_NUM_BRAGG) {
     const double bx = a.L.beta0 * x0, bd = bx - a.L.DeltaL[1];
+    double cp[NCPL];
+    if (a.kind == K_NUM_BRAGG) coupling_x(a, x0, cp);
     #pragma unroll 1
     for (int m = 0; m < 8; m++) {
       C own = v[m], oth = shfl_xor_c(v[m + 8], mask);
@@ -680,7 +706,7 @@ __device__ __noinline__ void nl_pair16_any(const NLArgs &a, cplx<R> *v, int c, i
         bragg_pair<R>(a.stable, a.dt, Vo, Vt, om, ec, c ? -es : es, own, oth, c != 0);
       } else {
         C w[2] = {c ? oth : own, c ? own : oth};
-        num_point<R, 2>(a, w, l0 + (int64_t)dl * (m ^ (8 * c)), x0);
+        num_point<R, 2>(a, w, l0 + (int64_t)dl * (m ^ (8 * c)), x0, cp);
         own = c ? w[1] : w[0];
         oth = c ? w[0] : w[1];
       }
@@ -804,17 +830,25 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
 // the caller has loaded the potential at l into vpre (0 without a potential).
 template <typename R, int TC = MAXC, bool PREV = false>
 __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, double Omega,
-                                         double eta_c, double eta_s, double vpre = 0.0) {
+                                         double eta_c, double eta_s, double vpre = 0.0, const double *cp = nullptr) {
   static_assert(!PREV || TC == 1, "a pre-loaded potential serves one component");
+  // couplings of the pencil, where the caller has not evaluated them
+  double own[NCPL];
+  if constexpr (TC >= 2) {
+    if (!cp && a.kind != K_BRAGG) {
+      coupling_x(a, x0, own);
+      cp = own;
+    }
+  }
   if constexpr (TC >= 3) {
     if (a.kind == K_DBRAGG) {
-      dbragg_point<R>(a, v, l, x0);
+      dbragg_point<R>(a, v, l, x0, cp);
       return;
     }
   }
   if constexpr (TC >= 4) {
     if (a.kind == K_BRAGG_DS) {
-      bragg_ds_point<R>(a, v, x0);
+      bragg_ds_point<R>(a, v, x0, cp);
       return;
     }
   }
@@ -826,7 +860,7 @@ __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l,
       cplx<R> w[TC];
       #pragma unroll
       for (int c = 0; c < TC; c++) w[c] = v[c];
-      num_point<R, TC>(a, w, l, x0);
+      num_point<R, TC>(a, w, l, x0, cp);
       #pragma unroll
       for (int c = 0; c < TC; c++) v[c] = w[c];
       return;

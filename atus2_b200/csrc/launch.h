@@ -24,7 +24,8 @@ int launch_block1d_f2(atus_ctx *ctx, Block1DArgs &a);
 // Register-staged passes (pencils of 32..256 points).  _t: one transform
 // (mode M2_FWD / M2_INV, strided or contiguous axis); _k: FFT, kinetic or
 // Sobolev filter, IFFT along a strided axis; _nl: IFFT, potential step, FFT
-// along the contiguous axis with tc components per tile (1 or 2).  All return
+// along the contiguous axis with tc components per tile (1 to 4; 3 and 4 in _nl3
+// and _nl4).  All return
 // ATUS_E_UNSUPPORTED, with the fields untouched, when they do not apply.
 int launch_pass2_d_t(atus_ctx *ctx, PassArgs &a, int axis, int mode, bool strided);
 int launch_pass2_f_t(atus_ctx *ctx, PassArgs &a, int axis, int mode, bool strided);
@@ -42,3 +43,7 @@ int launch_pass2_d_sob(atus_ctx *ctx, PassArgs &a, int axis, int mode);
 // 128..2048 points; tc: components of M2_FS_NL (1 or 2)
 int launch_fs_d(atus_ctx *ctx, PassArgs &a, int mode, int tc);
 int launch_fs_f(atus_ctx *ctx, PassArgs &a, int mode, int tc);
+int launch_pass2_d_nl3(atus_ctx *ctx, PassArgs &a, int axis);
+int launch_pass2_d_nl4(atus_ctx *ctx, PassArgs &a, int axis);
+int launch_pass2_f_nl3(atus_ctx *ctx, PassArgs &a, int axis);
+int launch_pass2_f_nl4(atus_ctx *ctx, PassArgs &a, int axis);

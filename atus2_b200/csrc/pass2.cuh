@@ -34,8 +34,9 @@ template <> struct Tile2<float> { static constexpr int E = 4096, NT = 256, MINB 
 // Sobolev iteration, the potential passes and the four-step passes hold
 // potential values or twiddles beside a thread's 16 points (256^3, one
 // component, z pass: 5 CTAs with spills 207 us, 4 without 178 us).
-template <typename R, int MODE>
+template <typename R, int MODE, int TC = 1>
 constexpr int p2_minb =
+    TC >= 3 ? (TC == 3 ? 3 : sizeof(R) == 8 ? 4 : 2) :
     (((MODE >= M2_FWD_SOB && MODE != M2_FILT) || MODE == M2_NL) && sizeof(R) == 8) ? 4 : Tile2<R>::MINB;
 
 // Passes whose two components meet inside a warp (the batched passes; a
@@ -46,14 +47,15 @@ template <typename R, int N, int TC>
 struct P2Cfg {
   static constexpr int R2 = N / 16;        // stage-2 radix
   static constexpr int T2 = 16 / R2;       // stage-2 butterflies per thread
-  static constexpr int E = Tile2<R>::E;
-  static constexpr int NT = Tile2<R>::NT;
-  static constexpr int B = E / (N * TC);   // pencils per tile
+  // threads: a power of two of pencil-components, or, for three components
+  // (no quarter of the threads idle), three times one
+  static constexpr int NT = TC == 3 ? 192 : Tile2<R>::NT;
+  static constexpr int B = NT / (R2 * TC); // pencils per tile
   static constexpr int NPC = B * TC;       // pencil-components per tile
   static constexpr int PB = 17 * R2 + 1;   // exchange pitch: R2 rows of 16 + 1 pad, odd
   static constexpr int TP = R2 + 1;        // twiddle row pitch (odd)
   static constexpr int TWP = 16 * TP;      // twiddle table: row k holds W_N^{r k}, r < R2
-  static constexpr size_t smem_ex = sizeof(cplx<R>) * NPC * PB;
+  static constexpr size_t smem_ex = (sizeof(cplx<R>) * NPC * PB + 15) / 16 * 16;  // 16-byte twiddles follow
   static constexpr size_t smem_tw = sizeof(typename TwTab<R>::type) * TWP;
   static constexpr size_t smem = smem_ex + smem_tw;
   // k-space passes also keep the along-axis kinetic factors of up to two
@@ -256,9 +258,17 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
   const int64_t step = (int64_t)R2 * a.sa;     // distance of points j + R2 m and j + R2 (m+1)
   const C *src = live ? f + lb + (int64_t)j * a.sa : nullptr;
 
-  if constexpr (MODE == M2_NL && TC > 1 && !PAIR) {
+  if constexpr (MODE == M2_NL && TC > 2) {
     // coupling of each pencil (x is constant along it); read after the
     // barriers of the first transform
+    for (int p = tid; p < B; p += NT)
+      if (p < g.nb) {
+        int ix, iy, iz;
+        idx3(a.g, g.base0 + p * g.pstride, ix, iy, iz);
+        coupling_x(a.nl, (double)(ix - a.nl.shift0) * a.nl.dx0, s_om + NCPL * p);
+      }
+  }
+  if constexpr (MODE == M2_NL && TC == 2 && !PAIR) {
     if (a.nl.kind == K_BRAGG && a.axis != 0)
     for (int p = tid; p < B; p += NT) {
       double om = 0, ec = 1, es = 0;
@@ -488,11 +498,9 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         my[ex_at(i >> 4, i & 15)] = v[m];
       }
       __syncthreads();
-      constexpr int PPT = 16 / TC;  // points per thread
-      const bool bragg = (a.nl.kind == K_BRAGG);
+      const bool bragg = TC == 2 && (a.nl.kind == K_BRAGG);
       #pragma unroll 1  // measured fastest: unrolling 2/4/8 points was 4-50 % slower
-      for (int u_ = 0; u_ < PPT; u_++) {
-        const int p = tid + NT * u_;
+      for (int p = tid; p < B * N; p += NT) {
         int pb, i;
         if (STRIDED) { pb = p % B; i = p / B; } else { i = p % N; pb = p / N; }
         if (pb < g.nb) {
@@ -505,10 +513,11 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
             if (a.axis == 0) bragg_coupling(a.nl, x0, om, ec, es);
             else { om = s_om[pb]; ec = s_ec[pb]; es = s_es[pb]; }
           }
+          const double *const cp = (MODE == M2_NL && TC > 2) ? s_om + NCPL * pb : nullptr;
           C u[MAXC];
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) u[cc] = ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)];
-          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es);
+          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, 0.0, cp);
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)] = u[cc];
         }
@@ -552,10 +561,10 @@ __device__ __forceinline__ void p2_prefetch_l2(const PassArgs &a, const TileGeo 
 }
 
 template <typename R, int N, int TC, int MODE, bool STRIDED>
-__global__ void __launch_bounds__(Tile2<R>::NT, p2_minb<R, MODE>) pass2_kernel(PassArgs a) {
+__global__ void __launch_bounds__(P2Cfg<R, N, TC>::NT, p2_minb<R, MODE, TC>) pass2_kernel(PassArgs a) {
   using Cfg = P2Cfg<R, N, TC>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double s_om[Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];
+  __shared__ double s_om[TC > 2 ? NCPL * Cfg::B : Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];  // couplings of the pencils
   const bool kt_shared = p2_setup<R, N, TC, MODE>(a, smem_raw);
   __syncthreads();  // twiddle rows and kinetic factors visible to every warp
   const int64_t W = a.per_comp ? a.ntiles * a.ncomp_grid : a.ntiles;

@@ -40,7 +40,8 @@ struct P3Cfg {
   static constexpr int BCAP = (sizeof(R) == 8 ? 512 : 1024) / (M * TC);  // pencils that fit the register file
   static constexpr int BMIN = STRIDED ? (BCAP < 8 ? BCAP : 8) : 1;
   static constexpr int NT_MIN = M * TC * BMIN;
-  static constexpr int NT = (NT_MIN > Tile3<R>::NT) ? NT_MIN : Tile3<R>::NT;
+  static constexpr int NT_LOW = (TC == 3) ? 192 : Tile3<R>::NT;  // a multiple of M TC
+  static constexpr int NT = (NT_MIN > NT_LOW) ? NT_MIN : NT_LOW;
   static constexpr int NPC = NT / M; // pencil-components per tile
   static constexpr int B = NPC / TC; // pencils per tile
   // Pencil pitch of the exchange rows.  A bank group (the threads whose
@@ -51,7 +52,8 @@ struct P3Cfg {
   static constexpr int G = 128 / (int)sizeof(cplx<R>);
   // Contiguous tiles of two components: G / 2 consecutive t of both.
   static constexpr int PB = 17 * M + ((STRIDED && B < G) ? G / B : (!STRIDED && TC == 2) ? G / 2 : 1);
-  static constexpr size_t smem_ex = sizeof(cplx<R>) * NPC * PB;
+  // the twiddles (16 bytes each) follow: an odd number of complex64 rows ends between
+  static constexpr size_t smem_ex = (sizeof(cplx<R>) * NPC * PB + 15) / 16 * 16;
   // W_N^{t q} (row q, column t) and W_M^{j2 q2} (row q2, column j2)
   static constexpr int TWN_N = 16 * M, TWN_M = 16 * R3;
   static constexpr size_t smem = smem_ex + sizeof(typename TwTab<R>::type) * (TWN_N + TWN_M);
@@ -137,7 +139,8 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
   using Cfg = P3Cfg<R, N, TC, STRIDED>;
   constexpr int M = Cfg::M, B = Cfg::B, NT = Cfg::NT, PB = Cfg::PB;
   static_assert(N >= 512 && N <= 2048, "three-stage pencils only");
-  static_assert(Cfg::NPC * M == NT, "one thread per stage-1 butterfly");
+  static_assert(Cfg::NPC * M == NT && Cfg::B * TC == Cfg::NPC, "one thread per stage-1 butterfly");
+  static_assert(Cfg::smem_ex % 16 == 0, "twiddles are read in 16 bytes");
   C *const ex = reinterpret_cast<C *>(smem_raw);
   const TW *const twN = reinterpret_cast<const TW *>(smem_raw + Cfg::smem_ex);
   const TW *const twM = twN + Cfg::TWN_N;
@@ -157,7 +160,15 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
   const int64_t step = (int64_t)M * a.sa;      // distance of points t + M r and t + M (r+1)
   const C *src = live ? f + lb + (int64_t)t * a.sa : nullptr;
 
-  if constexpr (MODE == M2_NL && TC > 1) {
+  if constexpr (MODE == M2_NL && TC > 2) {
+    for (int p = tid; p < B; p += NT)
+      if (p < g.nb) {
+        int ix, iy, iz;
+        idx3(a.g, g.base0 + p * g.pstride, ix, iy, iz);
+        coupling_x(a.nl, (double)(ix - a.nl.shift0) * a.nl.dx0, s_om + NCPL * p);
+      }
+  }
+  if constexpr (MODE == M2_NL && TC == 2) {
     if (a.nl.kind == K_BRAGG && a.axis != 0)
       for (int p = tid; p < B; p += NT) {
         double om = 0, ec = 1, es = 0;
@@ -306,11 +317,9 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
         my[ex_at(i >> 4, i & 15)] = v[m];
       }
       __syncthreads();
-      constexpr int PPT = 16 / TC;  // points per thread
-      const bool bragg = (a.nl.kind == K_BRAGG);
+      const bool bragg = TC == 2 && (a.nl.kind == K_BRAGG);
       #pragma unroll 1
-      for (int u_ = 0; u_ < PPT; u_++) {
-        const int p = tid + NT * u_;
+      for (int p = tid; p < B * N; p += NT) {
         int pb, i;
         if (STRIDED) { pb = p % B; i = p / B; } else { i = p % N; pb = p / N; }
         if (pb < g.nb) {
@@ -323,10 +332,11 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
             if (a.axis == 0) bragg_coupling(a.nl, x0, om, ec, es);
             else { om = s_om[pb]; ec = s_ec[pb]; es = s_es[pb]; }
           }
+          const double *const cp = (MODE == M2_NL && TC > 2) ? s_om + NCPL * pb : nullptr;
           C u[MAXC];
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) u[cc] = ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)];
-          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es);
+          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, 0.0, cp);
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)] = u[cc];
         }
@@ -371,7 +381,7 @@ __global__ void __launch_bounds__(P3Cfg<R, N, TC, STRIDED>::NT, P3Cfg<R, N, TC, 
     pass3_kernel(PassArgs a) {
   using Cfg = P3Cfg<R, N, TC, STRIDED>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double s_om[Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];
+  __shared__ double s_om[TC > 2 ? NCPL * Cfg::B : Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];  // couplings of the pencils
   p3_setup<R, N, TC, STRIDED>(a, smem_raw);
   __syncthreads();  // twiddle rows visible to every warp
   const int64_t W = a.per_comp ? a.ntiles * a.ncomp_grid : a.ntiles;
