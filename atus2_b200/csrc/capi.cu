@@ -470,7 +470,7 @@ static int launch_reduce(atus_ctx *ctx, RedArgs &a, double *dst) {
   const int64_t want = (ctx->npts + per - 1) / per;
   const unsigned grid = (unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS);
   const bool fp64 = ctx->prec == ATUS_PREC_FP64;
-#define ATUS_RED(R, M) reduce_kernel<R, M><<<grid, RED_THREADS, 0, ctx->stream>>>(a, ctx->red_partial, ctx->red_count, dst)
+#define ATUS_RED(R, M) CK(launch_pdl(ctx, reduce_kernel<R, M>, 148, RED_BLOCKS / 148, grid, RED_THREADS, 0, a, ctx->red_partial, ctx->red_count, dst))
   switch (a.mode) {
     case RED_NORM: if (fp64) ATUS_RED(double, RED_NORM); else ATUS_RED(float, RED_NORM); break;
     case RED_POS: if (fp64) ATUS_RED(double, RED_POS); else ATUS_RED(float, RED_POS); break;
@@ -1625,9 +1625,9 @@ static int sob_iterate_dev(atus_ctx *ctx) {
   for (int i = 0; i < n; i++) {
     const int64_t per = (int64_t)RED_THREADS * RED_AHEAD;
     const int64_t want = (ctx->npts + per - 1) / per;
-    sob_step_kernel<<<(unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS), RED_THREADS, 0, ctx->stream>>>(
-        (double2 *)ctx->psi[i], (const double2 *)ctx->sob_grad[i], (const double2 *)ctx->sob_psi[i], ctx->stepsize, d,
-        i, n, i == n - 1, ctx->ar, ctx->npts, ctx->red_partial, ctx->red_count);
+    CK(launch_pdl(ctx, sob_step_kernel, 148, RED_BLOCKS / 148, (unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS), RED_THREADS, 0,
+                  (double2 *)ctx->psi[i], (const double2 *)ctx->sob_grad[i], (const double2 *)ctx->sob_psi[i],
+                  ctx->stepsize, d, i, n, (int)(i == n - 1), ctx->ar, ctx->npts, ctx->red_partial, ctx->red_count));
     LAUNCHED(ctx);
   }
   return ATUS_OK;

@@ -88,6 +88,17 @@ struct NLArgs {
   double th;  // header time at the potential step (the numerical "bragg" step's t1)
 };
 
+// Programmatic dependent launch: a pass may be launched before the kernel it
+// depends on has ended, prepares its tables, and waits here until that
+// kernel's writes are visible; then it lets its own successor be launched.
+// (Without the launch attribute both are no-ops.)  Nothing that a kernel
+// writes may be touched before.  Worth it where passes are short: 64^3 x 2
+// passes of 6-15 us, 10 steps: PDL_OLD -> PDL_NEW us.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 struct Geo {
   int lg[3];                // log2 of n0, n1, n2 (unused axes: 0)
   int64_t npts;
@@ -1027,6 +1038,7 @@ __global__ void __launch_bounds__(Tile<R>::NT, Tile<R>::MINB) pass_kernel(PassAr
     }
   };
 
+  pdl_wait();
   int64_t w = blockIdx.x;
   int buf = 0;
   if (Cfg::NBUF == 2) {
@@ -1504,6 +1516,7 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs a, double *
   double q[RED_MAXQ];
   #pragma unroll
   for (int i = 0; i < RED_MAXQ; i++) q[i] = 0;
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * RED_THREADS;
   for (int64_t l0 = blockIdx.x * (int64_t)RED_THREADS + threadIdx.x; l0 < a.g.npts; l0 += RED_AHEAD * stride) {
     RedIn<R, MODE> in[RED_AHEAD];

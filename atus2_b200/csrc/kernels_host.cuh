@@ -76,6 +76,7 @@ struct SobDev {
 __global__ void __launch_bounds__(RED_THREADS) sob_step_kernel(double2 *psi, const double2 *sw, const double2 *ps,
                                                                double step, SobDev *d, int comp, int ncomp, int finish,
                                                                double ar, int64_t n, double *partial, unsigned *count) {
+  pdl_wait();
   const bool active = !d->done && d->iters < d->max_iter;
   if (!active) return;
   bool renorm = false;

@@ -57,7 +57,7 @@ static inline int launch_pass_t(atus_ctx *ctx, PassArgs &a, int axis) {
   const int64_t work = a.per_comp ? ntiles * ctx->ncomp : ntiles;
   const int64_t slots = (int64_t)nsm * resident;
   const unsigned grid = (unsigned)(work < slots ? work : slots);
-  pass_kernel<R, N, TC><<<grid, Cfg::NT, smem, ctx->stream>>>(a);
+  CK(launch_pdl(ctx, pass_kernel<R, N, TC>, nsm, resident, grid, Cfg::NT, smem, a));
   LAUNCHED(ctx);
   return ATUS_OK;
 }
@@ -257,7 +257,7 @@ static inline int launch_pass2_tma_t(atus_ctx *ctx, PassArgs &a, int axis) {
   const int64_t work = ntiles * ctx->ncomp;
   const int64_t slots = (int64_t)nsm * resident;
   const unsigned grid = (unsigned)(work < slots ? work : slots);
-  pass2_tma_kernel<R, N, MODE><<<grid, T::Cfg::NT, smem, ctx->stream>>>(a, maps);
+  CK(launch_pdl(ctx, pass2_tma_kernel<R, N, MODE>, nsm, resident, grid, T::Cfg::NT, smem, a, maps));
   LAUNCHED(ctx);
   ctx->err_armed = true;
   return ATUS_OK;
@@ -286,7 +286,8 @@ static inline int launch_pair_t(atus_ctx *ctx, PassArgs &a, int axis) {
   a.tw = (sizeof(R) == 8) ? ctx->tw64 : ctx->tw;
   const int64_t ctas = (a.npencils + Cfg::PW * Cfg::WPC - 1) / (Cfg::PW * Cfg::WPC);
   const int64_t slots = (int64_t)nsm * resident;
-  pass2_pair_kernel<R, N, BRAGG><<<(unsigned)(ctas < slots ? ctas : slots), Cfg::NT, Cfg::smem, ctx->stream>>>(a);
+  CK(launch_pdl(ctx, pass2_pair_kernel<R, N, BRAGG>, nsm, resident, (unsigned)(ctas < slots ? ctas : slots), Cfg::NT,
+                Cfg::smem, a));
   LAUNCHED(ctx);
   return ATUS_OK;
 }
@@ -348,7 +349,7 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   const int64_t slots = (int64_t)nsm * resident;
   unsigned grid = (unsigned)(work < slots ? work : slots);
   if ((MODE == M2_KIN_RABI || MODE == M2_INV_SOB) && grid > RED_ROWS) grid = RED_ROWS;  // one row of sums per CTA
-  pass2_kernel<R, N, TC, MODE, STRIDED><<<grid, Cfg::NT, smem, ctx->stream>>>(a);
+  CK(launch_pdl(ctx, pass2_kernel<R, N, TC, MODE, STRIDED>, nsm, resident, grid, Cfg::NT, smem, a));
   LAUNCHED(ctx);
   return ATUS_OK;
   }
@@ -399,7 +400,7 @@ static inline int launch_pass3_t(atus_ctx *ctx, PassArgs &a, int axis) {
   const int64_t work = a.per_comp ? ntiles * ctx->ncomp : ntiles;
   const int64_t slots = (int64_t)nsm * resident;
   const unsigned grid = (unsigned)(work < slots ? work : slots);
-  pass3_kernel<R, N, TC, MODE, STRIDED><<<grid, Cfg::NT, smem, ctx->stream>>>(a);
+  CK(launch_pdl(ctx, pass3_kernel<R, N, TC, MODE, STRIDED>, nsm, resident, grid, Cfg::NT, smem, a));
   LAUNCHED(ctx);
   return ATUS_OK;
 }

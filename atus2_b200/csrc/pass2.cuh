@@ -566,6 +566,7 @@ __global__ void __launch_bounds__(P2Cfg<R, N, TC>::NT, p2_minb<R, MODE, TC>) pas
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_om[TC > 2 ? NCPL * Cfg::B : Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];  // couplings of the pencils
   const bool kt_shared = p2_setup<R, N, TC, MODE>(a, smem_raw);
+  pdl_wait();
   __syncthreads();  // twiddle rows and kinetic factors visible to every warp
   const int64_t W = a.per_comp ? a.ntiles * a.ncomp_grid : a.ntiles;
   constexpr bool SUMS = (MODE == M2_KIN_RABI || MODE == M2_INV_SOB);

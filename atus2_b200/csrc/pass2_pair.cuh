@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(PairCfg<R, N>::NT, PairCfg<R, N>::MINB) pass2_
     const TW *tw = (const TW *)a.tw;
     for (int e = threadIdx.x; e < 16 * R2; e += Cfg::NT) twS[(e / R2) * Cfg::TP + e % R2] = tw[((e % R2) * (e / R2)) * (TWN / N)];
   }
+  pdl_wait();
   __syncthreads();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int j = lane % R2, c = (lane / R2) & 1, p = lane / (2 * R2);

@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(Tile2<R>::NT, 3) pass2_tma_kernel(PassArgs a, 
     mbar_init(mb, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();
   __syncthreads();
   const int64_t W = a.ntiles * a.ncomp_grid;
   auto issue = [&](int64_t w) {

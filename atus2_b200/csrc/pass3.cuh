@@ -383,6 +383,7 @@ __global__ void __launch_bounds__(P3Cfg<R, N, TC, STRIDED>::NT, P3Cfg<R, N, TC, 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_om[TC > 2 ? NCPL * Cfg::B : Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];  // couplings of the pencils
   p3_setup<R, N, TC, STRIDED>(a, smem_raw);
+  pdl_wait();
   __syncthreads();  // twiddle rows visible to every warp
   const int64_t W = a.per_comp ? a.ntiles * a.ncomp_grid : a.ntiles;
   for (int64_t w = blockIdx.x; w < W; w += gridDim.x) {
