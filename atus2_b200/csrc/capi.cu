@@ -312,9 +312,9 @@ static int fs_twiddle(atus_ctx *ctx, void *const *f, int nf, int conj_, bool fp6
 
 // One fused four-step pass (M2_FS_*) over nf fields; half: which kinetic
 // table.  ATUS_E_UNSUPPORTED, nothing launched, where a view axis is longer
-// than the register-staged passes (N >= 2^23) or tc > 2.
+// than the register-staged passes (N >= 2^25) or more than two fields meet.
 static int fs_pass(atus_ctx *ctx, int mode, void *const *f, int nf, int half, const NLArgs *nl) {
-  if (!ctx->use_pass2 || ctx->fs_n2 > 2048 || (mode == M2_FS_NL && nf > 2)) return ATUS_E_UNSUPPORTED;
+  if (!ctx->use_pass2 || ctx->fs_n2 > 4096 || (mode == M2_FS_NL && nf > 2)) return ATUS_E_UNSUPPORTED;
   PassArgs a;
   memset(&a, 0, sizeof(a));
   for (int c = 0; c < nf; c++) a.psi[c] = f[c];

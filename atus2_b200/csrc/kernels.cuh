@@ -174,6 +174,50 @@ __device__ __forceinline__ double reduce_2pi(double a) {
   return fma(-q, P3, r);
 }
 
+// v with its sign bits flipped by mask sg (0 or 0x80000000).
+__device__ __forceinline__ double flip1(double x, int sg) {
+  return __hiloint2double(__double2hiint(x) ^ sg, __double2loint(x));
+}
+__device__ __forceinline__ float flip1(float x, int sg) { return __int_as_float(__float_as_int(x) ^ sg); }
+template <typename C> __device__ __forceinline__ C flip(C v, int sg) {
+  v.x = flip1(v.x, sg);
+  v.y = flip1(v.y, sg);
+  return v;
+}
+
+// e^{i x} for |x| < 2^17: x - q pi/2 by Cody and Waite's reduction (the parts
+// of 2 pi above, over 4; q P1 is exact), then Taylor series on |r| <= pi/4 --
+// sin to r^17, cos to r^16, truncation below 1e-19 and 2e-18 -- and the
+// quadrant.  No branch, 30
+// FP64 operations.
+__device__ __forceinline__ double2 expi_cw(double x) {
+  constexpr double P1 = 6.2831853069365025 / 4, P2 = 2.430840202602477e-10 / 4, P3 = 1.40862394607328e-26 / 4;
+  const double q = rint(x * 0.63661977236758134308);
+  const int n = __double2int_rn(q);
+  double r = fma(-q, P1, x);
+  r = fma(-q, P2, r);
+  r = fma(-q, P3, r);
+  const double r2 = r * r;
+  double ps = fma(r2, 1.0 / 355687428096000.0, -1.0 / 1307674368000.0);
+  ps = fma(ps, r2, 1.0 / 6227020800.0);
+  ps = fma(ps, r2, -1.0 / 39916800.0);
+  ps = fma(ps, r2, 1.0 / 362880.0);
+  ps = fma(ps, r2, -1.0 / 5040.0);
+  ps = fma(ps, r2, 1.0 / 120.0);
+  ps = fma(ps, r2, -1.0 / 6.0);
+  const double sn = fma(ps * r2, r, r);
+  double pc = fma(r2, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
+  pc = fma(pc, r2, 1.0 / 479001600.0);
+  pc = fma(pc, r2, -1.0 / 3628800.0);
+  pc = fma(pc, r2, 1.0 / 40320.0);
+  pc = fma(pc, r2, -1.0 / 720.0);
+  pc = fma(pc, r2, 1.0 / 24.0);
+  pc = fma(pc, r2, -0.5);
+  const double cs = fma(pc, r2, 1.0);
+  const double c = (n & 1) ? sn : cs, s = (n & 1) ? cs : sn;
+  return make_double2(flip1(c, ((n + 1) & 2) << 30), flip1(s, (n & 2) << 30));
+}
+
 // sincos() out of line: the step kernels call it from 8 or 16 places each, for
 // arguments that a resolved time step rarely has, and its inlined copies cost
 // the common path registers.
@@ -670,16 +714,6 @@ __device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, d
 }
 
 
-// v with its sign bits flipped by mask sg (0 or 0x80000000).
-__device__ __forceinline__ double flip1(double x, int sg) {
-  return __hiloint2double(__double2hiint(x) ^ sg, __double2loint(x));
-}
-__device__ __forceinline__ float flip1(float x, int sg) { return __int_as_float(__float_as_int(x) ^ sg); }
-template <typename C> __device__ __forceinline__ C flip(C v, int sg) {
-  v.x = flip1(v.x, sg);
-  v.y = flip1(v.y, sg);
-  return v;
-}
 template <typename C> __device__ __forceinline__ C shfl_xor_c(C v, int mask) {
   v.x = __shfl_xor_sync(0xffffffffu, v.x, mask);
   v.y = __shfl_xor_sync(0xffffffffu, v.y, mask);
@@ -831,18 +865,70 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
   }
 }
 
+// Potential step of one component on 16 points a thread: register m is grid
+// index l0 + dl m; XP: x varies along the pencil (x0 + dx m), else it is x0.
+// Eight points at a time: their potential is loaded together, and where every
+// phase of the warp is small (or below 2^17) they take the series (or the
+// reduced series) without a branch a point
+// (16 sites with a call each for larger phases cost the loop its overlap).
+// One component with a potential, FP64: z pass of 256^3 178 -> 138 us, y pass of
+// 2048^2 60 -> 53.
+template <typename R> __device__ __noinline__ void phase8_any(cplx<R> *v, const double *ph) {
+  #pragma unroll 2
+  for (int m = 0; m < 8; m++) v[m] = from_d<R>(cmul(to_d<R>(v[m]), expi<R>(ph[m])));
+}
+template <typename R, bool XP>
+__device__ __forceinline__ void nl_single16(const NLArgs &a, cplx<R> *v, bool live, double x0, double dx, int64_t l0,
+                                            int64_t dl) {
+  using C = cplx<R>;
+  const double *const Vp = (a.kind == K_NL && live) ? a.V[0] : nullptr;
+  const double beta = a.kind == K_NL ? 0.0 : a.L.beta0, shift = a.kind == K_NL ? 0.0 : a.L.DeltaL[0], g = a.gs[0];
+  #pragma unroll
+  for (int h = 0; h < 16; h += 8) {
+    double ph[8];
+    #pragma unroll
+    for (int m = 0; m < 8; m++) ph[m] = Vp ? __ldg(&Vp[l0 + dl * (h + m)]) : 0.0;
+    bool small = true, mid = true;
+    #pragma unroll
+    for (int m = 0; m < 8; m++) {
+      const double rho = (double)v[h + m].x * (double)v[h + m].x + (double)v[h + m].y * (double)v[h + m].y;
+      const double x = XP ? x0 + dx * (h + m) : x0;
+      ph[m] = (a.kind == K_NL ? ph[m] + g * rho : g * rho + (beta * x - shift)) * a.mdt;
+      small = small && fabs(ph[m]) <= 0.03125;
+      mid = mid && fabs(ph[m]) < 131072.0;
+    }
+    if (__all_sync(0xffffffffu, small)) {
+      #pragma unroll
+      for (int m = 0; m < 8; m++) v[h + m] = from_d<R>(cmul(to_d<R>(v[h + m]), expi_series(ph[m])));
+    } else if (__all_sync(0xffffffffu, mid)) {
+      #pragma unroll
+      for (int m = 0; m < 8; m++) v[h + m] = from_d<R>(cmul(to_d<R>(v[h + m]), expi_cw(ph[m])));
+    } else {  // on copies in local memory: calls from here would take the common path's registers
+      C w[8];
+      double q[8];
+      #pragma unroll
+      for (int m = 0; m < 8; m++) {
+        w[m] = v[h + m];
+        q[m] = ph[m];
+      }
+      phase8_any<R>(w, q);
+      #pragma unroll
+      for (int m = 0; m < 8; m++) v[h + m] = w[m];
+    }
+  }
+}
+
 // ------------------------------------------------------------ potential step
 // Point-wise potential step on the ncomp values v[] at grid index l.
 // FP64: the reference's formulas (include/CRT_Base.h:410-439,
 // CRT_Base_IF.h:392-418, bragg.cpp:210-302).  Mixed: FP64 phase arguments,
 // FP32 field arithmetic, and the eigenvalue-free form of the 2x2 exponential.
 // TC: the number of components the calling kernel holds (ncomp <= TC); step
-// kinds that need more components are compiled out.  PREV (one component):
-// the caller has loaded the potential at l into vpre (0 without a potential).
-template <typename R, int TC = MAXC, bool PREV = false>
+// kinds that need more components are compiled out.  cp: the
+// pencil's couplings where the caller has them (coupling_x).
+template <typename R, int TC = MAXC>
 __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, double Omega,
-                                         double eta_c, double eta_s, double vpre = 0.0, const double *cp = nullptr) {
-  static_assert(!PREV || TC == 1, "a pre-loaded potential serves one component");
+                                         double eta_c, double eta_s, const double *cp = nullptr) {
   // couplings of the pencil, where the caller has not evaluated them
   double own[NCPL];
   if constexpr (TC >= 2) {
@@ -888,8 +974,7 @@ __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l,
       if (i >= n) break;
       double phi;
       if (a.kind == K_NL) {
-        if constexpr (PREV) phi = vpre;
-        else phi = a.V[i] ? a.V[i][l] : 0.0;
+        phi = a.V[i] ? a.V[i][l] : 0.0;
         #pragma unroll
         for (int j = 0; j < TC; j++)
           if (j < n) phi += a.gs[i * MAXC + j] * rho[j];

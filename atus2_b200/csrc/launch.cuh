@@ -10,6 +10,7 @@
 #include "pass2_pair.cuh"
 #include "pass2_tma.cuh"
 #include "pass3.cuh"
+#include "pass3_pipe.cuh"
 
 template <typename R, int N, int TC>
 static inline int launch_pass_t(atus_ctx *ctx, PassArgs &a, int axis) {
@@ -355,11 +356,38 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   }
 }
 
-// Launch of pass3_kernel (pencils of 512..2048 points); as launch_pass2_t.
+// Launch of pass3_kernel (pencils of 512..4096 points); as launch_pass2_t.
+// 4096 points where tables and exchange rows fit (one or two components): the
+// shared-memory tile kernel took 385 us for the x pass of 4096 x 2048 FP64 and
+// 602 us for the y pass of 2048 x 4096, these 157 and 129.
+// The tile of launch_pass3_t's strided FP64 passes, the next one prefetched.
+// ATUS_E_UNSUPPORTED, nothing launched, where no CTA would have a next one.
+template <int N, int MODE>
+static inline int launch_pass3_pipe_t(atus_ctx *ctx, PassArgs &a) {
+  using Cfg = P3PipeCfg<N>;
+  static int nsm = 0;
+  if (!nsm) {
+    CK(cudaFuncSetAttribute(pass3_pipe_kernel<N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
+    int dev = 0, n = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    nsm = n;
+  }
+  const int64_t inner = (a.sa + Cfg::B - 1) / Cfg::B, ntiles = (ctx->npts / (N * a.sa)) * inner;
+  const int64_t work = ntiles * ctx->ncomp;
+  if (work <= nsm) return ATUS_E_UNSUPPORTED;
+  a.inner_tiles = inner;
+  a.ntiles = ntiles;
+  CK(launch_pdl(ctx, pass3_pipe_kernel<N, MODE>, nsm, 1, (unsigned)nsm, Cfg::NT, Cfg::smem, a));
+  LAUNCHED(ctx);
+  return ATUS_OK;
+}
+
 template <typename R, int N, int TC, int MODE, bool STRIDED>
 static inline int launch_pass3_t(atus_ctx *ctx, PassArgs &a, int axis) {
   using Cfg = P3Cfg<R, N, TC, STRIDED>;
   constexpr size_t smem = Cfg::smem;
+  static_assert(smem + 2048 <= 227 * 1024 && Cfg::NT <= 1024, "tile too large");
   static int resident = 0;
   static int nsm = 0;
   if (!resident) {
@@ -397,6 +425,12 @@ static inline int launch_pass3_t(atus_ctx *ctx, PassArgs &a, int axis) {
   }
   a.ntiles = ntiles;
   a.ncomp_grid = ctx->ncomp;
+  if constexpr (sizeof(R) == 8 && STRIDED && TC == 1 && N >= 1024 && (MODE == M2_FWD || MODE == M2_INV || MODE == M2_KIN)) {
+    if (a.per_comp) {
+      const int r = launch_pass3_pipe_t<N, MODE>(ctx, a);
+      if (r != ATUS_E_UNSUPPORTED) return r;
+    }
+  }
   const int64_t work = a.per_comp ? ntiles * ctx->ncomp : ntiles;
   const int64_t slots = (int64_t)nsm * resident;
   const unsigned grid = (unsigned)(work < slots ? work : slots);
@@ -421,6 +455,9 @@ static inline int launch_pass2_n(atus_ctx *ctx, PassArgs &a, int axis) {
       case 2048: return launch_pass3_t<R, 2048, TC, MODE, STRIDED>(ctx, a, axis);
       default: break;
     }
+    if constexpr (TC <= 2) {
+      if (ctx->n[axis] == 4096) return launch_pass3_t<R, 4096, TC, MODE, STRIDED>(ctx, a, axis);
+    }
   }
   return ATUS_E_UNSUPPORTED;
 }
@@ -435,6 +472,7 @@ static inline int launch_fs_n(atus_ctx *ctx, PassArgs &a) {
     case 512: return launch_pass3_t<R, 512, TC, MODE, STRIDED>(ctx, a, axis);
     case 1024: return launch_pass3_t<R, 1024, TC, MODE, STRIDED>(ctx, a, axis);
     case 2048: return launch_pass3_t<R, 2048, TC, MODE, STRIDED>(ctx, a, axis);
+    case 4096: return launch_pass3_t<R, 4096, TC, MODE, STRIDED>(ctx, a, axis);
     default: return ATUS_E_UNSUPPORTED;
   }
 }

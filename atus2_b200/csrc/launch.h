@@ -40,7 +40,7 @@ int launch_pass2_f_nl(atus_ctx *ctx, PassArgs &a, int axis, int tc);
 // along the contiguous axis (32..256 points)
 int launch_pass2_d_sob(atus_ctx *ctx, PassArgs &a, int axis, int mode);
 // _fs: the passes of a long 1D axis seen as n1 x n2 points (M2_FS_*), axes of
-// 128..2048 points; tc: components of M2_FS_NL (1 or 2)
+// 128..4096 points; tc: components of M2_FS_NL (1 or 2)
 int launch_fs_d(atus_ctx *ctx, PassArgs &a, int mode, int tc);
 int launch_fs_f(atus_ctx *ctx, PassArgs &a, int mode, int tc);
 int launch_pass2_d_nl3(atus_ctx *ctx, PassArgs &a, int axis);

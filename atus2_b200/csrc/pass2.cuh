@@ -466,28 +466,13 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
     } else if constexpr (TC == 1) {
       int p0[3];
       idx3(a.g, lb, p0[0], p0[1], p0[2]);
-      // the potential, loaded four points ahead of its use (behind the
-      // per-point branches each load would wait on its own)
-      const double *const Vp = a.nl.V[0];
-      const bool preV = a.nl.kind == K_NL && Vp != nullptr && live;
-      constexpr int AHEAD = 4;
-      double vpre[16];
-      auto load_v = [&](int m) { vpre[m] = preV ? __ldg(&Vp[lb + (int64_t)(j + R2 * m) * a.sa]) : 0.0; };
-      #pragma unroll
-      for (int m = 0; m < AHEAD; m++) load_v(m);
-      #pragma unroll
-      for (int m = 0; m < 16; m++) {
-        if (m + AHEAD < 16) load_v(m + AHEAD);
-        const int i = j + R2 * m;
-        const int64_t l = lb + (int64_t)i * a.sa;
-        const int ix = FS ? (int)l : (a.axis == 0) ? i : p0[0];
-        const double x0 = (double)(ix - a.nl.shift0) * a.nl.dx0;
-        double om = 0, ec = 1, es = 0;
-        if (a.nl.kind == K_BRAGG) bragg_coupling(a.nl, x0, om, ec, es);
-        C u[MAXC];
-        u[0] = v[m];
-        if (live) nl_point<R, TC, true>(a.nl, u, l, x0, om, ec, es, vpre[m]);
-        v[m] = u[0];
+      const int64_t l0 = lb + (int64_t)j * a.sa;
+      if (FS || a.axis == 0) {
+        const int i0 = FS ? (int)l0 : j;
+        nl_single16<R, true>(a.nl, v, live, (double)(i0 - a.nl.shift0) * a.nl.dx0,
+                             (double)(FS ? step : R2) * a.nl.dx0, l0, step);
+      } else {
+        nl_single16<R, false>(a.nl, v, live, (double)(p0[0] - a.nl.shift0) * a.nl.dx0, 0.0, l0, step);
       }
     } else {
       // all components of a point meet in shared memory (natural order)
@@ -517,7 +502,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
           C u[MAXC];
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) u[cc] = ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)];
-          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, 0.0, cp);
+          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, cp);
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)] = u[cc];
         }

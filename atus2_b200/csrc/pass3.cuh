@@ -1,6 +1,6 @@
-// pass3.cuh -- register-staged passes for pencils of 512, 1024 and 2048 points.
+// pass3.cuh -- register-staged passes for pencils of 512 to 4096 points.
 //
-// N = 16 M, M = 16 R3 (R3 = 2, 4, 8).  With n = t + M r (t < M, r < 16) and
+// N = 16 M, M = 16 R3 (R3 = 2, 4, 8, 16).  With n = t + M r (t < M, r < 16) and
 // k = q + 16 k2:
 //
 //   X[q + 16 k2] = sum_t W_M^{t k2} W_N^{t q} sum_r x[t + M r] W_16^{r q}
@@ -138,7 +138,7 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
   using TW = typename TwTab<R>::type;
   using Cfg = P3Cfg<R, N, TC, STRIDED>;
   constexpr int M = Cfg::M, B = Cfg::B, NT = Cfg::NT, PB = Cfg::PB;
-  static_assert(N >= 512 && N <= 2048, "three-stage pencils only");
+  static_assert(N >= 512 && N <= 4096, "three-stage pencils only");
   static_assert(Cfg::NPC * M == NT && Cfg::B * TC == Cfg::NPC, "one thread per stage-1 butterfly");
   static_assert(Cfg::smem_ex % 16 == 0, "twiddles are read in 16 bytes");
   C *const ex = reinterpret_cast<C *>(smem_raw);
@@ -185,10 +185,8 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
   #pragma unroll
   for (int r = 0; r < 16; r++) v[r] = live ? src[r * step] : mk<R>(0, 0);
 
-  // one-component potential step: the potential of the thread's 16 points
-  // is requested into L2 now and loaded eight points ahead of its use after
-  // the inverse transform (behind the per-point branches each load would
-  // wait on its own)
+  // one-component potential step: the potential of the thread's 16 points is
+  // requested into L2 now
   const double *const Vp = a.nl.V[0];
   const bool preV = (MODE == M2_NL || MODE == M2_FS_NL) && TC == 1 && a.nl.kind == K_NL && Vp != nullptr && live;
   if (preV) {
@@ -289,24 +287,13 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
     } else if constexpr (TC == 1) {
       int p0[3];
       idx3(a.g, lb, p0[0], p0[1], p0[2]);
-      constexpr int AHEAD = 8;  // potential loads in flight
-      double vpre[16];
-      auto load_v = [&](int m) { vpre[m] = preV ? __ldg(&Vp[lb + (int64_t)(t + M * m) * a.sa]) : 0.0; };
-      #pragma unroll
-      for (int m = 0; m < AHEAD; m++) load_v(m);
-      #pragma unroll
-      for (int m = 0; m < 16; m++) {
-        if (m + AHEAD < 16) load_v(m + AHEAD);
-        const int i = t + M * m;
-        const int64_t l = lb + (int64_t)i * a.sa;
-        const int ix = FS ? (int)l : (a.axis == 0) ? i : p0[0];
-        const double x0 = (double)(ix - a.nl.shift0) * a.nl.dx0;
-        double om = 0, ec = 1, es = 0;
-        if (a.nl.kind == K_BRAGG) bragg_coupling(a.nl, x0, om, ec, es);
-        C u[MAXC];
-        u[0] = v[m];
-        if (live) nl_point<R, TC, true>(a.nl, u, l, x0, om, ec, es, vpre[m]);
-        v[m] = u[0];
+      const int64_t l0 = lb + (int64_t)t * a.sa;
+      if (FS || a.axis == 0) {
+        const int i0 = FS ? (int)l0 : t;
+        nl_single16<R, true>(a.nl, v, live, (double)(i0 - a.nl.shift0) * a.nl.dx0,
+                             (double)(FS ? step : M) * a.nl.dx0, l0, step);
+      } else {
+        nl_single16<R, false>(a.nl, v, live, (double)(p0[0] - a.nl.shift0) * a.nl.dx0, 0.0, l0, step);
       }
     } else {
       // all components of a point meet in shared memory (natural order)
@@ -336,7 +323,7 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
           C u[MAXC];
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) u[cc] = ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)];
-          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, 0.0, cp);
+          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, cp);
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)] = u[cc];
         }
