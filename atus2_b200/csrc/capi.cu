@@ -729,6 +729,14 @@ static int wait_check(atus_ctx *ctx) {
   return fail(ctx, ATUS_E_CUDA, "a TMA tile copy did not complete within the wait limit");
 }
 
+// The captured Sobolev iterations hold the kernels' arguments (interaction
+// matrix, potential pointers, filter coefficients, wait limits): a call that
+// changes one of them drops the graph, and the next descent captures it again.
+static void drop_sob_graph(atus_ctx *ctx) {
+  if (ctx->sob_graph) cudaGraphExecDestroy(ctx->sob_graph);
+  ctx->sob_graph = nullptr;
+}
+
 int atus_set_stream(atus_ctx *ctx, void *stream) {
   if (!ctx) return ATUS_E_ARG;
   CK(cudaStreamSynchronize(ctx->stream));
@@ -768,6 +776,7 @@ int atus_get_dt(const atus_ctx *ctx, double *dt) {
 
 int atus_set_wait_limits(atus_ctx *ctx, int64_t wait_rounds, int drop_copies) {
   if (!ctx || wait_rounds < 1 || (drop_copies != 0 && drop_copies != 1)) return ATUS_E_ARG;
+  drop_sob_graph(ctx);
   ctx->wait_limit = (long)wait_rounds;
   ctx->drop_copies = drop_copies;
   return ATUS_OK;
@@ -793,6 +802,7 @@ int atus_get_time(const atus_ctx *ctx, double *t) {
 
 int atus_set_gs(atus_ctx *ctx, const double *gs) {
   if (!ctx || !gs) return ATUS_E_ARG;
+  drop_sob_graph(ctx);
   for (int i = 0; i < MAXC * MAXC; i++) ctx->gs[i] = 0;
   for (int i = 0; i < ctx->ncomp; i++)
     for (int j = 0; j < ctx->ncomp; j++) ctx->gs[i * MAXC + j] = gs[j + ctx->ncomp * i];
@@ -859,6 +869,7 @@ int atus_clone(const atus_ctx *src, atus_ctx **out) {
 
 int atus_set_potential(atus_ctx *ctx, int comp, const double *V) {
   if (!ctx || comp < 0 || comp >= ctx->ncomp) return ATUS_E_ARG;
+  if (!V || !ctx->V[comp]) drop_sob_graph(ctx);  // the pointer changes
   if (!V) {
     CK(cudaStreamSynchronize(ctx->stream));
     cudaFree(ctx->V[comp]);
@@ -1636,6 +1647,7 @@ static int sob_iterate_dev(atus_ctx *ctx) {
 int atus_sob_init(atus_ctx *ctx, const double *alpha, double stepsize) {
   if (!ctx || !alpha) return ATUS_E_ARG;
   if (ctx->prec != ATUS_PREC_FP64) return fail(ctx, ATUS_E_UNSUPPORTED, "the Sobolev descent runs in FP64");
+  drop_sob_graph(ctx);
   for (int i = 0; i < ctx->ncomp; i++) {
     ctx->sob_alpha[i] = alpha[i];
     if (!ctx->sob_lap[i]) {

@@ -68,3 +68,30 @@ def test_descent_matches_numpy(shape, ncomp):
     for c in range(ncomp):
         assert np.linalg.norm(s.psi(c) - ref[c]) <= 1e-12 * np.linalg.norm(ref[c])
     s.close()
+
+
+def test_descent_follows_changed_parameters():
+    """A second descent on the same context with another interaction strength,
+    then without the potential, equals a fresh context's (the iterations
+    captured by the first hold neither)."""
+    shape = (4, 8, 32)
+    h = binfmt.make_header(3, list(shape), [-4.0] * 3, [4.0] * 3)
+    X = np.meshgrid(*[binfmt.x_coords(h, a) for a in range(3)], indexing="ij")
+    psi = np.exp(-0.4 * sum(x * x for x in X))
+    V = sum(0.5 * x * x for x in X)
+
+    def run(s, g, V):
+        s.set_psi(0, psi)
+        s.set_gs([g])
+        s.set_potential(0, V)
+        s.sob_init([0.5], STEP)
+        s.sob_run(0.0, ITERS)
+        return s.psi(0)
+
+    used = Solver(h, 1, PREC_FP64)
+    run(used, 10.0, V)
+    for g, pot in ((200.0, V), (200.0, None), (50.0, V)):
+        fresh = Solver(h, 1, PREC_FP64)
+        np.testing.assert_array_equal(run(used, g, pot), run(fresh, g, pot))
+        fresh.close()
+    used.close()
