@@ -78,6 +78,8 @@ struct atus_batch {
   double *d_t0 = nullptr, *h_t0 = nullptr;
   void *tw = nullptr;              // twiddles in the field precision
   double2 *unit = nullptr;         // factor (1, 0) of the absent third axis
+  double2 *stage = nullptr;        // complex128 copy of a complex64 field on its way out
+  int64_t stage_n = 0;
   std::vector<Class> cls;
   cudaStream_t st = nullptr;
   std::vector<cudaStream_t> side;   // one per 1D class (concurrent persistent kernels)
@@ -506,6 +508,7 @@ void atus_batch_destroy(atus_batch *b) {
   if (b->h_t0) cudaFreeHost(b->h_t0);
   cudaFree(b->tw);
   cudaFree(b->unit);
+  cudaFree(b->stage);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
   for (cudaEvent_t e : b->joins) cudaEventDestroy(e);
   if (b->e0) cudaEventDestroy(b->e0);
@@ -534,17 +537,27 @@ int atus_batch_upload_psi(atus_batch *b, int i, int comp, const double *psi) {
 int atus_batch_download_psi(atus_batch *b, int i, int comp, double *psi) {
   if (!b || !psi || i < 0 || i >= (int)b->inst.size() || comp < 0 || comp > 1) return ATUS_E_ARG;
   const int64_t np = npts(b->inst[i]);
-  BCK(cudaStreamSynchronize(b->st));
-  if (b->prec == ATUS_PREC_FP64) {
-    BCK(cudaMemcpy(psi, b->psi[comp][i], 16 * np, cudaMemcpyDeviceToHost));
-  } else {
-    std::vector<float2> f(np);
-    BCK(cudaMemcpy(f.data(), b->psi[comp][i], 8 * np, cudaMemcpyDeviceToHost));
-    for (int64_t l = 0; l < np; l++) {
-      psi[2 * l] = f[l].x;
-      psi[2 * l + 1] = f[l].y;
+  const void *src = b->psi[comp][i];
+  if (b->prec != ATUS_PREC_FP64) {
+    // widened on the device into a buffer kept for the batch (the largest
+    // instance's size), so the host only receives
+    if (b->stage_n < np) {
+      BCK(cudaStreamSynchronize(b->st));
+      cudaFree(b->stage);
+      b->stage = nullptr;
+      b->stage_n = 0;
+      int64_t most = 0;
+      for (const atus_batch_instance &in : b->inst) most = std::max(most, npts(in));
+      if (cudaMalloc(&b->stage, 16 * most) != cudaSuccess) return fail(b, ATUS_E_NOMEM, "download buffer");
+      b->stage_n = most;
     }
+    const int blocks = (int)std::min<int64_t>((np + 255) / 256, b->nsm * 8);
+    convert_out_kernel<float><<<blocks, 256, 0, b->st>>>(b->stage, b->psi[comp][i], np);
+    BCK(cudaGetLastError());
+    src = b->stage;
   }
+  BCK(cudaMemcpyAsync(psi, src, 16 * np, cudaMemcpyDeviceToHost, b->st));
+  BCK(cudaStreamSynchronize(b->st));
   return ATUS_OK;
 }
 

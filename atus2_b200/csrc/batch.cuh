@@ -79,10 +79,12 @@ __global__ void __launch_bounds__(Tile2<R>::NT, Tile2<R>::MINB) batch_pass2_kern
   __shared__ double s_om[Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];
   __shared__ __align__(16) PassArgs sa;
   bool setup = false;
+  int cur = -1;
   const int64_t W = bp.items * bp.ninst;
   for (int64_t w = blockIdx.x; w < W; w += gridDim.x) {
     const int inst = (int)(w / bp.items);
-    bpass_args(bp, inst, &sa);
+    if (inst != cur) bpass_args(bp, inst, &sa);  // a CTA's items come instance by instance
+    cur = inst;
     if (!setup) {  // twiddle rows (the same for every instance of the class)
       p2_setup<R, N, TC, M2_INV>(sa, smem_raw);
       setup = true;
@@ -107,10 +109,12 @@ __global__ void __launch_bounds__(P5Cfg<R, TC>::NT, 4) batch_pass512_kernel(BPas
   __shared__ double s_om[Cfg::B], s_ec[Cfg::B], s_es[Cfg::B];
   __shared__ __align__(16) PassArgs sa;
   bool setup = false;
+  int cur = -1;
   const int64_t W = bp.items * bp.ninst;
   for (int64_t w = blockIdx.x; w < W; w += gridDim.x) {
     const int inst = (int)(w / bp.items);
-    bpass_args(bp, inst, &sa);
+    if (inst != cur) bpass_args(bp, inst, &sa);  // a CTA's items come instance by instance
+    cur = inst;
     if (!setup) {
       p5_setup<R, TC>(sa, smem_raw);
       setup = true;
@@ -143,10 +147,12 @@ __global__ void __launch_bounds__(Tile<R>::NT) batch_tile_kernel(BPass bp) {
   C *const s = reinterpret_cast<C *>(smem_raw);
   __shared__ double s_om[B], s_ec[B], s_es[B];
   __shared__ __align__(16) PassArgs sa;
+  int cur = -1;
   const int64_t W = bp.items * bp.ninst;
   for (int64_t w = blockIdx.x; w < W; w += gridDim.x) {
     const int inst = (int)(w / bp.items);
-    bpass_args(bp, inst, &sa);
+    if (inst != cur) bpass_args(bp, inst, &sa);  // a CTA's items come instance by instance
+    cur = inst;
     const PassArgs &a = sa;
     const typename TwTab<R>::type *tw = (const typename TwTab<R>::type *)a.tw;
     const TileGeo g = tile_geo<B, N>(a, w % bp.items);

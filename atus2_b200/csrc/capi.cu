@@ -75,16 +75,18 @@ static int build_kinetic(atus_ctx *ctx) {
     for (int c = 0; c < ctx->ncomp; c++) {
       for (int ax = 0; ax < 3; ax++) {
         const int64_t n = ctx->n[ax];
+        const bool fs = ctx->fs_tw && ax == 0;
+        const int lg1 = fs ? ilog2(ctx->fs_n1) : 0, lg2 = fs ? ilog2(ctx->fs_n2) : 0;
         std::vector<double2> tab(n);
-        for (int64_t i = 0; i < n; i++) {
+        for (int64_t at = 0; at < n; at++) {
+          // a long 1D axis: wavenumber k1 + n1 k2 at k1 n2 + k2, where the
+          // four-step spectrum holds it
+          const int64_t i = fs ? (at >> lg2) + ((at & (ctx->fs_n2 - 1)) << lg1) : at;
           double phi = 0.0;
           if (ax < ctx->dim) {
             const double k = ctx->dk[ax] * (double)wrapped(i, n);
             phi = (-ctx->dt) * ((k * ctx->alpha[c][ax]) * k);
           }
-          // a long 1D axis: wavenumber k1 + n1 k2 at k1 n2 + k2, where the
-          // four-step spectrum holds it
-          const int64_t at = (ctx->fs_tw && ax == 0) ? (i % ctx->fs_n1) * ctx->fs_n2 + i / ctx->fs_n1 : i;
           tab[at].x = (hf == 0) ? cos(0.5 * phi) : cos(phi);
           tab[at].y = (hf == 0) ? sin(0.5 * phi) : sin(phi);
         }
@@ -241,6 +243,13 @@ static int grid_blocks(int64_t n, int threads) {
 // view axis 1, contiguous).  Forward: transform along r, times W_N^{r' c}
 // (r' the transformed index), transform along c; element (k1, k2) then holds
 // X[k1 + n1 k2].  Inverse: the same steps backwards with conjugate twiddles.
+// The twiddles in the order of the field, r n2 + c holding W_N^{r c} (w: W_N^m):
+// the passes read them with their own points instead of gathering.
+__global__ void fs_table_kernel(const double2 *w, double2 *t, int64_t n2c, int64_t N) {
+  for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < N; l += (int64_t)gridDim.x * blockDim.x)
+    t[l] = w[((l / n2c) * (l % n2c)) % N];
+}
+
 template <typename R>
 __global__ void fs_twiddle_kernel(void *psi, const double2 *tw, int64_t N, int conj_) {
   cplx<R> *p = static_cast<cplx<R> *>(psi);
@@ -656,18 +665,18 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
     ctx->fs_n2 = ctx->n[0] / ctx->fs_n1;
     std::vector<double2> t(ctx->n[0]);
     const long double two_pi = 6.283185307179586476925286766559005768L;
-    std::vector<double2> w(ctx->n[0]);
     for (int64_t m = 0; m < ctx->n[0]; m++) {
       const long double th = two_pi * (long double)m / (long double)ctx->n[0];
-      w[m].x = (double)cosl(th);
-      w[m].y = (double)(-sinl(th));
+      t[m].x = (double)cosl(th);
+      t[m].y = (double)(-sinl(th));
     }
-    // in the order of the field, r n2 + c holding W_N^{r c}: the passes read
-    // it with their own points instead of gathering
-    for (int64_t r = 0; r < ctx->fs_n1; r++)
-      for (int64_t c = 0; c < ctx->fs_n2; c++) t[r * ctx->fs_n2 + c] = w[(r * c) % ctx->n[0]];
     ok = cudaMalloc(&ctx->fs_tw, sizeof(double2) * ctx->n[0]) == cudaSuccess &&
-         cudaMemcpy(ctx->fs_tw, t.data(), sizeof(double2) * ctx->n[0], cudaMemcpyHostToDevice) == cudaSuccess;
+         cudaMemcpy(ctx->scratch, t.data(), sizeof(double2) * ctx->n[0], cudaMemcpyHostToDevice) == cudaSuccess;
+    if (ok) {
+      fs_table_kernel<<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>((const double2 *)ctx->scratch, ctx->fs_tw,
+                                                                            ctx->fs_n2, ctx->npts);
+      ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(ctx->stream) == cudaSuccess;
+    }
     if (!ok) {
       atus_destroy(ctx);
       return ATUS_E_NOMEM;
