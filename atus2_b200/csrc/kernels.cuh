@@ -8,8 +8,8 @@
 //              as  FFT_a -> kinetic phase -> IFFT_a   (k-space half-step) and
 //              IFFT_a -> potential/Bragg step -> FFT_a (real-space half-step),
 //              so each Strang step of a 2D grid is two passes over the fields.
-// block1d_kernel  1D grids: a whole Strang block (Nk steps) with the field
-//              resident in shared memory.
+// block1d_kernel  1D grids of 2..128 points: a whole Strang block (Nk steps) with
+//              the field resident in shared memory (longer ones: line1d.cuh).
 // nl_kernel    the potential step alone (Do_NL_Step / Do_Bragg_ad).
 // reduce_*     deterministic two-level FP64 reductions.
 #pragma once

@@ -345,10 +345,9 @@ ATUS_API int atus_guess_decode(atus_ctx *ctx, int comp, const double *coef, cons
  * Independent two-component bragg_ad instances (1D lengths 1024..16384, square
  * 2D grids 64^2..512^2; powers of two), all advanced by one CUDA-graph launch
  * per Strang block: 1D instances by one persistent kernel per length with the
- * instance resident in shared memory, 2D instances by batched passes over all
- * instances of a size.  atus_batch_tune picks, per size class, the kernel
- * variant (threads per CTA and resident components for 1D; register-staged or
- * shared-memory tile passes for 2D) from timed probe runs on copies of the
+ * instance on chip, 2D instances by batched passes over all instances of a
+ * size.  atus_batch_tune picks, per size class, the kernel variant (CTAs per
+ * instance for 1D; register-staged or shared-memory tile passes for 2D) from timed probe runs on copies of the
  * fields.  Each instance computes what a context with the same parameters
  * computes with atus_strang_block(ATUS_STEP_BRAGG_AD) and F[j] =
  * AMP_T(t1_j) = exp(-(t1_j - tc)^2 / (2 sigma^2)), t1_j = t0 + dt (j + 1). */
