@@ -900,7 +900,7 @@ __device__ __forceinline__ void nl_single16(const NLArgs &a, cplx<R> *v, bool li
     if (__all_sync(0xffffffffu, small)) {
       #pragma unroll
       for (int m = 0; m < 8; m++) v[h + m] = from_d<R>(cmul(to_d<R>(v[h + m]), expi_series(ph[m])));
-    } else if (__all_sync(0xffffffffu, mid)) {
+    } else if (sizeof(R) == 8 && __all_sync(0xffffffffu, mid)) {  // complex64: expi<float>, as everywhere
       #pragma unroll
       for (int m = 0; m < 8; m++) v[h + m] = from_d<R>(cmul(to_d<R>(v[h + m]), expi_cw(ph[m])));
     } else {  // on copies in local memory: calls from here would take the common path's registers
