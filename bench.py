@@ -369,7 +369,7 @@ def config1_inputs():
 
 def run_config1(stream, with_cpu):
     """Config 1 at full length: 20 blocks of 1000 Strang steps of the 1D
-    rt_solver workload, FP64, one CTA holding the field in shared memory."""
+    rt_solver workload, FP64, the field on chip."""
     import torch
 
     from atus2_b200 import PREC_FP64, STEP_NL, Solver
@@ -406,7 +406,7 @@ def run_config1(stream, with_cpu):
         "gpu_launches": s.launches - l0,
         "norm_drift": (s.particle_number(0) - n0) / n0,
         "dtype": "f64",
-        "bound": "latency / FP64 issue of one SM: the 64 KB field stays in one CTA's shared memory for a "
+        "bound": "step latency: the 64 KB field stays on chip, on one cluster of 8 CTAs, for a "
                  "whole block, so HBM is not on the path (72 B/pt-step model: "
                  f"{72.0 * C1_N * steps / (ms * 1e-3) / 1e9:.1f} GB/s equivalent)",
     }
@@ -626,7 +626,7 @@ def run_cpu_baseline(n_short=1, n_long=5, repeats=3):
 # FP64 256^3 x 2 kernels, each from one ncu capture of that kernel on this
 # workload on a B200 (a profiler cannot run inside the timed bench, so the
 # capture's figure is carried here).
-NCU_TRAFFIC_FP64 = {"pass2_kernel M2_NL (z)": 1.0941e9, "pass2_tma_kernel M2_KIN (x)": 1.0155e9}
+NCU_TRAFFIC_FP64 = {"pass2_tma_kernel M2_KIN (x)": 1.0155e9}
 
 
 def roofline(s, kind, peak, peak_kind, fp64=True):
@@ -635,7 +635,7 @@ def roofline(s, kind, peak, peak_kind, fp64=True):
     # three axis passes of the real-space half step (strided passes take
     # their tiles by TMA unless ATUS_TMA=0)
     sk = "pass2_kernel" if os.environ.get("ATUS_TMA") == "0" else "pass2_tma_kernel"
-    names = [f"{sk} M2_KIN (x)", f"{sk} M2_INV (y)", "pass2_kernel M2_NL (z)", f"{sk} M2_FWD (y)"]
+    names = [f"{sk} M2_KIN (x)", f"{sk} M2_INV (y)", "pass2_pair_kernel (z)", f"{sk} M2_FWD (y)"]
     # dominant pass: largest device time per Strang step
     bi = max(range(len(prof)), key=lambda q: prof[q][0] * prof[q][1])
     ms, lps, by = prof[bi]
