@@ -610,15 +610,23 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
   if (cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return ATUS_E_CUDA; }
   ctx->stream = ctx->own_stream;
   bool ok = true;
+  // Every copy and fill below runs on the context's stream, which is waited
+  // for before the call returns (build_kinetic).  On the default stream they
+  // would not be ordered before the context's kernels: that stream does not
+  // block this one, and a copy from pageable memory returns while its last
+  // part is still on its way.
+  auto upload = [&](void *dst, const void *src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream) == cudaSuccess;
+  };
   for (int c = 0; c < ncomp && ok; c++) {
     ok = cudaMalloc(&ctx->psi[c], ctx->csize * ctx->npts) == cudaSuccess;
-    if (ok) ok = cudaMemset(ctx->psi[c], 0, ctx->csize * ctx->npts) == cudaSuccess;
+    if (ok) ok = cudaMemsetAsync(ctx->psi[c], 0, ctx->csize * ctx->npts, ctx->stream) == cudaSuccess;
   }
   if (ok) ok = cudaMalloc(&ctx->scratch, 16 * ctx->npts) == cudaSuccess;
   if (ok) ok = cudaMalloc(&ctx->red_partial, sizeof(double) * RED_ROWS * RED_MAXQ) == cudaSuccess;
   if (ok)
     ok = cudaMalloc(&ctx->red_count, sizeof(unsigned)) == cudaSuccess &&
-         cudaMemset(ctx->red_count, 0, sizeof(unsigned)) == cudaSuccess;
+         cudaMemsetAsync(ctx->red_count, 0, sizeof(unsigned), ctx->stream) == cudaSuccess;
   if (ok) {  // one pinned block: reduction totals, the descent's scalars, the error word
     constexpr size_t red = sizeof(double) * RED_MAXQ, sob = (sizeof(SobDev) + 15) / 16 * 16;
     ok = cudaMallocHost(&ctx->pinned, red + sob + sizeof(int)) == cudaSuccess;
@@ -633,7 +641,7 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
     ok = cudaMalloc(&ctx->tw64, 16 * TWN) == cudaSuccess;
     if (ok) {
       auto t = twiddles<double>();
-      ok = cudaMemcpy(ctx->tw64, t.data(), 16 * TWN, cudaMemcpyHostToDevice) == cudaSuccess;
+      ok = upload(ctx->tw64, t.data(), 16 * TWN);
     }
     ctx->tw = ctx->tw64;
     if (ok && precision == ATUS_PREC_MIXED) {
@@ -648,7 +656,7 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
           t4[m].z = (float)(t[m].x - (double)t4[m].x);
           t4[m].w = (float)(t[m].y - (double)t4[m].y);
         }
-        ok = cudaMemcpy(ctx->tw, t4.data(), sizeof(float4) * TWN, cudaMemcpyHostToDevice) == cudaSuccess;
+        ok = upload(ctx->tw, t4.data(), sizeof(float4) * TWN);
       }
     }
   }
@@ -671,11 +679,11 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
       t[m].y = (double)(-sinl(th));
     }
     ok = cudaMalloc(&ctx->fs_tw, sizeof(double2) * ctx->n[0]) == cudaSuccess &&
-         cudaMemcpy(ctx->scratch, t.data(), sizeof(double2) * ctx->n[0], cudaMemcpyHostToDevice) == cudaSuccess;
+         upload(ctx->scratch, t.data(), sizeof(double2) * ctx->n[0]);
     if (ok) {
       fs_table_kernel<<<grid_blocks(ctx->npts, 256), 256, 0, ctx->stream>>>((const double2 *)ctx->scratch, ctx->fs_tw,
                                                                             ctx->fs_n2, ctx->npts);
-      ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(ctx->stream) == cudaSuccess;
+      ok = cudaGetLastError() == cudaSuccess;
     }
     if (!ok) {
       atus_destroy(ctx);
