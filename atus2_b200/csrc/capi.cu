@@ -156,7 +156,7 @@ static int tc_for(int ncomp) { return ncomp <= 1 ? 1 : (ncomp <= 2 ? 2 : 4); }
 // points, the pass shapes of the split-step schedule), else the tile kernel.
 static int dispatch_pass(atus_ctx *ctx, PassArgs &a, int axis, int tc) {
   const bool dbl = (ctx->prec == ATUS_PREC_FP64);
-  if (ctx->use_pass2) {
+  if (ctx->use_pass2 && !(ctx->dense && ctx->n[axis] == 4096)) {
     const bool strided = axis < ctx->dim - 1;
     int r = ATUS_E_UNSUPPORTED;
     if (a.op == OP_NONE && a.t2 == T_NONE && (a.t1 == T_FWD || a.t1 == T_INV)) {
@@ -164,10 +164,12 @@ static int dispatch_pass(atus_ctx *ctx, PassArgs &a, int axis, int tc) {
       r = dbl ? launch_pass2_d_t(ctx, a, axis, mode, strided) : launch_pass2_f_t(ctx, a, axis, mode, strided);
     } else if ((a.op == OP_KIN || a.op == OP_FILT) && a.t1 == T_FWD && a.t2 == T_INV && strided) {
       r = dbl ? launch_pass2_d_k(ctx, a, axis) : launch_pass2_f_k(ctx, a, axis);
-    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 3) {
+    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 3 && !ctx->dense) {
       r = dbl ? launch_pass2_d_nl3(ctx, a, axis) : launch_pass2_f_nl3(ctx, a, axis);
-    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 4) {
+    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 4 && !ctx->dense) {
       r = dbl ? launch_pass2_d_nl4(ctx, a, axis) : launch_pass2_f_nl4(ctx, a, axis);
+    } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && tc == 2 && ctx->dense) {
+      r = launch_pass2_d_meet(ctx, a, axis);
     } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && tc <= 2) {
       r = dbl ? launch_pass2_d_nl(ctx, a, axis, tc) : launch_pass2_f_nl(ctx, a, axis, tc);
     }
@@ -594,6 +596,7 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
   else if (grid->dim == 2) { ctx->ar = ctx->d[0] * ctx->d[1]; ctx->ar_k = ctx->dk[0] * ctx->dk[1]; }
   else { ctx->ar = ctx->d[0] * ctx->d[1] * ctx->d[2]; ctx->ar_k = ctx->dk[0] * ctx->dk[1] * ctx->dk[2]; }
   ctx->t = grid->t;
+  ctx->dense = ctx->dim >= 2 && ncomp >= 2 && precision == ATUS_PREC_FP64 && ctx->npts <= 8192;
   {
     // ATUS_PASS2=0: tile kernel only (A/B comparisons of the two pass kernels)
     const char *p2 = getenv("ATUS_PASS2");

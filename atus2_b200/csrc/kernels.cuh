@@ -50,13 +50,15 @@ enum { K_NL = 0, K_NL_IF = 1, K_BRAGG = 2, K_DBRAGG = 3, K_NL_IF2 = 4, K_BRAGG_D
 // S psi and S(W psi) with their products with psi).
 // M2_FILT: FFT, Sobolev or Laplace filter, IFFT (apart from M2_KIN, whose
 // complex64 x pass went from 160 to 170 us on 256^3 x 2 with both in one).
+// M2_NL_MEET: M2_NL of two components that meet in shared memory, a point at a
+// time (atus_ctx::dense).
 // M2_FS_*: the passes of a long 1D axis seen as n1 x n2 points (four-step
 // transforms), the twiddles W_N^{r c} applied in registers:
 //   M2_FS_FWD  strided axis: FFT, twiddles
 //   M2_FS_NL   strided axis: IFFT, potential step, FFT, twiddles
 //   M2_FS_KIN  contiguous axis: FFT, kinetic factor, IFFT, conjugate twiddles
 enum { M2_FWD = 0, M2_INV = 1, M2_KIN = 2, M2_NL = 3, M2_KIN_RABI = 4, M2_FWD_SOB = 5, M2_INV_SOB = 6,
-       M2_FS_FWD = 7, M2_FS_NL = 8, M2_FS_KIN = 9, M2_FILT = 10 };
+       M2_FS_FWD = 7, M2_FS_NL = 8, M2_FS_KIN = 9, M2_FILT = 10, M2_NL_MEET = 11 };
 
 struct LaserD {
   double beta0, DeltaL[MAXC], Amp0, laser_k0, laser_dk0, laser_domh0, phase0, chirp_rate0, chirp;
@@ -243,13 +245,29 @@ __device__ __forceinline__ double2 expi_series(double x) {
 }
 __device__ __forceinline__ void sincos_step(double x, double *s, double *c) {
   if (fabs(x) <= 0.03125) {
-    const double2 e = expi_series(x);
+    // Taylor series to x^7 (sin) and x^8 (cos): the first omitted terms,
+    // x^9/9! and x^10/10!, are below 2.5e-18 x and 2.5e-22 for |x| <= 1/32
+    const double x2 = x * x;
+    double ps = fma(x2, -1.0 / 5040.0, 1.0 / 120.0);
+    ps = fma(ps, x2, -1.0 / 6.0);
+    *s = fma(ps * x2, x, x);
+    double pc = fma(x2, 1.0 / 40320.0, -1.0 / 720.0);
+    pc = fma(pc, x2, 1.0 / 24.0);
+    pc = fma(pc, x2, -0.5);
+    *c = fma(pc, x2, 1.0);
+  } else {
+    sincos(x, s, c);
+  }
+}
+
+// The same with its far arguments out of line (FAR), or not.
+template <bool FAR> __device__ __forceinline__ void sincos_step_t(double x, double *s, double *c) {
+  if constexpr (FAR) {
+    const double2 e = fabs(x) <= 0.03125 ? expi_series(x) : sincos_far(x);
     *c = e.x;
     *s = e.y;
   } else {
-    const double2 e = sincos_far(x);
-    *c = e.x;
-    *s = e.y;
+    sincos_step(x, s, c);
   }
 }
 
@@ -274,20 +292,24 @@ template <> __device__ __forceinline__ double2 expi<double>(double phi) {
   sincos_step(phi, &s, &c);
   return make_double2(c, s);
 }
-static __device__ __noinline__ double2 expi_far_mixed(double phi) {
-  float s, c;
-  sincosf((float)reduce_2pi(phi), &s, &c);
-  const double cd = c, sd = s;
-  const double inv = rsqrt(cd * cd + sd * sd);
-  return make_double2(cd * inv, sd * inv);
-}
 template <> __device__ __forceinline__ double2 expi<float>(double phi) {
   if (fabs(phi) <= 0.03125) {  // the usual phase of one time step: FP64 Taylor, |e| = 1 to FP64
     double sd, cd;
     sincos_step(phi, &sd, &cd);
     return make_double2(cd, sd);
   }
-  return expi_far_mixed(phi);
+  float s, c;
+  sincosf((float)reduce_2pi(phi), &s, &c);
+  const double cd = c, sd = s;
+  const double inv = rsqrt(cd * cd + sd * sd);
+  return make_double2(cd * inv, sd * inv);
+}
+// The same with its far arguments out of line.
+static __device__ __noinline__ double2 expi_far_mixed(double phi) { return expi<float>(phi); }
+template <typename R> __device__ __forceinline__ double2 expi_f(double phi) {
+  if (fabs(phi) <= 0.03125) return expi_series(phi);
+  if constexpr (sizeof(R) == 8) return sincos_far(phi);
+  else return expi_far_mixed(phi);
 }
 
 // ------------------------------------------------------------ couplings
@@ -337,8 +359,8 @@ __device__ __forceinline__ void coupling_x(const NLArgs &a, double x0, double *c
 // V includes beta . x over all axes.  The reference's operation order,
 // including its O32 update that reads the already-updated O23 imaginary part
 // (double_bragg.cpp:233).  FP64 arithmetic for both field precisions.
-// cp: Omega_+, Omega_-, cos and sin of -dk x / 2 (coupling_x).
-template <typename R>
+// CP: cp holds Omega_+, Omega_-, cos and sin of -dk x / 2 (coupling_x).
+template <typename R, bool CP>
 __device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, const double *cp) {
   double bx = a.L.beta0 * x0;
   if (a.lg1 > 0) {
@@ -356,29 +378,46 @@ __device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_
   const double *gs = a.gs;  // padded rows: g_ij at i * MAXC + j
   const double V11 = gs[0] * tmp1 + gs[1] * tmp2 + gs[2] * tmp3 + bx;
   const double V22 = gs[MAXC] * tmp1 + gs[MAXC + 1] * tmp2 + gs[MAXC + 2] * tmp3 - a.L.DeltaL[1] + bx;
-  const double dt = a.dt, Op = cp[0], Om = cp[1];
+  const double t1 = a.t1, dt = a.dt;
+  double Op, Om;
+  if constexpr (CP) {
+    Op = cp[0];
+    Om = cp[1];
+  } else {
+    const double F = a.F < 0 ? 0.0 : a.F;
+    double dw = a.L.laser_domh0 + a.L.chirp_rate0 * t1;
+    Op = F * a.L.Amp0 * cos(a.L.laser_k0 * x0 - dw * t1 - a.L.phase0 / 2);
+    dw = a.L.laser_domh0 - a.L.chirp_rate0 * t1;
+    Om = F * a.L.Amp0 * cos(-a.L.laser_k0 * x0 - dw * t1 - a.L.phase0 / 2);
+  }
   double re1, im1;
   if (Om == 0.0 && Op == 0.0) {
-    sincos_step(-dt * V11, &im1, &re1);
+    sincos_step_t<CP>(-dt * V11, &im1, &re1);
     v[0] = from_d<R>(cmul(p1, make_double2(re1, im1)));
-    sincos_step(-dt * V22, &im1, &re1);
+    sincos_step_t<CP>(-dt * V22, &im1, &re1);
     v[1] = from_d<R>(cmul(p2, make_double2(re1, im1)));
     v[2] = from_d<R>(cmul(p3, make_double2(re1, im1)));
     return;
   }
-  const double e0 = cp[2], e1 = cp[3];
+  double e0, e1;
+  if constexpr (CP) {
+    e0 = cp[2];
+    e1 = cp[3];
+  } else {
+    sincos(-0.5 * a.L.laser_dk0 * x0, &e1, &e0);
+  }
   const double OO = Op * Op + Om * Om;
   tmp1 = sqrt((V11 - V22) * (V11 - V22) + 4.0 * OO);
   const double E1 = 0.5 * (V11 + V22 + tmp1);
   const double E2 = 0.5 * (V11 + V22 - tmp1);
   double2 g1, g2, g3;
-  sincos_step(-dt * E1, &im1, &re1);
+  sincos_step_t<CP>(-dt * E1, &im1, &re1);
   tmp1 = 1.0 / fabs((V22 - E1) * (V22 - E1) + Op * Op + Om * Om);
   g1 = make_double2(tmp1 * re1, tmp1 * im1);
-  sincos_step(-dt * E2, &im1, &re1);
+  sincos_step_t<CP>(-dt * E2, &im1, &re1);
   tmp1 = 1.0 / fabs((V22 - E2) * (V22 - E2) + Op * Op + Om * Om);
   g2 = make_double2(tmp1 * re1, tmp1 * im1);
-  sincos_step(-dt * V22, &im1, &re1);
+  sincos_step_t<CP>(-dt * V22, &im1, &re1);
   tmp1 = 1.0 / fabs(OO);
   g3 = make_double2(tmp1 * re1, tmp1 * im1);
   tmp1 = (V22 - E2) * (V22 - E2);
@@ -408,64 +447,67 @@ __device__ __forceinline__ void dbragg_point(const NLArgs &a, cplx<R> *v, int64_
 
 // ------------------------------------------------------------ two-level exponential
 // exp(-i dt [[V11, Omega eta], [Omega conj(eta), V22]]) applied to (p1, p2).
-// With m = (V11+V22)/2, d = (V11-V22)/2, r = sqrt(d^2 + Omega^2), x = r dt:
-//   U = e^{-i dt m} [cos x I - i dt (sin x / x) [[d, Omega eta], [Omega conj(eta), -d]]].
-// cos x and sin x / x are even in x, so for x <= 1/32 -- a time step that
-// resolves the coupling -- they are short Taylor series in x^2 and the step
-// needs no square root and no division.  Truncation below 2.5e-22 (cos, to
-// x^8) and 2.6e-23 (sin x / x, to x^8).
-//
-// FP64 and not `stable` follows the reference's eigenvalue form (bragg.cpp:
-// 226-302, bragg_ds.cpp:215-248), in bragg_pair_eigen below, which divides by
-// (V11 - E+-)^2 + Omega^2 and so carries an error of about 2^-53 |V| / |Omega|
-// (and no unitarity at all once Omega^2 underflows).  Where that error is
-// below 2^-41 (Omega^2 >= 2^-24 (V11^2 + V22^2)) the two forms are the same
-// map to 4.5e-13 and the series serves; below that line, and for longer
-// steps, the reference's operations stay.  Complex64 fields and `stable`
-// always take the eigenvalue-free form.
-// swapped: states 1 and 2 exchanged throughout (V11 with V22, eta with its
-// conjugate, q1 with q2) -- the same step for a thread that holds state 2.
-// 256^3, two components, z pass (components meeting in shared memory):
-// eigenvalue form everywhere 0.368 ms, series 0.337 ms, no exponential 0.283.
-template <typename R>
-__device__ __noinline__ void bragg_pair_general(int stable, double dt, double V11, double V22, double Omega,
-                                                double eta_c, double eta_s, double2 p1, double2 p2, double2 *o1,
-                                                double2 *o2) {
+// FP64 and not `stable`: the reference's eigenvalue form (bragg.cpp:226-302,
+// bragg_ds.cpp:215-248): E+- = (V11 + V22 +- sqrt((V11 - V22)^2 + 4 Omega^2))/2,
+// gamma+- = e^{-i dt E+-} / |(V11 - E+-)^2 + Omega^2|, pure phases when
+// Omega == 0.  Its error, about 2^-53 |V| / |Omega|, is part of what a caller
+// of this form gets: on small dense grids (dt V of 1 and more) the nonlinear
+// step multiplies a difference by 10 to 1000 a block, so that another form of
+// the same map, however exact, ends elsewhere.  Otherwise the eigenvalue-free
+// form
+//   U = e^{-i dt m} [cos(r dt) I - i sin(r dt)/r [[d, W], [W, -d]]],
+// m = (V11+V22)/2, d = (V11-V22)/2, W = Omega, r = sqrt(d^2 + W^2), built in
+// FP64 from unit (cos, sin) pairs, so it is unitary to FP64 accuracy for every
+// Omega (the eigenvalue form divides by (V11 - E)^2 + Omega^2, which loses
+// unitarity once Omega is below the spacing of V and divides by zero once
+// Omega^2 underflows).
+template <bool FAR>
+__device__ __forceinline__ void bragg_eigen(double dt, double V11, double V22, double Omega, double eta_c, double eta_s,
+                                            double2 &q1, double2 &q2) {
+  double re1, im1;
+  if (Omega == 0.0) {
+    sincos_step_t<FAR>(-dt * V11, &im1, &re1);
+    q1 = cmul(q1, make_double2(re1, im1));
+    sincos_step_t<FAR>(-dt * V22, &im1, &re1);
+    q2 = cmul(q2, make_double2(re1, im1));
+    return;
+  }
+  double tmp1 = sqrt((V11 - V22) * (V11 - V22) + 4.0 * Omega * Omega);
+  const double Ep = 0.5 * (V11 + V22 + tmp1);
+  const double Em = 0.5 * (V11 + V22 - tmp1);
+  double2 gp, gm;
+  // the reference's 1 / |(V11 - E+-)^2 + Omega^2| (sums of squares, so
+  // |.| is the identity) from one division: 1/A = B/(AB), 1/B = A/(AB)
+  const double Ap = (V11 - Ep) * (V11 - Ep) + Omega * Omega;
+  const double Am = (V11 - Em) * (V11 - Em) + Omega * Omega;
+  const double inv = 1.0 / (Ap * Am);
+  sincos_step_t<FAR>(-dt * Ep, &im1, &re1);
+  tmp1 = Am * inv;
+  gp = make_double2(tmp1 * re1, tmp1 * im1);
+  sincos_step_t<FAR>(-dt * Em, &im1, &re1);
+  tmp1 = Ap * inv;
+  gm = make_double2(tmp1 * re1, tmp1 * im1);
+  const double O2 = Omega * Omega;
+  const double2 O11 = make_double2(O2 * (gp.x + gm.x), O2 * (gp.y + gm.y));
+  const double a1 = V11 - Ep, a2 = V11 - Em;
+  const double2 O22 = make_double2(a1 * a1 * gp.x + a2 * a2 * gm.x, a1 * a1 * gp.y + a2 * a2 * gm.y);
+  const double2 Os = make_double2(-Omega * (a1 * gp.x + a2 * gm.x), -Omega * (a1 * gp.y + a2 * gm.y));
   const double2 eta = make_double2(eta_c, eta_s);
-  if (sizeof(R) == 8 && !stable) {
-    double re1, im1;
-    if (Omega == 0.0) {
-      sincos_step(-dt * V11, &im1, &re1);
-      *o1 = cmul(p1, make_double2(re1, im1));
-      sincos_step(-dt * V22, &im1, &re1);
-      *o2 = cmul(p2, make_double2(re1, im1));
+  const double2 O12 = cmul(Os, eta);   // eta * O12
+  const double2 O21 = cmulc(Os, eta);  // conj(eta) * O21
+  const double2 p1 = q1, p2 = q2;
+  q1 = cadd(cmul(O11, p1), cmul(O12, p2));
+  q2 = cadd(cmul(O21, p1), cmul(O22, p2));
+}
+
+template <typename R>
+__device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, double V22, double Omega, double eta_c,
+                                           double eta_s, cplx<R> &q1, cplx<R> &q2) {
+  if constexpr (sizeof(R) == 8) {
+    if (!stable) {
+      bragg_eigen<false>(dt, V11, V22, Omega, eta_c, eta_s, q1, q2);
       return;
     }
-    double tmp1 = sqrt((V11 - V22) * (V11 - V22) + 4.0 * Omega * Omega);
-    const double Ep = 0.5 * (V11 + V22 + tmp1);
-    const double Em = 0.5 * (V11 + V22 - tmp1);
-    double2 gp, gm;
-    // the reference's 1 / |(V11 - E+-)^2 + Omega^2| (sums of squares, so
-    // |.| is the identity) from one division: 1/A = B/(AB), 1/B = A/(AB)
-    const double Ap = (V11 - Ep) * (V11 - Ep) + Omega * Omega;
-    const double Am = (V11 - Em) * (V11 - Em) + Omega * Omega;
-    const double inv = 1.0 / (Ap * Am);
-    sincos_step(-dt * Ep, &im1, &re1);
-    tmp1 = Am * inv;
-    gp = make_double2(tmp1 * re1, tmp1 * im1);
-    sincos_step(-dt * Em, &im1, &re1);
-    tmp1 = Ap * inv;
-    gm = make_double2(tmp1 * re1, tmp1 * im1);
-    const double O2 = Omega * Omega;
-    const double2 O11 = make_double2(O2 * (gp.x + gm.x), O2 * (gp.y + gm.y));
-    const double a1 = V11 - Ep, a2 = V11 - Em;
-    const double2 O22 = make_double2(a1 * a1 * gp.x + a2 * a2 * gm.x, a1 * a1 * gp.y + a2 * a2 * gm.y);
-    const double2 Os = make_double2(-Omega * (a1 * gp.x + a2 * gm.x), -Omega * (a1 * gp.y + a2 * gm.y));
-    const double2 O12 = cmul(Os, eta);   // eta * O12
-    const double2 O21 = cmulc(Os, eta);  // conj(eta) * O21
-    *o1 = cadd(cmul(O11, p1), cmul(O12, p2));
-    *o2 = cadd(cmul(O21, p1), cmul(O22, p2));
-    return;
   }
   const double m = 0.5 * (V11 + V22), d = 0.5 * (V11 - V22);
   const double r = sqrt(d * d + Omega * Omega);
@@ -488,12 +530,26 @@ __device__ __noinline__ void bragg_pair_general(int stable, double dt, double V1
   const double2 U11 = cmul(e, make_double2(rr.x, -fd));
   const double2 U22 = cmul(e, make_double2(rr.x, fd));
   const double2 Uo = cmul(e, make_double2(0.0, -fw));
-  const double2 U12 = cmul(Uo, eta), U21 = cmulc(Uo, eta);
-  *o1 = cadd(cmul(U11, p1), cmul(U12, p2));
-  *o2 = cadd(cmul(U21, p1), cmul(U22, p2));
+  const double2 et = make_double2(eta_c, eta_s);
+  const double2 U12 = cmul(Uo, et), U21 = cmulc(Uo, et);
+  const double2 p1 = to_d<R>(q1), p2 = to_d<R>(q2);
+  q1 = from_d<R>(cadd(cmul(U11, p1), cmul(U12, p2)));
+  q2 = from_d<R>(cadd(cmul(U21, p1), cmul(U22, p2)));
 }
 
-// The series form for x^2 = x2 (<= 2^-10), e = e^{-i dt m}.
+template <typename R>
+__device__ __noinline__ void bragg_stable_far(double dt, double V11, double V22, double Omega, double eta_c,
+                                              double eta_s, double2 p1, double2 p2, double2 *o1, double2 *o2) {
+  cplx<R> a = from_d<R>(p1), b = from_d<R>(p2);  // exact: they come from fields of this type
+  bragg_pair<R>(1, dt, V11, V22, Omega, eta_c, eta_s, a, b);
+  *o1 = to_d<R>(a);
+  *o2 = to_d<R>(b);
+}
+
+// The eigenvalue-free form for x^2 = (r dt)^2 = x2 <= 2^-10, e = e^{-i dt m}:
+// cos x and sin x / x are even in x, so they are short Taylor series in x^2
+// and the step needs no square root and no division.  Truncation below 2.5e-22
+// (cos, to x^8) and 2.6e-23 (sin x / x, to x^8).
 template <typename R>
 __device__ __forceinline__ void bragg_series(double dt, double x2, double d, double Omega, double2 e, double eta_c,
                                              double eta_s, cplx<R> &q1, cplx<R> &q2) {
@@ -517,19 +573,26 @@ __device__ __forceinline__ void bragg_series(double dt, double x2, double d, dou
   q2 = from_d<R>(cmul(e, b));
 }
 
+// The same map for kernels that hold their fields in registers: the
+// eigenvalue form with its far phases out of line; the eigenvalue-free form by
+// series for a time step that resolves the coupling, and out of line beyond.
 template <typename R>
-__device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, double V22, double Omega, double eta_c,
-                                           double eta_s, cplx<R> &q1, cplx<R> &q2, bool swapped = false) {
+__device__ __forceinline__ void bragg_pair_far(int stable, double dt, double V11, double V22, double Omega,
+                                               double eta_c, double eta_s, cplx<R> &q1, cplx<R> &q2) {
+  if constexpr (sizeof(R) == 8) {
+    if (!stable) {
+      bragg_eigen<true>(dt, V11, V22, Omega, eta_c, eta_s, q1, q2);
+      return;
+    }
+  }
   const double m = 0.5 * (V11 + V22), d = 0.5 * (V11 - V22), O2 = Omega * Omega;
   const double x2 = (dt * dt) * (d * d + O2);
-  if (x2 <= 0x1p-10 && (sizeof(R) == 4 || stable || O2 >= 0x1p-24 * (V11 * V11 + V22 * V22))) {
-    bragg_series<R>(dt, x2, d, Omega, expi<R>(-dt * m), eta_c, eta_s, q1, q2);
+  if (x2 <= 0x1p-10) {
+    bragg_series<R>(dt, x2, d, Omega, expi_f<R>(-dt * m), eta_c, eta_s, q1, q2);
     return;
   }
-  const double2 p1 = to_d<R>(q1), p2 = to_d<R>(q2);
   double2 o1, o2;
-  if (swapped) bragg_pair_general<R>(stable, dt, V22, V11, Omega, eta_c, -eta_s, p2, p1, &o2, &o1);
-  else bragg_pair_general<R>(stable, dt, V11, V22, Omega, eta_c, eta_s, p1, p2, &o1, &o2);
+  bragg_stable_far<R>(dt, V11, V22, Omega, eta_c, eta_s, to_d<R>(q1), to_d<R>(q2), &o1, &o2);
   q1 = from_d<R>(o1);
   q2 = from_d<R>(o2);
 }
@@ -542,8 +605,9 @@ __device__ __forceinline__ void bragg_pair(int stable, double dt, double V11, do
 // with Omega_s = F_s Amp_s cos(k_s x - (domh_s + rate_s t1) t1 + phase_s/2),
 // eta_s = e^{-i (dk_s x + phase_s)/2}.  F_s is 0 outside the species' pulse
 // window (bragg_ds.cpp:117-127), set on the host.
-// cp: Omega_s, cos and sin of -(dk_s x + phase_s) / 2 per species (coupling_x).
-template <typename R>
+// CP: cp holds Omega_s, cos and sin of -(dk_s x + phase_s) / 2 per species
+// (coupling_x).
+template <typename R, bool CP>
 __device__ __forceinline__ void bragg_ds_point(const NLArgs &a, cplx<R> *v, double x0, const double *cp) {
   double rho[MAXC];
   #pragma unroll
@@ -556,10 +620,21 @@ __device__ __forceinline__ void bragg_ds_point(const NLArgs &a, cplx<R> *v, doub
     for (int j = 1; j < MAXC; j++) p += a.gs[i * MAXC + j] * rho[j];
     phi[i] = p + (((i < 2) ? a.L.beta0 : a.L2.beta0) * x0 - a.L.DeltaL[i]);
   }
+  const double t1 = a.t1, dt = a.dt;
   #pragma unroll
-  for (int s = 0; s < 2; s++)
-    bragg_pair<R>(a.stable, a.dt, phi[2 * s], phi[2 * s + 1], cp[3 * s], cp[3 * s + 1], cp[3 * s + 2], v[2 * s],
-                  v[2 * s + 1]);
+  for (int s = 0; s < 2; s++) {
+    if constexpr (CP) {
+      bragg_pair_far<R>(a.stable, dt, phi[2 * s], phi[2 * s + 1], cp[3 * s], cp[3 * s + 1], cp[3 * s + 2], v[2 * s],
+                        v[2 * s + 1]);
+    } else {
+      const LaserD &L = s ? a.L2 : a.L;
+      const double Omega = (s ? a.F2 : a.F) * L.Amp0 *
+                           cos(L.laser_k0 * x0 - (L.laser_domh0 + L.chirp_rate0 * t1) * t1 + L.phase0 / 2);
+      double es, ec;
+      sincos(-0.5 * (L.laser_dk0 * x0 + L.phase0), &es, &ec);
+      bragg_pair<R>(a.stable, dt, phi[2 * s], phi[2 * s + 1], Omega, ec, es, v[2 * s], v[2 * s + 1]);
+    }
+  }
 }
 
 // ------------------------------------------------------------ numerical n-state steps
@@ -661,8 +736,8 @@ __device__ __forceinline__ double beta_dot_x(const NLArgs &a, int64_t l, double 
 // Then psi <- exp(-i dt A) psi in FP64 for both field precisions.
 // Not inlined: the pass kernels that carry it keep their register budget for
 // the common steps.
-template <typename R, int TC>
-__device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, const double *cp) {
+template <typename R, int TC, bool CP = false>
+__device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, const double *cp = nullptr) {
   constexpr int NC = TC < 3 ? TC : 3;
   const int n = a.ncomp;
   const double bx = beta_dot_x(a, l, x0);
@@ -690,7 +765,13 @@ __device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, d
   if (a.kind == K_RAMAN) {
     if constexpr (NC >= 3) {
       A[2][2].x += a.L.laser_domh0;
-      const double cs = cp[0], sn = cp[1];
+      double sn, cs;
+      if constexpr (CP) {
+        cs = cp[0];
+        sn = cp[1];
+      } else {
+        sincos(a.L.laser_k0 * x0, &sn, &cs);
+      }
       const double h0 = a.L.Amp0 / 2, h1 = a.L.Amp1 / 2;
       A[0][2] = make_double2(h0 * cs, h0 * sn);
       A[2][0] = make_double2(h0 * cs, -h0 * sn);
@@ -698,10 +779,19 @@ __device__ __noinline__ void num_point(const NLArgs &a, cplx<R> *v, int64_t l, d
       A[2][1] = make_double2(h1 * cs, h1 * sn);
     }
   } else {
+    const double t1 = a.th;
     #pragma unroll
     for (int i = 0; i + 1 < NC; i++) {
       if (i + 1 >= n) break;
-      const double cs = cp[2 * i], sn = cp[2 * i + 1];
+      double sn, cs;
+      if constexpr (CP) {
+        cs = cp[2 * i];
+        sn = cp[2 * i + 1];
+      } else {
+        const double k = i == 0 ? a.L.laser_k0 : -a.L.laser_k0;
+        const double rate = i == 0 ? a.L.chirp_rate0 : -a.L.chirp_rate0;
+        sincos((-a.L.laser_domh0 + rate * t1) * t1 + k * x0 - 0.5 * a.L.phase0, &sn, &cs);
+      }
       const double er = a.L.Amp0 * cs / 2 + a.L.Amp1 * cs / 2, ei = a.L.Amp0 * sn / 2 - a.L.Amp1 * sn / 2;
       A[i + 1][0] = make_double2(er, ei);
       A[0][i + 1] = make_double2(er, -ei);
@@ -718,6 +808,22 @@ template <typename C> __device__ __forceinline__ C shfl_xor_c(C v, int mask) {
   v.x = __shfl_xor_sync(0xffffffffu, v.x, mask);
   v.y = __shfl_xor_sync(0xffffffffu, v.y, mask);
   return v;
+}
+
+// The Bragg step of a point whose component c the thread holds as own, the
+// other as oth, in the order of the components whichever thread does it.
+template <typename R>
+__device__ __forceinline__ void bragg_pair_at(const NLArgs &a, int stable, int c, double x0, double om, double ec,
+                                              double es, cplx<R> &own, cplx<R> &oth) {
+  using C = cplx<R>;
+  C p1 = c ? oth : own, p2 = c ? own : oth;
+  const double r1 = (double)p1.x * (double)p1.x + (double)p1.y * (double)p1.y;
+  const double r2 = (double)p2.x * (double)p2.x + (double)p2.y * (double)p2.y;
+  const double V11 = fma(a.L.beta0, x0, a.gs[0] * r1 + a.gs[1] * r2);
+  const double V22 = fma(a.L.beta0, x0, a.gs[MAXC] * r1 + a.gs[MAXC + 1] * r2 - a.L.DeltaL[1]);
+  bragg_pair_far<R>(stable, a.dt, V11, V22, om, ec, es, p1, p2);
+  own = c ? p2 : p1;
+  oth = c ? p1 : p2;
 }
 
 // Potential step of two components on 16 points a thread, the components of a
@@ -737,21 +843,16 @@ __device__ __noinline__ void nl_pair16_any(const NLArgs &a, cplx<R> *v, int c, i
                                            double om, double ec, double es, int64_t l0, int dl) {
   using C = cplx<R>;
   if (a.kind == K_BRAGG || a.kind == K_NUM_BRAGG) {
-    const double bx = a.L.beta0 * x0, bd = bx - a.L.DeltaL[1];
     double cp[NCPL];
     if (a.kind == K_NUM_BRAGG) coupling_x(a, x0, cp);
     #pragma unroll 1
     for (int m = 0; m < 8; m++) {
       C own = v[m], oth = shfl_xor_c(v[m + 8], mask);
       if (a.kind == K_BRAGG) {
-        const double ro = (double)own.x * (double)own.x + (double)own.y * (double)own.y;
-        const double rt = (double)oth.x * (double)oth.x + (double)oth.y * (double)oth.y;
-        const double Vo = a.gs[c * (MAXC + 1)] * ro + a.gs[c ? MAXC : 1] * rt + (c ? bd : bx);
-        const double Vt = a.gs[c ? 1 : MAXC] * ro + a.gs[c ? 0 : MAXC + 1] * rt + (c ? bx : bd);
-        bragg_pair<R>(a.stable, a.dt, Vo, Vt, om, ec, c ? -es : es, own, oth, c != 0);
+        bragg_pair_at<R>(a, a.stable, c, x0, om, ec, es, own, oth);
       } else {
         C w[2] = {c ? oth : own, c ? own : oth};
-        num_point<R, 2>(a, w, l0 + (int64_t)dl * (m ^ (8 * c)), x0, cp);
+        num_point<R, 2, true>(a, w, l0 + (int64_t)dl * (m ^ (8 * c)), x0, cp);
         own = c ? w[1] : w[0];
         oth = c ? w[0] : w[1];
       }
@@ -773,8 +874,8 @@ __device__ __noinline__ void nl_pair16_any(const NLArgs &a, cplx<R> *v, int c, i
     const double r1 = (double)v1.x * (double)v1.x + (double)v1.y * (double)v1.y;
     const double t0 = __shfl_xor_sync(0xffffffffu, r1, mask), t1 = __shfl_xor_sync(0xffffffffu, r0, mask);
     const double g_oo = a.gs[c * (MAXC + 1)], g_ot = a.gs[c ? MAXC : 1];
-    v[m] = from_d<R>(cmul(to_d<R>(v0), expi<R>((w0 + (g_oo * r0 + g_ot * t0 + off)) * a.mdt)));
-    v[m + 8] = from_d<R>(cmul(to_d<R>(v1), expi<R>((w1 + (g_oo * r1 + g_ot * t1 + off)) * a.mdt)));
+    v[m] = from_d<R>(cmul(to_d<R>(v0), expi_f<R>((w0 + (g_oo * r0 + g_ot * t0 + off)) * a.mdt)));
+    v[m + 8] = from_d<R>(cmul(to_d<R>(v1), expi_f<R>((w1 + (g_oo * r1 + g_ot * t1 + off)) * a.mdt)));
   }
 }
 
@@ -799,6 +900,33 @@ template <typename R, bool BRAGG>
 __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, int mask, bool live, double x0, double om,
                                           double ec, double es, int64_t l0, int dl) {
   using C = cplx<R>;
+  if constexpr (BRAGG && sizeof(R) == 8) {
+    if (!a.stable) {
+      // the reference's form, bound by its FP64 operations (a square root, a
+      // division, two phases): two points at a time from v[0], v[1] and their
+      // partners, then the registers move up by two.  z pass of 256^3: two at
+      // a time 336 us, one 347, four 370 (spills).
+      #pragma unroll 1
+      for (int it = 0; it < 4; it++) {
+        #pragma unroll
+        for (int u = 0; u < 2; u++) {
+          C own = v[u], oth = shfl_xor_c(v[8 + u], mask);
+          bragg_pair_at<R>(a, 0, c, x0, om, ec, es, own, oth);
+          v[u] = own;
+          v[8 + u] = shfl_xor_c(oth, mask);
+        }
+        #pragma unroll
+        for (int h = 0; h < 16; h += 8) {
+          const C v0 = v[h], v1 = v[h + 1];
+          #pragma unroll
+          for (int m = 0; m < 6; m++) v[h + m] = v[h + m + 2];
+          v[h + 6] = v0;
+          v[h + 7] = v1;
+        }
+      }
+      return;
+    }
+  }
   // The series serve every point of the warp if they do for the largest
   // potential that its points allow: |V| <= G rho + |off| + max |V_c|, with
   // rho <= 2 max(|re|, |im|)^2 over the pencil and G the larger row sum of |g|.
@@ -814,8 +942,7 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
   bool small = false;
   if constexpr (BRAGG) {
     const double V = Vrho + fmax(fabs(bx), fabs(bd)), O2 = om * om;
-    small = fabs(a.dt) * V <= 0.03125 && (a.dt * a.dt) * (V * V + O2) <= 0x1p-10 &&
-            (sizeof(R) == 4 || a.stable || O2 >= 0x1p-23 * (V * V));
+    small = fabs(a.dt) * V <= 0.03125 && (a.dt * a.dt) * (V * V + O2) <= 0x1p-10;
   } else if (a.kind != K_NUM_BRAGG) {
     int h = 0;
     if (Vp) {
@@ -875,7 +1002,7 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
 // 2048^2 60 -> 53.
 template <typename R> __device__ __noinline__ void phase8_any(cplx<R> *v, const double *ph) {
   #pragma unroll 2
-  for (int m = 0; m < 8; m++) v[m] = from_d<R>(cmul(to_d<R>(v[m]), expi<R>(ph[m])));
+  for (int m = 0; m < 8; m++) v[m] = from_d<R>(cmul(to_d<R>(v[m]), expi_f<R>(ph[m])));
 }
 template <typename R, bool XP>
 __device__ __forceinline__ void nl_single16(const NLArgs &a, cplx<R> *v, bool live, double x0, double dx, int64_t l0,
@@ -924,28 +1051,21 @@ __device__ __forceinline__ void nl_single16(const NLArgs &a, cplx<R> *v, bool li
 // CRT_Base_IF.h:392-418, bragg.cpp:210-302).  Mixed: FP64 phase arguments,
 // FP32 field arithmetic, and the eigenvalue-free form of the 2x2 exponential.
 // TC: the number of components the calling kernel holds (ncomp <= TC); step
-// kinds that need more components are compiled out.  cp: the
-// pencil's couplings where the caller has them (coupling_x).
-template <typename R, int TC = MAXC>
+// kinds that need more components are compiled out.  CP: the caller has the
+// pencil's couplings of three- and four-component steps (coupling_x).  FAR: as
+// in bragg_pair_far.
+template <typename R, int TC = MAXC, bool CP = false, bool FAR = false>
 __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l, double x0, double Omega,
                                          double eta_c, double eta_s, const double *cp = nullptr) {
-  // couplings of the pencil, where the caller has not evaluated them
-  double own[NCPL];
-  if constexpr (TC >= 2) {
-    if (!cp && a.kind != K_BRAGG) {
-      coupling_x(a, x0, own);
-      cp = own;
-    }
-  }
   if constexpr (TC >= 3) {
     if (a.kind == K_DBRAGG) {
-      dbragg_point<R>(a, v, l, x0, cp);
+      dbragg_point<R, CP>(a, v, l, x0, cp);
       return;
     }
   }
   if constexpr (TC >= 4) {
     if (a.kind == K_BRAGG_DS) {
-      bragg_ds_point<R>(a, v, x0, cp);
+      bragg_ds_point<R, CP>(a, v, x0, cp);
       return;
     }
   }
@@ -957,7 +1077,7 @@ __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l,
       cplx<R> w[TC];
       #pragma unroll
       for (int c = 0; c < TC; c++) w[c] = v[c];
-      num_point<R, TC>(a, w, l, x0, cp);
+      num_point<R, TC, CP>(a, w, l, x0, cp);
       #pragma unroll
       for (int c = 0; c < TC; c++) v[c] = w[c];
       return;
@@ -997,7 +1117,8 @@ __device__ __forceinline__ void nl_point(const NLArgs &a, cplx<R> *v, int64_t l,
     // Bragg 2x2 (components 0 and 1)
     const double V11 = a.gs[0] * rho[0] + a.gs[1] * rho[1] + a.L.beta0 * x0;
     const double V22 = a.gs[MAXC] * rho[0] + a.gs[MAXC + 1] * rho[1] - a.L.DeltaL[1] + a.L.beta0 * x0;
-    bragg_pair<R>(a.stable, a.dt, V11, V22, Omega, eta_c, eta_s, v[0], v[1]);
+    if constexpr (FAR) bragg_pair_far<R>(a.stable, a.dt, V11, V22, Omega, eta_c, eta_s, v[0], v[1]);
+    else bragg_pair<R>(a.stable, a.dt, V11, V22, Omega, eta_c, eta_s, v[0], v[1]);
   }
 }
 
@@ -1188,7 +1309,7 @@ __global__ void __launch_bounds__(Tile<R>::NT, Tile<R>::MINB) pass_kernel(PassAr
           double phi = 0;
           #pragma unroll
           for (int ax = 0; ax < 3; ax++) {
-            const int t = (ijk[ax] + a.n[ax] / 2) & (a.n[ax] - 1);
+            const int t = (ijk[ax] + a.n[ax] / 2) % a.n[ax];
             const double k = a.dk[ax] * (double)(t - a.n[ax] / 2);
             phi += (k * a.filt_alpha) * k;
           }

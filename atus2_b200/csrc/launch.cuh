@@ -455,7 +455,7 @@ static inline int launch_pass2_n(atus_ctx *ctx, PassArgs &a, int axis) {
       case 2048: return launch_pass3_t<R, 2048, TC, MODE, STRIDED>(ctx, a, axis);
       default: break;
     }
-    if constexpr (TC <= 2) {
+    if constexpr (TC <= 2 && MODE != M2_NL_MEET) {
       if (ctx->n[axis] == 4096) return launch_pass3_t<R, 4096, TC, MODE, STRIDED>(ctx, a, axis);
     }
   }

@@ -269,7 +269,6 @@ __device__ __forceinline__ void line_run(const LineInst &in, const NLArgs &nl, c
       sincos(nl.L.laser_k0 * x0, &kx[m].y, &kx[m].x);
       eta[m] = make_double2(1.0, 0.0);
       if (nl.L.laser_dk0 != 0.0) sincos(-0.5 * (nl.L.laser_dk0 * x0), &eta[m].y, &eta[m].x);
-      if (c) eta[m].y = -eta[m].y;
     }
   } else {
     const double *const Vp = nl.kind == K_NL ? (TC == 2 && c ? nl.V[1] : nl.V[0]) : nullptr;
@@ -370,15 +369,11 @@ __device__ __forceinline__ void line_run(const LineInst &in, const NLArgs &nl, c
     if constexpr (BRAGG) {
       {
         const double2 a = s_th[j % LINE_CHUNK];
-        const double g_to = c ? nl.gs[1] : nl.gs[MAXC], g_tt = c ? nl.gs[0] : nl.gs[MAXC + 1];
         #pragma unroll
         for (int m = 0; m < 4; m++) {
           V own = v[m], oth = shfl_xor_c(v[m + 4], 1);
-          const double bx = nl.L.beta0 * ((double)(p + P * (m ^ sw) - nl.shift0) * nl.dx0), bd = bx - nl.L.DeltaL[1];
-          const double ro = (double)own.x * (double)own.x + (double)own.y * (double)own.y;
-          const double rt = (double)oth.x * (double)oth.x + (double)oth.y * (double)oth.y;
-          bragg_pair<R>(nl.stable, dt, g_oo * ro + g_ot * rt + (c ? bd : bx), g_to * ro + g_tt * rt + (c ? bx : bd),
-                        kx[m].x * a.x - kx[m].y * a.y, eta[m].x, eta[m].y, own, oth, c != 0);
+          bragg_pair_at<R>(nl, nl.stable, c, (double)(p + P * (m ^ sw) - nl.shift0) * nl.dx0,
+                           kx[m].x * a.x - kx[m].y * a.y, eta[m].x, eta[m].y, own, oth);
           v[m] = own;
           v[m + 4] = shfl_xor_c(oth, 1);
         }
@@ -391,10 +386,10 @@ __device__ __forceinline__ void line_run(const LineInst &in, const NLArgs &nl, c
           const double a1 = (double)v[r + 4].x * (double)v[r + 4].x + (double)v[r + 4].y * (double)v[r + 4].y;
           const double f0 = g_oo * a0 + g_ot * __shfl_xor_sync(0xffffffffu, a1, 1);
           const double f1 = g_oo * a1 + g_ot * __shfl_xor_sync(0xffffffffu, a0, 1);
-          v[r] = from_d<R>(cmul(to_d<R>(v[r]), cmul(es[r], expi<double>(f0 * nl.mdt))));
-          v[r + 4] = from_d<R>(cmul(to_d<R>(v[r + 4]), cmul(es[r + 4], expi<double>(f1 * nl.mdt))));
+          v[r] = from_d<R>(cmul(to_d<R>(v[r]), cmul(es[r], expi_f<double>(f0 * nl.mdt))));
+          v[r + 4] = from_d<R>(cmul(to_d<R>(v[r + 4]), cmul(es[r + 4], expi_f<double>(f1 * nl.mdt))));
         } else {
-          v[r] = from_d<R>(cmul(to_d<R>(v[r]), cmul(es[r], expi<double>(g_oo * a0 * nl.mdt))));
+          v[r] = from_d<R>(cmul(to_d<R>(v[r]), cmul(es[r], expi_f<double>(g_oo * a0 * nl.mdt))));
         }
       }
     }

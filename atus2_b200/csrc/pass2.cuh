@@ -37,7 +37,7 @@ template <> struct Tile2<float> { static constexpr int E = 4096, NT = 256, MINB 
 template <typename R, int MODE, int TC = 1>
 constexpr int p2_minb =
     TC >= 3 ? (TC == 3 ? 3 : sizeof(R) == 8 ? 4 : 2) :
-    (((MODE >= M2_FWD_SOB && MODE != M2_FILT) || MODE == M2_NL) && sizeof(R) == 8) ? 4 : Tile2<R>::MINB;
+    (((MODE >= M2_FWD_SOB && MODE < M2_FILT) || MODE == M2_NL) && sizeof(R) == 8) ? 4 : Tile2<R>::MINB;
 
 // Passes whose two components meet inside a warp (the batched passes; a
 // single grid's run in pass2_pair.cuh).
@@ -268,8 +268,8 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
         coupling_x(a.nl, (double)(ix - a.nl.shift0) * a.nl.dx0, s_om + NCPL * p);
       }
   }
-  if constexpr (MODE == M2_NL && TC == 2 && !PAIR) {
-    if (a.nl.kind == K_BRAGG && a.axis != 0)
+  if constexpr (MODE == M2_NL_MEET) {
+    if (a.nl.kind == K_BRAGG)
     for (int p = tid; p < B; p += NT) {
       double om = 0, ec = 1, es = 0;
       if (p < g.nb) {
@@ -453,7 +453,7 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
       }
     }
     p2_transform<R, N, +1, !STRIDED>(v, my, twS, j);
-  } else {  // M2_NL, M2_FS_NL: IFFT -> potential step -> FFT
+  } else {  // M2_NL, M2_NL_MEET, M2_FS_NL: IFFT -> potential step -> FFT
     constexpr bool FS = (MODE == M2_FS_NL);  // axis 0 is the whole grid index
     const int sg = (PAIR && c) ? (int)0x80000000 : 0;
     p2_transform<R, N, +1, !STRIDED, PAIR ? 2 : 0>(v, my, twS, j, sg);
@@ -495,14 +495,14 @@ __device__ __forceinline__ void p2_item(const PassArgs &a, const TileGeo &g, uns
           const double x0 = (double)((FS ? (int)l : ix) - a.nl.shift0) * a.nl.dx0;
           double om = 0, ec = 1, es = 0;
           if (bragg) {
-            if (a.axis == 0) bragg_coupling(a.nl, x0, om, ec, es);
+            if constexpr (FS) bragg_coupling(a.nl, x0, om, ec, es);
             else { om = s_om[pb]; ec = s_ec[pb]; es = s_es[pb]; }
           }
           const double *const cp = (MODE == M2_NL && TC > 2) ? s_om + NCPL * pb : nullptr;
           C u[MAXC];
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) u[cc] = ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)];
-          nl_point<R, TC>(a.nl, u, l, x0, om, ec, es, cp);
+          nl_point<R, TC, (MODE == M2_NL && TC > 2), MODE != M2_NL_MEET>(a.nl, u, l, x0, om, ec, es, cp);
           #pragma unroll
           for (int cc = 0; cc < TC; cc++) ex[(cc * B + pb) * PB + ex_at(i >> 4, i & 15)] = u[cc];
         }

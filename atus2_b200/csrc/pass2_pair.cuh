@@ -15,9 +15,10 @@
 // item is transformed.  To make room for them FP64 values cross the exchange
 // as real parts, then imaginary parts, in half the space.  16 warps per SM at
 // 128 registers.  z pass of 256^3, two components, against the CTA-wide form
-// with the components meeting in shared memory: bragg_ad FP64 0.337 -> 0.266
-// ms, complex64 0.279 -> 0.238; freeprop (NL_IF) FP64 0.321 -> 0.228, complex64
-// 0.252 -> 0.223.  Shuffles alone, loads not ahead: 0.349-0.361 (FP64).  The
+// with the components meeting in shared memory: bragg_ad FP64 0.368 -> 0.336
+// ms (eigenvalue form; eigenvalue-free 0.337 -> 0.266), complex64 0.279 ->
+// 0.227; freeprop (NL_IF) FP64 0.321 -> 0.219, complex64 0.252 -> 0.217.
+// Shuffles alone, loads not ahead: 0.349-0.361 (FP64, eigenvalue-free).  The
 // Bragg step and the pure phases are two instantiations: in one, the Bragg
 // step lost 0.026 ms to spills.
 #pragma once

@@ -180,7 +180,12 @@ ATUS_API int atus_set_pulse_windows(atus_ctx *ctx, double t_start, const double 
  * do).  No counterpart in the reference: its eigen-form (bragg.cpp:254-277)
  * divides by (V11 - E)^2 + Omega^2, loses unitarity once |Omega| is below the
  * spacing of V11 and divides by zero once Omega^2 underflows -- the tails of a
- * Gaussian pulse reach both.  Default 0: the reference's form, bit for bit. */
+ * Gaussian pulse reach both.  Default 0: the reference's form (its two
+ * divisions from one, products fused as the compiler does), error about
+ * 2^-53 |V| / |Omega| a step.  On small dense grids, where g |psi|^2 dt is 0.5
+ * and more, the nonlinear step multiplies a rounding difference by up to 10^15
+ * over some hundred steps: there the two forms, or two grids' worth of
+ * otherwise equal programs, end in different states. */
 ATUS_API int atus_set_bragg_stable(atus_ctx *ctx, int on);
 
 /* No counterpart in the reference.  Bounded waits of the TMA-fed strided
