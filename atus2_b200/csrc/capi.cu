@@ -1149,7 +1149,11 @@ static int resident_block(atus_ctx *ctx, int nk, int kind, const double *F) {
       CK(cudaMalloc(&ctx->blk_F, sizeof(double) * nk));
       ctx->blk_F_n = nk;
     }
-    CK(cudaMemcpyAsync(ctx->blk_F, F, sizeof(double) * nk, cudaMemcpyHostToDevice, ctx->stream));
+    // F is the caller's for the duration of the call only.  A copy from
+    // pageable memory has taken it by the time it returns; from page-locked
+    // memory it would read it when the stream gets there.
+    const std::vector<double> own(F, F + nk);
+    CK(cudaMemcpyAsync(ctx->blk_F, own.data(), sizeof(double) * nk, cudaMemcpyHostToDevice, ctx->stream));
   }
   if (line) {
     LineArgs a;
