@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -80,6 +81,7 @@ struct atus_batch {
   double2 *unit = nullptr;         // factor (1, 0) of the absent third axis
   double2 *stage = nullptr;        // complex128 copy of a complex64 field on its way out
   int64_t stage_n = 0;
+  std::mutex reading;              // one download at a time uses stage
   std::vector<Class> cls;
   cudaStream_t st = nullptr;
   std::vector<cudaStream_t> side;   // one per 1D class (concurrent persistent kernels)
@@ -537,6 +539,7 @@ int atus_batch_upload_psi(atus_batch *b, int i, int comp, const double *psi) {
 int atus_batch_download_psi(atus_batch *b, int i, int comp, double *psi) {
   if (!b || !psi || i < 0 || i >= (int)b->inst.size() || comp < 0 || comp > 1) return ATUS_E_ARG;
   const int64_t np = npts(b->inst[i]);
+  const std::lock_guard<std::mutex> one(b->reading);  // readers in several threads share stage
   const void *src = b->psi[comp][i];
   if (b->prec != ATUS_PREC_FP64) {
     // widened on the device into a buffer kept for the batch (the largest
