@@ -204,7 +204,7 @@ int build_2d_args(atus_batch *b, Class &c) {
     std::vector<PassArgs> h(m);
     for (int q = 0; q < m; q++) h[q] = pass_of(b, c.ids[q], p, k.B);
     if (!c.d_args[p]) BCK(cudaMalloc(&c.d_args[p], sizeof(PassArgs) * m));
-    BCK(cudaMemcpy(c.d_args[p], h.data(), sizeof(PassArgs) * m, cudaMemcpyHostToDevice));
+    BCK(cudaMemcpyAsync(c.d_args[p], h.data(), sizeof(PassArgs) * m, cudaMemcpyHostToDevice, b->st));
     c.items[p] = h[0].ntiles * (h[0].per_comp ? 2 : 1);
   }
   return ATUS_OK;
@@ -345,6 +345,10 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
       cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&b->e0) != cudaSuccess || cudaEventCreate(&b->e1) != cudaSuccess)
     return bail(ATUS_E_CUDA);
+  // Copies and fills run on the batch's stream here and below.  The default
+  // stream does not block it, a copy from pageable memory returns while its
+  // last part is on its way, and one between device buffers returns at once:
+  // kernels of the batch could overtake them there.
   // twiddles exp(-2 pi i m / TWN): double2, or float4 (hi, lo) for complex64
   {
     const long double two_pi = 6.283185307179586476925286766559005768L;
@@ -360,7 +364,7 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     }
     if (precision == ATUS_PREC_FP64) {
       if (cudaMalloc(&b->tw, 16 * TWN) != cudaSuccess) return bail(ATUS_E_NOMEM);
-      cudaMemcpy(b->tw, t64.data(), 16 * TWN, cudaMemcpyHostToDevice);
+      cudaMemcpyAsync(b->tw, t64.data(), 16 * TWN, cudaMemcpyHostToDevice, b->st);
     } else {
       std::vector<float4> t4(TWN);
       for (int m = 0; m < TWN; m++) {
@@ -370,7 +374,7 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
         t4[m].w = (float)(t64[m].y - (double)t4[m].y);
       }
       if (cudaMalloc(&b->tw, sizeof(float4) * TWN) != cudaSuccess) return bail(ATUS_E_NOMEM);
-      cudaMemcpy(b->tw, t4.data(), sizeof(float4) * TWN, cudaMemcpyHostToDevice);
+      cudaMemcpyAsync(b->tw, t4.data(), sizeof(float4) * TWN, cudaMemcpyHostToDevice, b->st);
     }
   }
   // fields and kinetic factors (the reference's double arithmetic,
@@ -385,7 +389,7 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     const int64_t np = npts(in);
     for (int c = 0; c < 2; c++) {
       if (cudaMalloc(&b->psi[c][i], csize(b) * np) != cudaSuccess) return bail(ATUS_E_NOMEM);
-      cudaMemset(b->psi[c][i], 0, csize(b) * np);
+      cudaMemsetAsync(b->psi[c][i], 0, csize(b) * np, b->st);
     }
     for (int ax = 0; ax < in.grid.dim; ax++) {
       const int64_t n = in.grid.n[ax];
@@ -398,8 +402,8 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
       }
       if (cudaMalloc(&b->kt[0][ax][i], 16 * n) != cudaSuccess || cudaMalloc(&b->kt[1][ax][i], 16 * n) != cudaSuccess)
         return bail(ATUS_E_NOMEM);
-      cudaMemcpy(b->kt[0][ax][i], th.data(), 16 * n, cudaMemcpyHostToDevice);
-      cudaMemcpy(b->kt[1][ax][i], tf.data(), 16 * n, cudaMemcpyHostToDevice);
+      cudaMemcpyAsync(b->kt[0][ax][i], th.data(), 16 * n, cudaMemcpyHostToDevice, b->st);
+      cudaMemcpyAsync(b->kt[1][ax][i], tf.data(), 16 * n, cudaMemcpyHostToDevice, b->st);
     }
     pulse[i].tc = in.pulse_tc;
     pulse[i].two_sigma2 = in.pulse_sigma > 0 ? 2.0 * in.pulse_sigma * in.pulse_sigma : 0.0;
@@ -418,15 +422,15 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
   {
     const double2 one = make_double2(1.0, 0.0);
     if (cudaMalloc(&b->unit, sizeof(double2)) != cudaSuccess) return bail(ATUS_E_NOMEM);
-    cudaMemcpy(b->unit, &one, sizeof(double2), cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(b->unit, &one, sizeof(double2), cudaMemcpyHostToDevice, b->st);
   }
   if (cudaMalloc(&b->d_b1, sizeof(LineInst) * count) != cudaSuccess ||
       cudaMalloc(&b->d_pulse, sizeof(Pulse) * count) != cudaSuccess ||
       cudaMalloc(&b->d_t0, sizeof(double) * count) != cudaSuccess ||
       cudaMallocHost(&b->h_t0, sizeof(double) * count) != cudaSuccess)
     return bail(ATUS_E_NOMEM);
-  cudaMemcpy(b->d_b1, b1.data(), sizeof(LineInst) * count, cudaMemcpyHostToDevice);
-  cudaMemcpy(b->d_pulse, pulse.data(), sizeof(Pulse) * count, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(b->d_b1, b1.data(), sizeof(LineInst) * count, cudaMemcpyHostToDevice, b->st);
+  cudaMemcpyAsync(b->d_pulse, pulse.data(), sizeof(Pulse) * count, cudaMemcpyHostToDevice, b->st);
   // size classes, instances longest run first (equal here) in batch order
   std::map<std::pair<int, int>, int> key;
   for (int i = 0; i < count; i++) {
@@ -442,7 +446,7 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
   }
   for (Class &c : b->cls) {
     if (cudaMalloc(&c.d_ids, sizeof(int) * c.ids.size()) != cudaSuccess) return bail(ATUS_E_NOMEM);
-    cudaMemcpy(c.d_ids, c.ids.data(), sizeof(int) * c.ids.size(), cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(c.d_ids, c.ids.data(), sizeof(int) * c.ids.size(), cudaMemcpyHostToDevice, b->st);
     BKernel k;
     if (c.dim == 1) {
       for (int ctas : {1, 2, 4, 8}) {
@@ -525,14 +529,15 @@ const char *atus_batch_last_error(const atus_batch *b) { return b ? b->err.c_str
 int atus_batch_upload_psi(atus_batch *b, int i, int comp, const double *psi) {
   if (!b || !psi || i < 0 || i >= (int)b->inst.size() || comp < 0 || comp > 1) return ATUS_E_ARG;
   const int64_t np = npts(b->inst[i]);
-  BCK(cudaStreamSynchronize(b->st));
+  std::vector<float2> f;
   if (b->prec == ATUS_PREC_FP64) {
-    BCK(cudaMemcpy(b->psi[comp][i], psi, 16 * np, cudaMemcpyHostToDevice));
+    BCK(cudaMemcpyAsync(b->psi[comp][i], psi, 16 * np, cudaMemcpyHostToDevice, b->st));
   } else {
-    std::vector<float2> f(np);
+    f.resize(np);
     for (int64_t l = 0; l < np; l++) f[l] = make_float2((float)psi[2 * l], (float)psi[2 * l + 1]);
-    BCK(cudaMemcpy(b->psi[comp][i], f.data(), 8 * np, cudaMemcpyHostToDevice));
+    BCK(cudaMemcpyAsync(b->psi[comp][i], f.data(), 8 * np, cudaMemcpyHostToDevice, b->st));
   }
+  BCK(cudaStreamSynchronize(b->st));  // psi is the caller's again
   return ATUS_OK;
 }
 
@@ -574,7 +579,7 @@ int atus_batch_tune(atus_batch *b, int probe_steps) {
   if (!b || probe_steps < 1) return ATUS_E_ARG;
   BCK(cudaStreamSynchronize(b->st));
   for (int i = 0; i < (int)b->inst.size(); i++) b->h_t0[i] = b->t[i];
-  BCK(cudaMemcpy(b->d_t0, b->h_t0, sizeof(double) * b->inst.size(), cudaMemcpyHostToDevice));
+  BCK(cudaMemcpyAsync(b->d_t0, b->h_t0, sizeof(double) * b->inst.size(), cudaMemcpyHostToDevice, b->st));
   for (Class &c : b->cls) {
     // probe on the real fields, restored from a copy afterwards
     std::vector<void *> keep[2];
@@ -583,7 +588,7 @@ int atus_batch_tune(atus_batch *b, int probe_steps) {
         void *p = nullptr;
         const size_t bytes = csize(b) * npts(b->inst[i]);
         BCK(cudaMalloc(&p, bytes));
-        BCK(cudaMemcpy(p, b->psi[comp][i], bytes, cudaMemcpyDeviceToDevice));
+        BCK(cudaMemcpyAsync(p, b->psi[comp][i], bytes, cudaMemcpyDeviceToDevice, b->st));
         keep[comp].push_back(p);
       }
     c.cand_ms.assign(c.cands.size(), -1.0);
@@ -607,9 +612,10 @@ int atus_batch_tune(atus_batch *b, int probe_steps) {
       if (best < 0 || ms < c.cand_ms[best]) best = (int)q;
       for (int comp = 0; comp < 2; comp++)
         for (size_t m = 0; m < c.ids.size(); m++)
-          BCK(cudaMemcpy(b->psi[comp][c.ids[m]], keep[comp][m], csize(b) * npts(b->inst[c.ids[m]]),
-                         cudaMemcpyDeviceToDevice));
+          BCK(cudaMemcpyAsync(b->psi[comp][c.ids[m]], keep[comp][m], csize(b) * npts(b->inst[c.ids[m]]),
+                              cudaMemcpyDeviceToDevice, b->st));
     }
+    BCK(cudaStreamSynchronize(b->st));  // the fields are back before their copies go
     for (int comp = 0; comp < 2; comp++)
       for (void *p : keep[comp]) cudaFree(p);
     c.v = c.cands[best];
