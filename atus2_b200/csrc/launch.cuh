@@ -139,7 +139,7 @@ template <typename R, int N, int TC, bool BRAGG>
 static inline int launch_line_c(atus_ctx *ctx, const LineArgs &a) {
   int r = ATUS_E_UNSUPPORTED;
   constexpr int C = line_ctas<R, N, TC>;
-  if (ctx->use_cluster1d) r = launch_line_t<R, N, TC, C, BRAGG>(ctx, a);
+  if (C == 1 || ctx->use_cluster1d) r = launch_line_t<R, N, TC, C, BRAGG>(ctx, a);
   if constexpr (C > 1) {
     if (r == ATUS_E_UNSUPPORTED) r = launch_line_t<R, N, TC, 1, BRAGG>(ctx, a);
   }
