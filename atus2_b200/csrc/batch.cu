@@ -26,6 +26,8 @@ using namespace atus;
 
 bool batch1d_info_f(int N, int C, BKernel *k);
 bool batch1d_info_d(int N, int C, BKernel *k);
+bool batch1d_cta_info_f(int N, BKernel *k);
+bool batch1d_cta_info_d(int N, BKernel *k);
 bool batch2d_p2_info_f(int N, int mode, BKernel *k);
 bool batch2d_p2_info_d(int N, int mode, BKernel *k);
 bool batch2d_tile_info_f(int N, int mode, BKernel *k);
@@ -37,7 +39,7 @@ namespace {
 enum { P_FWD = 0, P_INV = 1, P_KH = 2, P_KF = 3, P_POT = 4, NPASS = 5 };
 
 struct Variant {
-  int a = 0;  // 1D: CTAs an instance runs on; 2D: BV_P2 / BV_P5 / BV_TILE
+  int a = 0;  // 1D: CTAs an instance runs on (0: batch1d_cta_kernel); 2D: BV_P2 / BV_P5 / BV_TILE
 };
 
 struct Class {
@@ -111,6 +113,7 @@ int64_t npts(const atus_batch_instance &in) {
 }
 
 bool info1d(const atus_batch *b, int N, const Variant &v, BKernel *k) {
+  if (v.a == 0) return b->prec == ATUS_PREC_FP64 ? batch1d_cta_info_d(N, k) : batch1d_cta_info_f(N, k);
   return b->prec == ATUS_PREC_FP64 ? batch1d_info_d(N, v.a, k) : batch1d_info_f(N, v.a, k);
 }
 bool info2d(const atus_batch *b, int N, int variant, int mode, BKernel *k) {
@@ -234,7 +237,10 @@ int prepare(atus_batch *b, const BKernel &k) {
   if (k.cluster > 1) {  // clusters the device holds at once
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = cluster_config(k, k.cluster, nullptr, &attr);
-    BCK(cudaOccupancyMaxActiveClusters(&res, k.fn, &cfg));
+    if (cudaOccupancyMaxActiveClusters(&res, k.fn, &cfg) != cudaSuccess) {
+      res = 0;
+      cudaGetLastError();  // a refused query: none placeable, and no sticky error
+    }
   } else {
     BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, k.fn, k.nt, k.smem));
   }
@@ -306,7 +312,8 @@ void drop_graphs(atus_batch *b) {
 
 std::string variant_name(const Class &c, const Variant &v) {
   char buf[64];
-  if (c.dim == 1) snprintf(buf, sizeof(buf), "%d CTA%s per instance", v.a, v.a > 1 ? "s" : "");
+  if (c.dim == 1 && v.a == 0) snprintf(buf, sizeof(buf), "1 CTA per instance, one component in L2");
+  else if (c.dim == 1) snprintf(buf, sizeof(buf), "%d CTA%s per instance", v.a, v.a > 1 ? "s" : "");
   else snprintf(buf, sizeof(buf), "%s", v.a == BV_P2 ? "register-staged passes" : v.a == BV_P5 ? "register-staged 512-point passes" : "shared-memory tile passes");
   return buf;
 }
@@ -449,13 +456,17 @@ int atus_batch_create(const atus_batch_instance *inst, int count, int precision,
     cudaMemcpyAsync(c.d_ids, c.ids.data(), sizeof(int) * c.ids.size(), cudaMemcpyHostToDevice, b->st);
     BKernel k;
     if (c.dim == 1) {
-      for (int ctas : {1, 2, 4, 8}) {
+      // the last (0 CTAs) where no other is to be had: a length that only a
+      // cluster holds on chip, and none placeable or wanted
+      const char *c1 = getenv("ATUS_CLUSTER1D");
+      const bool clusters = !(c1 && c1[0] == '0');
+      for (int ctas : {1, 2, 4, 8, 0}) {
         Variant v;
         v.a = ctas;
-        if (!info1d(b, c.n, v, &k)) continue;
+        if ((ctas > 1 && !clusters) || (ctas == 0 && !c.cands.empty()) || !info1d(b, c.n, v, &k)) continue;
         const int r = prepare(b, k);
         if (r == ATUS_OK) c.cands.push_back(v);
-        else if (ctas == 1 || b->err.find("does not fit") == std::string::npos) return bail(ATUS_E_CUDA);
+        else if (r != ATUS_E_UNSUPPORTED) return bail(r);
       }
     } else {
       for (int var : {BV_P2, BV_P5, BV_TILE}) {

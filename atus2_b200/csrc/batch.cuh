@@ -39,6 +39,92 @@ __device__ __forceinline__ void coupling_at(const NLArgs &a, double x0, double &
   else bragg_coupling_mixed(a, x0, om, ec, es);
 }
 
+// ------------------------------------------------------------------ 1D without a cluster
+// The runs of line1d_batch_kernel on one CTA each, for lengths whose two
+// components one CTA does not hold as line1d.cuh lays them out, where no
+// cluster is to be had (ATUS_CLUSTER1D=0, or a device that places none).  One
+// component (index rc) is in shared memory, the other in global memory (L2);
+// they change places around each kinetic step.
+constexpr int BCTA_NT = 512;
+
+template <typename R, int N>
+__device__ __forceinline__ void bcta_kinetic(cplx<R> *s, const typename TwTab<R>::type *tw, const double2 *K, double s_f,
+                                             double s_b) {
+  fft_tile<R, N, 1, BCTA_NT, -1, TWN>(s, tw);
+  for (int i = threadIdx.x; i < N; i += BCTA_NT) {
+    cplx<R> &v = s[Pad<N>::idx(0, i)];
+    v = kin_mul<R>(v, __ldg(&K[i]), s_f, s_b);
+  }
+  __syncthreads();
+  fft_tile<R, N, 1, BCTA_NT, +1, TWN>(s, tw);
+}
+template <typename R, int N> __device__ __forceinline__ void bcta_load(cplx<R> *s, const cplx<R> *src) {
+  for (int i = threadIdx.x; i < N; i += BCTA_NT) s[Pad<N>::idx(0, i)] = src[i];
+  __syncthreads();
+}
+template <typename R, int N> __device__ __forceinline__ void bcta_store(const cplx<R> *s, cplx<R> *dst) {
+  for (int i = threadIdx.x; i < N; i += BCTA_NT) dst[i] = s[Pad<N>::idx(0, i)];
+  __syncthreads();  // read again by other threads, and s is free
+}
+
+template <typename R, int N>
+__global__ void __launch_bounds__(BCTA_NT, 1)
+    batch1d_cta_kernel(const LineInst *__restrict__ insts, const int *__restrict__ order, const double *__restrict__ t0,
+                       int ninst, int nk, const void *twv) {
+  using C = cplx<R>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  C *const s = reinterpret_cast<C *>(smem_raw);
+  const typename TwTab<R>::type *tw = (const typename TwTab<R>::type *)twv;
+  __shared__ LineInst in;  // thread 0 sets the step's time and amplitude
+  for (int k = blockIdx.x; k < ninst; k += gridDim.x) {
+    const int id = order[k];
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&insts[id]);
+    for (int e = threadIdx.x; e < (int)(sizeof(LineInst) / 8); e += BCTA_NT)
+      reinterpret_cast<unsigned long long *>(&in)[e] = src[e];
+    __syncthreads();
+    const double dt = in.nl.dt;
+    double t = t0[id];
+    C *fld[2] = {(C *)in.psi[0], (C *)in.psi[1]};
+    // half a kinetic step of component 0, then of component 1, which stays
+    bcta_load<R, N>(s, fld[0]);
+    bcta_kinetic<R, N>(s, tw, in.kh[0], in.s_f, in.s_b);
+    bcta_store<R, N>(s, fld[0]);
+    bcta_load<R, N>(s, fld[1]);
+    bcta_kinetic<R, N>(s, tw, in.kh[1], in.s_f, in.s_b);
+    int rc = 1;
+    t += 0.5 * dt;
+    for (int j = 0; j < nk; j++) {
+      if (threadIdx.x == 0) {
+        in.nl.t1 = t + 0.5 * dt;
+        in.nl.F = pulse_at(in.pulse, in.nl.t1);
+      }
+      __syncthreads();
+      C *const other = rc ? fld[0] : fld[1];
+      for (int i = threadIdx.x; i < N; i += BCTA_NT) {
+        const double x0 = (double)(i - in.nl.shift0) * in.nl.dx0;
+        double om, ec, es;
+        bragg_coupling(in.nl, x0, om, ec, es);
+        const C res = s[Pad<N>::idx(0, i)], oth = other[i];
+        C v[MAXC];
+        v[0] = rc ? oth : res;
+        v[1] = rc ? res : oth;
+        nl_point<R, 2, false, true>(in.nl, v, i, x0, om, ec, es);
+        s[Pad<N>::idx(0, i)] = rc ? v[1] : v[0];
+        other[i] = rc ? v[0] : v[1];
+      }
+      __syncthreads();
+      const bool last = (j == nk - 1);
+      bcta_kinetic<R, N>(s, tw, last ? in.kh[rc] : in.kf[rc], in.s_f, in.s_b);
+      bcta_store<R, N>(s, rc ? fld[1] : fld[0]);
+      rc ^= 1;
+      bcta_load<R, N>(s, rc ? fld[1] : fld[0]);
+      bcta_kinetic<R, N>(s, tw, last ? in.kh[rc] : in.kf[rc], in.s_f, in.s_b);
+      t += last ? 0.5 * dt : dt;
+    }
+    bcta_store<R, N>(s, rc ? fld[1] : fld[0]);  // ends with a barrier: shared memory is free for the next run
+  }
+}
+
 // ------------------------------------------------------------------ 2D
 // One batched pass: per instance a complete PassArgs (this pass kind, the
 // instance's fields, tables and tile counts), the pulse and the header time

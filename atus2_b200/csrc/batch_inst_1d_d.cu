@@ -29,6 +29,26 @@ static bool k1c(int C, BKernel *k) {
   }
 }
 
+// One CTA a run, one component in shared memory (lengths without a one-CTA
+// line1d_batch_kernel).
+template <int N>
+static bool kcta(BKernel *k) {
+  k->fn = (const void *)batch1d_cta_kernel<double, N>;
+  k->cluster = 1;
+  k->nt = BCTA_NT;
+  k->smem = sizeof(cplx<double>) * Pad<N>::NP;
+  k->B = 0;
+  return true;
+}
+bool batch1d_cta_info_d(int N, BKernel *k) {
+  switch (N) {
+    case 2048: return kcta<2048>(k);
+    case 4096: return kcta<4096>(k);
+    case 8192: return kcta<8192>(k);
+    default: return false;
+  }
+}
+
 bool batch1d_info_d(int N, int C, BKernel *k) {
   switch (N) {
     case 1024: return k1c<1024>(C, k);

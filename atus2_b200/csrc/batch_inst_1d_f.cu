@@ -29,6 +29,26 @@ static bool k1c(int C, BKernel *k) {
   }
 }
 
+// One CTA a run, one component in shared memory (lengths without a one-CTA
+// line1d_batch_kernel).
+template <int N>
+static bool kcta(BKernel *k) {
+  k->fn = (const void *)batch1d_cta_kernel<float, N>;
+  k->cluster = 1;
+  k->nt = BCTA_NT;
+  k->smem = sizeof(cplx<float>) * Pad<N>::NP;
+  k->B = 0;
+  return true;
+}
+bool batch1d_cta_info_f(int N, BKernel *k) {
+  switch (N) {
+    case 4096: return kcta<4096>(k);
+    case 8192: return kcta<8192>(k);
+    case 16384: return kcta<16384>(k);
+    default: return false;
+  }
+}
+
 bool batch1d_info_f(int N, int C, BKernel *k) {
   switch (N) {
     case 1024: return k1c<1024>(C, k);
