@@ -94,8 +94,10 @@ struct NLArgs {
 // depends on has ended, prepares its tables, and waits here until that
 // kernel's writes are visible; then it lets its own successor be launched.
 // (Without the launch attribute both are no-ops.)  Nothing that a kernel
-// writes may be touched before.  Worth it where passes are short: 64^3 x 2
-// passes of 6-15 us, 10 steps: PDL_OLD -> PDL_NEW us.
+// writes may be touched before.  Worth it where passes are short and a launch
+// waits for the last CTAs of the one before: ten steps of 2^20 points 462 ->
+// 410 us, twenty of 512 x 256 x 3 603 -> 502; none on 64^3 x 2 (391 -> 393),
+// whose launches follow one another without a gap.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -879,20 +881,24 @@ __device__ __noinline__ void nl_pair16_any(const NLArgs &a, cplx<R> *v, int c, i
   }
 }
 
-// Largest |re| or |im| of v[0..16), rounded up.
+// A double above every finite one whose high word (less the sign) is at most
+// h: the next high word, or NaN, which no bound holds, for infinity and NaN.
+__device__ __forceinline__ double above(int h) { return __hiloint2double(min(h, 0x7ff00000) + 1, 0); }
+
+// Largest |re| or |im| of v[0..16), rounded up; NaN if one is not finite.
 __device__ __forceinline__ double abs_bound(const double2 *v) {
   int h = 0;
   #pragma unroll
   for (int m = 0; m < 16; m++)
     h = max(h, max(__double2hiint(v[m].x) & 0x7fffffff, __double2hiint(v[m].y) & 0x7fffffff));
-  return __hiloint2double(h + 1, 0);  // NaN and infinity stay above every bound
+  return above(h);
 }
 __device__ __forceinline__ double abs_bound(const float2 *v) {
   int h = 0;
   #pragma unroll
   for (int m = 0; m < 16; m++)
     h = max(h, max(__float_as_int(v[m].x) & 0x7fffffff, __float_as_int(v[m].y) & 0x7fffffff));
-  return (double)__int_as_float(h);
+  return h < 0x7f800000 ? (double)__int_as_float(h) : above(0x7ff00000);
 }
 
 // BRAGG: a.kind is K_BRAGG (else it is not); apart, each keeps its registers.
@@ -931,7 +937,8 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
   // potential that its points allow: |V| <= G rho + |off| + max |V_c|, with
   // rho <= 2 max(|re|, |im|)^2 over the pencil and G the larger row sum of |g|.
   const double bx = a.L.beta0 * x0, bd = bx - a.L.DeltaL[1];
-  const double m1 = abs_bound(v), mx = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, mask));
+  const double m1 = abs_bound(v), m2 = __shfl_xor_sync(0xffffffffu, m1, mask);
+  const double mx = m1 >= m2 ? m1 : m2 >= m1 ? m2 : m1 + m2;  // NaN where one is (fmax would drop it)
   const double G = fmax(fabs(a.gs[0]) + fabs(a.gs[1]), fabs(a.gs[MAXC]) + fabs(a.gs[MAXC + 1]));
   const double Vrho = 2.0 * G * (mx * mx);
   const double *const Vp = (a.kind == K_NL && live) ? (c ? a.V[1] : a.V[0]) : nullptr;
@@ -948,9 +955,8 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
     if (Vp) {
       #pragma unroll
       for (int m = 0; m < 16; m++) h = max(h, __double2hiint(__ldg(&Vp[l0 + (int64_t)dl * m])) & 0x7fffffff);
-      h++;
     }
-    small = fabs(a.dt) * (Vrho + fabs(off) + __hiloint2double(h, 0)) <= 0.03125;
+    small = fabs(a.dt) * (Vrho + fabs(off) + (Vp ? above(h) : 0.0)) <= 0.03125;
   }
   if (!__all_sync(0xffffffffu, small)) {
     C w[16];

@@ -176,8 +176,6 @@ static inline int launch_block1d_n(atus_ctx *ctx, Block1DArgs &a) {
 }
 
 // ------------------------------------------------------------ register-staged passes
-// Launch of pass2_kernel (pencils of 32..256 points); ATUS_E_UNSUPPORTED,
-// without an error message, for lengths it has no instantiation for.
 // cuTensorMapEncodeTiled from the driver (no link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -293,6 +291,8 @@ static inline int launch_pair_t(atus_ctx *ctx, PassArgs &a, int axis) {
   return ATUS_OK;
 }
 
+// Launch of pass2_kernel (pencils of 32..256 points); ATUS_E_UNSUPPORTED,
+// without an error message, for lengths it has no instantiation for.
 template <typename R, int N, int TC, int MODE, bool STRIDED>
 static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   // 256-point pencils only: on 128-point pencils (the 128^3 Sobolev
@@ -356,10 +356,6 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
   }
 }
 
-// Launch of pass3_kernel (pencils of 512..4096 points); as launch_pass2_t.
-// 4096 points where tables and exchange rows fit (one or two components): the
-// shared-memory tile kernel took 385 us for the x pass of 4096 x 2048 FP64 and
-// 602 us for the y pass of 2048 x 4096, these 157 and 129.
 // The tile of launch_pass3_t's strided FP64 passes, the next one prefetched.
 // ATUS_E_UNSUPPORTED, nothing launched, where no CTA would have a next one.
 template <int N, int MODE>
@@ -383,6 +379,11 @@ static inline int launch_pass3_pipe_t(atus_ctx *ctx, PassArgs &a) {
   return ATUS_OK;
 }
 
+// Launch of pass3_kernel (pencils of 512..4096 points); as launch_pass2_t.
+// 4096 points where tables and exchange rows fit (one or two components): the
+// shared-memory tile kernel took 385 us for the x pass of 4096 x 2048 FP64 and
+// 602 us for the y pass of 2048 x 4096, these 139 (the next tile prefetched)
+// and 129.
 template <typename R, int N, int TC, int MODE, bool STRIDED>
 static inline int launch_pass3_t(atus_ctx *ctx, PassArgs &a, int axis) {
   using Cfg = P3Cfg<R, N, TC, STRIDED>;
