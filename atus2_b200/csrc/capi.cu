@@ -466,8 +466,14 @@ static int potential_pass(atus_ctx *ctx, const NLArgs &nl) {
 }
 
 // ------------------------------------------------------------------ reductions
+static unsigned red_grid(const atus_ctx *ctx) {
+  const int64_t per = (int64_t)RED_THREADS * RED_AHEAD;
+  const int64_t want = (ctx->npts + per - 1) / per;
+  return (unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS);
+}
+
 // One launch: as many blocks as give each thread RED_AHEAD points, at most
-// four per SM; totals to dst (device memory, or host memory mapped into the
+// RED_BLOCKS; totals to dst (device memory, or host memory mapped into the
 // device, which saves the copy back).
 static int launch_reduce(atus_ctx *ctx, RedArgs &a, double *dst) {
   a.g = geo(ctx);
@@ -477,11 +483,9 @@ static int launch_reduce(atus_ctx *ctx, RedArgs &a, double *dst) {
     a.n[ax] = (int)ctx->n[ax];
     a.shift[ax] = (int)(ctx->n[ax] / 2);
   }
-  const int64_t per = (int64_t)RED_THREADS * RED_AHEAD;
-  const int64_t want = (ctx->npts + per - 1) / per;
-  const unsigned grid = (unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS);
+  const unsigned grid = red_grid(ctx);
   const bool fp64 = ctx->prec == ATUS_PREC_FP64;
-#define ATUS_RED(R, M) CK(launch_pdl(ctx, reduce_kernel<R, M>, 148, RED_BLOCKS / 148, grid, RED_THREADS, 0, a, ctx->red_partial, ctx->red_count, dst))
+#define ATUS_RED(R, M) CK(launch_pdl(ctx, reduce_kernel<R, M>, ctx->nsm, RED_PER_SM, grid, RED_THREADS, 0, a, ctx->red_partial, ctx->red_count, dst))
   switch (a.mode) {
     case RED_NORM: if (fp64) ATUS_RED(double, RED_NORM); else ATUS_RED(float, RED_NORM); break;
     case RED_POS: if (fp64) ATUS_RED(double, RED_POS); else ATUS_RED(float, RED_POS); break;
@@ -609,7 +613,11 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
     ctx->use_tma = !(tm && tm[0] == '0');
   }
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) { delete ctx; return ATUS_E_CUDA; }
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    delete ctx;
+    return ATUS_E_CUDA;
+  }
   if (cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return ATUS_E_CUDA; }
   ctx->stream = ctx->own_stream;
   bool ok = true;
@@ -1658,9 +1666,7 @@ static int sob_iterate_dev(atus_ctx *ctx) {
     RUN(launch_reduce(ctx, q, d->q[i]));
   }
   for (int i = 0; i < n; i++) {
-    const int64_t per = (int64_t)RED_THREADS * RED_AHEAD;
-    const int64_t want = (ctx->npts + per - 1) / per;
-    CK(launch_pdl(ctx, sob_step_kernel, 148, RED_BLOCKS / 148, (unsigned)(want < RED_BLOCKS ? want : RED_BLOCKS), RED_THREADS, 0,
+    CK(launch_pdl(ctx, sob_step_kernel, ctx->nsm, RED_PER_SM, red_grid(ctx), RED_THREADS, 0,
                   (double2 *)ctx->psi[i], (const double2 *)ctx->sob_grad[i], (const double2 *)ctx->sob_psi[i],
                   ctx->stepsize, d, i, n, (int)(i == n - 1), ctx->ar, ctx->npts, ctx->red_partial, ctx->red_count));
     LAUNCHED(ctx);

@@ -37,6 +37,7 @@ struct atus_ctx {
   double *h_red = nullptr;        // totals of a reduction, written by the device
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int64_t launches = 0;
+  int nsm = 0;                    // SMs of the device
   const void *prev_fn = nullptr;  // the last launch of launch_pdl
   int prev_resident = 0;
   bool use_pass2 = true;        // register-staged passes for pencils of 32..256 points

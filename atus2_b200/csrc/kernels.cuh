@@ -1559,7 +1559,8 @@ struct SobArgs {
 // tree per block, block sums in a fixed order).
 enum { RED_NORM = 0, RED_POS = 1, RED_MOM = 2, RED_RABI = 3, RED_DOT2 = 4, RED_MU = 5 };
 constexpr int RED_MAXQ = 8;
-constexpr int RED_BLOCKS = 592;  // 4 x 148 SMs
+constexpr int RED_PER_SM = 4;
+constexpr int RED_BLOCKS = RED_PER_SM * 148;  // fixed: the order of the sums does not follow the device
 constexpr int RED_ROWS = 1184;   // rows of block sums (the passes that sum run up to 8 CTAs per SM)
 constexpr int RED_THREADS = 256;
 
