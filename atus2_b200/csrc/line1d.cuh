@@ -97,18 +97,28 @@ struct LineCfg {
 };
 
 // CTAs of a single context's block: as many as shorten a step.  Measured, us a
-// step (FP64 one component with a potential / two components bragg_ad; the
-// last column the kernels these replace, one CTA up to 1024 points, 16 CTAs up
-// to 8192, four-step passes beyond):
+// step (one component with a potential / two components bragg_ad, FP64 in the
+// eigenvalue form; last column: the FP64 kernels these replace, one CTA up to
+// 1024 points, 16 CTAs up to 8192, four-step passes beyond):
 //   points      1 CTA        2            4            8          before
-//     256    1.5 / 2.0    -- / 2.4     --           --          2.8 / 4.2
-//     512    1.4 / 2.2   1.9 / 2.5    -- / 2.5     --           4.3 / 6.6
-//    1024    2.0 / 4.0   2.3 / 3.3   2.2 / 3.0    -- / 3.0      5.6 / 10.7
-//    2048    3.3 / --    2.8 / 5.3   2.5 / 4.0   2.6 / 3.4      4.9 / 6.4
-//    4096       --       4.8 / --    3.4 / 5.7   2.9 / 4.4      6.7 / 8.7
-//    8192       --          --       6.1 / --    4.3 / 7.3      9.4 / 12.5
-//   16384       --          --          --       6.9 / --      42.1 / 55.6
-// (-- : does not fit, or leaves a CTA less than a warp.)
+//   FP64
+//     256    1.6 / 2.6    -- / 3.1     --           --          2.8 / 4.2
+//     512    1.4 / 2.9   1.9 / 3.2    -- / 3.2     --           4.3 / 6.6
+//    1024    2.1 / 4.8   2.3 / 4.0   2.2 / 3.8    -- / 3.7      5.6 / 10.7
+//    2048    3.3 / --    2.8 / 6.2   2.5 / 4.8   2.5 / 4.2      4.9 / 6.4
+//    4096       --       4.9 / --    3.4 / 6.7   2.9 / 5.0      6.7 / 8.7
+//    8192       --          --       6.1 / --    4.2 / 8.2      9.4 / 12.5
+//   16384       --          --          --       6.8 / --      42.1 / 55.6
+//   complex64
+//     256    1.4 / 1.8    -- / 2.2     --           --
+//     512    1.4 / 1.9   1.8 / 2.3    -- / 2.3     --
+//    1024    1.8 / 3.2   2.1 / 2.7   2.1 / 2.6    -- / 2.6
+//    2048    3.0 / 5.8   2.5 / 4.0   2.3 / 3.0   2.3 / 2.8
+//    4096    5.5 / --    3.9 / 6.9   2.7 / 4.3   2.4 / 3.4
+//    8192       --       7.9 / --    4.9 / 8.5   3.4 / 5.1
+//   16384       --          --       8.9 / --    5.4 / 9.2
+// (-- : does not fit, or leaves a CTA less than a warp.)  The counts taken are
+// within 3 % of the fastest at every length, precision and component count.
 template <typename R, int N, int TC> constexpr int line_ctas = N <= 512 ? 1 : N == 1024 ? (TC == 1 ? 1 : 4) : 8;
 
 // dft8 with 1/sqrt 2 as hi + lo in FP64 too (FP32 always: kmul).  The constant
