@@ -169,7 +169,7 @@ static int dispatch_pass(atus_ctx *ctx, PassArgs &a, int axis, int tc) {
     } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && a.nc == 4 && !ctx->dense) {
       r = dbl ? launch_pass2_d_nl4(ctx, a, axis) : launch_pass2_f_nl4(ctx, a, axis);
     } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && tc == 2 && ctx->dense) {
-      r = launch_pass2_d_meet(ctx, a, axis);
+      r = dbl ? launch_pass2_d_meet(ctx, a, axis) : launch_pass2_f_meet(ctx, a, axis);
     } else if (a.op == OP_NL && a.t1 == T_INV && a.t2 == T_FWD && !strided && tc <= 2) {
       r = dbl ? launch_pass2_d_nl(ctx, a, axis, tc) : launch_pass2_f_nl(ctx, a, axis, tc);
     }
@@ -600,7 +600,7 @@ int atus_create(const atus_grid *grid, int ncomp, int precision, atus_ctx **out)
   else if (grid->dim == 2) { ctx->ar = ctx->d[0] * ctx->d[1]; ctx->ar_k = ctx->dk[0] * ctx->dk[1]; }
   else { ctx->ar = ctx->d[0] * ctx->d[1] * ctx->d[2]; ctx->ar_k = ctx->dk[0] * ctx->dk[1] * ctx->dk[2]; }
   ctx->t = grid->t;
-  ctx->dense = ctx->dim >= 2 && ncomp >= 2 && precision == ATUS_PREC_FP64 && ctx->npts <= 8192;
+  ctx->dense = ctx->dim >= 2 && ncomp >= 2 && ctx->npts <= 8192;
   {
     // ATUS_PASS2=0: tile kernel only (A/B comparisons of the two pass kernels)
     const char *p2 = getenv("ATUS_PASS2");

@@ -41,13 +41,13 @@ struct atus_ctx {
   const void *prev_fn = nullptr;  // the last launch of launch_pdl
   int prev_resident = 0;
   bool use_pass2 = true;        // register-staged passes for pencils of 32..256 points
-  // 2D and 3D FP64 grids of at most 8192 points with coupled components.  Boxes
+  // 2D and 3D grids of at most 8192 points with coupled components.  Boxes
   // this small hold so dense a field (dt g |psi|^2 of 0.5 and more) that a block
   // multiplies a rounding difference by up to 10^15, so their results are those
   // of one order of operations only; their potential passes, and their passes
   // over 4096 points, are the point-at-a-time ones (components meeting in
   // shared memory), which keep the order that these results have always had.
-  // From 16384 points up rounding differences stay below 1e-10 over 200 steps.
+  // From 16384 points up FP64 rounding differences stay below 1e-10 over 200 steps.
   // What it costs, us a step: two components 64 x 64 12.1 (the warp-autonomous
   // pass 12.4), three 21.0 (register-staged 15.9), four 27.3 (18.2).
   bool dense = false;

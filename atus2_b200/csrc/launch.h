@@ -49,3 +49,4 @@ int launch_pass2_f_nl3(atus_ctx *ctx, PassArgs &a, int axis);
 int launch_pass2_f_nl4(atus_ctx *ctx, PassArgs &a, int axis);
 // _meet: as _nl with two components, 32..2048 points, on dense grids (ctx.h)
 int launch_pass2_d_meet(atus_ctx *ctx, PassArgs &a, int axis);
+int launch_pass2_f_meet(atus_ctx *ctx, PassArgs &a, int axis);
