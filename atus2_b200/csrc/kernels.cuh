@@ -901,37 +901,42 @@ __device__ __forceinline__ double abs_bound(const float2 *v) {
   return h < 0x7f800000 ? (double)__int_as_float(h) : above(0x7ff00000);
 }
 
-// BRAGG: a.kind is K_BRAGG (else it is not); apart, each keeps its registers.
-template <typename R, bool BRAGG>
+// The step's form; apart, each keeps its registers (z pass of 256^3 FP64 with
+// both forms of the Bragg step in one kernel 336 us, the eigenvalue form alone
+// 309, the other 276).
+enum { PAIR_PHASE = 0, PAIR_FREE = 1, PAIR_EIGEN = 2 };  // not K_BRAGG; K_BRAGG eigenvalue-free; its eigenvalue form
+template <typename R>
+__device__ __host__ __forceinline__ int pair_form(const NLArgs &a) {
+  return a.kind != K_BRAGG ? PAIR_PHASE : (sizeof(R) == 8 && !a.stable) ? PAIR_EIGEN : PAIR_FREE;
+}
+template <typename R, int FORM>
 __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, int mask, bool live, double x0, double om,
                                           double ec, double es, int64_t l0, int dl) {
   using C = cplx<R>;
-  if constexpr (BRAGG && sizeof(R) == 8) {
-    if (!a.stable) {
-      // the reference's form, bound by its FP64 operations (a square root, a
-      // division, two phases): two points at a time from v[0], v[1] and their
-      // partners, then the registers move up by two.  z pass of 256^3: two at
-      // a time 336 us, one 347, four 370 (spills).
-      #pragma unroll 1
-      for (int it = 0; it < 4; it++) {
-        #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          C own = v[u], oth = shfl_xor_c(v[8 + u], mask);
-          bragg_pair_at<R>(a, 0, c, x0, om, ec, es, own, oth);
-          v[u] = own;
-          v[8 + u] = shfl_xor_c(oth, mask);
-        }
-        #pragma unroll
-        for (int h = 0; h < 16; h += 8) {
-          const C v0 = v[h], v1 = v[h + 1];
-          #pragma unroll
-          for (int m = 0; m < 6; m++) v[h + m] = v[h + m + 2];
-          v[h + 6] = v0;
-          v[h + 7] = v1;
-        }
+  if constexpr (FORM == PAIR_EIGEN) {
+    // the reference's form, bound by its FP64 operations (a square root, a
+    // division, two phases): two points at a time from v[0], v[1] and their
+    // partners, then the registers move up by two.  z pass of 256^3: two at a
+    // time 309 us, one 315, four 321.
+    #pragma unroll 1
+    for (int it = 0; it < 4; it++) {
+      #pragma unroll
+      for (int u = 0; u < 2; u++) {
+        C own = v[u], oth = shfl_xor_c(v[8 + u], mask);
+        bragg_pair_at<R>(a, 0, c, x0, om, ec, es, own, oth);
+        v[u] = own;
+        v[8 + u] = shfl_xor_c(oth, mask);
       }
-      return;
+      #pragma unroll
+      for (int h = 0; h < 16; h += 8) {
+        const C v0 = v[h], v1 = v[h + 1];
+        #pragma unroll
+        for (int m = 0; m < 6; m++) v[h + m] = v[h + m + 2];
+        v[h + 6] = v0;
+        v[h + 7] = v1;
+      }
     }
+    return;
   }
   // The series serve every point of the warp if they do for the largest
   // potential that its points allow: |V| <= G rho + |off| + max |V_c|, with
@@ -947,7 +952,7 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
                                       : ((a.kind == K_NL_IF2 && c) ? a.L2.beta0 : a.L.beta0) * x0 -
                                             (c ? a.L.DeltaL[1] : a.L.DeltaL[0]);
   bool small = false;
-  if constexpr (BRAGG) {
+  if constexpr (FORM == PAIR_FREE) {
     const double V = Vrho + fmax(fabs(bx), fabs(bd)), O2 = om * om;
     small = fabs(a.dt) * V <= 0.03125 && (a.dt * a.dt) * (V * V + O2) <= 0x1p-10;
   } else if (a.kind != K_NUM_BRAGG) {
@@ -967,7 +972,7 @@ __device__ __forceinline__ void nl_pair16(const NLArgs &a, cplx<R> *v, int c, in
     for (int m = 0; m < 16; m++) v[m] = w[m];
     return;
   }
-  if constexpr (!BRAGG) {  // a point needs only the partner's density
+  if constexpr (FORM == PAIR_PHASE) {  // a point needs only the partner's density
     const double s_oo = a.gs[c * (MAXC + 1)], s_ot = a.gs[c ? MAXC : 1];
     #pragma unroll
     for (int m = 0; m < 8; m++) {  // registers m and m + 8 together: their densities cross over

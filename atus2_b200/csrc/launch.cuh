@@ -263,19 +263,19 @@ static inline int launch_pass2_tma_t(atus_ctx *ctx, PassArgs &a, int axis) {
 }
 
 // IFFT -> potential step -> FFT of two components along the contiguous axis.
-template <typename R, int N, bool BRAGG>
+template <typename R, int N, int FORM>
 static inline int launch_pair_t(atus_ctx *ctx, PassArgs &a, int axis) {
   using Cfg = PairCfg<R, N>;
   static int resident = 0;
   static int nsm = 0;
   if (!resident) {
-    CK(cudaFuncSetAttribute(pass2_pair_kernel<R, N, BRAGG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
-    CK(cudaFuncSetAttribute(pass2_pair_kernel<R, N, BRAGG>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    CK(cudaFuncSetAttribute(pass2_pair_kernel<R, N, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
+    CK(cudaFuncSetAttribute(pass2_pair_kernel<R, N, FORM>, cudaFuncAttributePreferredSharedMemoryCarveout,
                             cudaSharedmemCarveoutMaxShared));
     int dev = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pass2_pair_kernel<R, N, BRAGG>, Cfg::NT, Cfg::smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pass2_pair_kernel<R, N, FORM>, Cfg::NT, Cfg::smem));
     if (resident < 1) return fail(ctx, ATUS_E_UNSUPPORTED, "pass kernel does not fit on an SM");
   }
   a.sa = 1;
@@ -285,7 +285,7 @@ static inline int launch_pair_t(atus_ctx *ctx, PassArgs &a, int axis) {
   a.tw = (sizeof(R) == 8) ? ctx->tw64 : ctx->tw;
   const int64_t ctas = (a.npencils + Cfg::PW * Cfg::WPC - 1) / (Cfg::PW * Cfg::WPC);
   const int64_t slots = (int64_t)nsm * resident;
-  CK(launch_pdl(ctx, pass2_pair_kernel<R, N, BRAGG>, nsm, resident, (unsigned)(ctas < slots ? ctas : slots), Cfg::NT,
+  CK(launch_pdl(ctx, pass2_pair_kernel<R, N, FORM>, nsm, resident, (unsigned)(ctas < slots ? ctas : slots), Cfg::NT,
                 Cfg::smem, a));
   LAUNCHED(ctx);
   return ATUS_OK;
@@ -305,7 +305,11 @@ static inline int launch_pass2_t(atus_ctx *ctx, PassArgs &a, int axis) {
     }
   }
   if constexpr (MODE == M2_NL && TC == 2 && !STRIDED) {
-    return a.nl.kind == K_BRAGG ? launch_pair_t<R, N, true>(ctx, a, axis) : launch_pair_t<R, N, false>(ctx, a, axis);
+    const int form = pair_form<R>(a.nl);
+    if constexpr (sizeof(R) == 8) {
+      if (form == PAIR_EIGEN) return launch_pair_t<R, N, PAIR_EIGEN>(ctx, a, axis);
+    }
+    return form == PAIR_FREE ? launch_pair_t<R, N, PAIR_FREE>(ctx, a, axis) : launch_pair_t<R, N, PAIR_PHASE>(ctx, a, axis);
   } else {
   using Cfg = P2Cfg<R, N, TC>;
   constexpr size_t smem = ((MODE == M2_KIN || MODE == M2_KIN_RABI) && Cfg::kin_smem) ? Cfg::smem_kin : Cfg::smem;

@@ -15,12 +15,12 @@
 // item is transformed.  To make room for them FP64 values cross the exchange
 // as real parts, then imaginary parts, in half the space.  16 warps per SM at
 // 128 registers.  z pass of 256^3, two components, against the CTA-wide form
-// with the components meeting in shared memory: bragg_ad FP64 0.368 -> 0.336
-// ms (eigenvalue form; eigenvalue-free 0.337 -> 0.266), complex64 0.279 ->
+// with the components meeting in shared memory: bragg_ad FP64 0.368 -> 0.309
+// ms (eigenvalue form; eigenvalue-free 0.337 -> 0.276), complex64 0.279 ->
 // 0.227; freeprop (NL_IF) FP64 0.321 -> 0.219, complex64 0.252 -> 0.217.
 // Shuffles alone, loads not ahead: 0.349-0.361 (FP64, eigenvalue-free).  The
-// Bragg step and the pure phases are two instantiations: in one, the Bragg
-// step lost 0.026 ms to spills.
+// two forms of the Bragg step and the pure phases are three instantiations: with
+// the phases in one, the Bragg step lost 0.026 ms to spills.
 #pragma once
 #include "pass2.cuh"
 
@@ -101,8 +101,9 @@ __device__ __forceinline__ void pair_stage2(cplx<R> *v, const typename TwTab<R>:
   for (int m = 0; m < 16; m++) v[m] = o[m];
 }
 
-template <typename R, int N, bool BRAGG>
+template <typename R, int N, int FORM>
 __global__ void __launch_bounds__(PairCfg<R, N>::NT, PairCfg<R, N>::MINB) pass2_pair_kernel(PassArgs a) {
+  constexpr bool BRAGG = FORM != PAIR_PHASE;
   using C = cplx<R>;
   using TW = typename TwTab<R>::type;
   using Cfg = PairCfg<R, N>;
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(PairCfg<R, N>::NT, PairCfg<R, N>::MINB) pass2_
     pair_stage2<R, N, +1, true>(v, twS, j, sg);
     int ix, iy, iz;
     idx3(a.g, lb, ix, iy, iz);
-    nl_pair16<R, BRAGG>(a.nl, v, c, R2, live, (double)(ix - a.nl.shift0) * a.nl.dx0, om, ec, es,
+    nl_pair16<R, FORM>(a.nl, v, c, R2, live, (double)(ix - a.nl.shift0) * a.nl.dx0, om, ec, es,
                  lb + j, R2);
     dft16<-1>(v);
     #pragma unroll

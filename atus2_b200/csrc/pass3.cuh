@@ -282,8 +282,13 @@ __device__ __forceinline__ void p3_item(const PassArgs &a, const TileGeo &g, uns
       int p0[3];
       idx3(a.g, lb, p0[0], p0[1], p0[2]);
       const double x0 = (double)(p0[0] - a.nl.shift0) * a.nl.dx0;
-      if (a.nl.kind == K_BRAGG) nl_pair16<R, true>(a.nl, v, c, 1, live, x0, s_om[b], s_ec[b], s_es[b], lb + t, M);
-      else nl_pair16<R, false>(a.nl, v, c, 1, live, x0, 0.0, 1.0, 0.0, lb + t, M);
+      const int form = pair_form<R>(a.nl);
+      if (sizeof(R) == 8 && form == PAIR_EIGEN)
+        nl_pair16<R, PAIR_EIGEN>(a.nl, v, c, 1, live, x0, s_om[b], s_ec[b], s_es[b], lb + t, M);
+      else if (form == PAIR_FREE)
+        nl_pair16<R, PAIR_FREE>(a.nl, v, c, 1, live, x0, s_om[b], s_ec[b], s_es[b], lb + t, M);
+      else
+        nl_pair16<R, PAIR_PHASE>(a.nl, v, c, 1, live, x0, 0.0, 1.0, 0.0, lb + t, M);
     } else if constexpr (TC == 1) {
       int p0[3];
       idx3(a.g, lb, p0[0], p0[1], p0[2]);
