@@ -370,7 +370,8 @@ ATUS_API int atus_batch_create(const atus_batch_instance *inst, int count, int p
                                atus_batch **out);
 ATUS_API void atus_batch_destroy(atus_batch *b);
 ATUS_API const char *atus_batch_last_error(const atus_batch *b);
-/* Interleaved complex128 host buffers of the instance's grid size. */
+/* Interleaved complex128 host buffers of the instance's grid size.  Several
+ * host threads may read fields of one batch at the same time. */
 ATUS_API int atus_batch_upload_psi(atus_batch *b, int inst, int comp, const double *psi);
 ATUS_API int atus_batch_download_psi(atus_batch *b, int inst, int comp, double *psi);
 ATUS_API int atus_batch_get_time(const atus_batch *b, int inst, double *t);
